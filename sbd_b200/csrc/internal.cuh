@@ -58,11 +58,16 @@ struct SpinTables {
   double* d_val = nullptr;    // sign * ((p1q1|p2q2) - (p1q2|p2q1))
   uint64_t ns = 0, nd = 0;
   int max_s = 0;
-  // sliced ELL of the singles, keyed by bra: ket | pair<<16 | neg<<31
+  // sliced ELL of the beta singles, keyed by bra: ket | pair<<16 | neg<<31
   size_t nslice = 0;
   int64_t* sell_off = nullptr;  // [nslice+1]
   int32_t* sell_w = nullptr;    // [nslice]
   uint32_t* sell = nullptr;
+  // n8 x k4 tiles of the singles for the FP64 tensor pipe (ab_mma.cu): per 16
+  // bras {first entry / 32, k4 steps of both tiles, of the first, of the second}
+  size_t n_tile_grp = 0;
+  int4* tile_grp = nullptr;
+  uint32_t* tile_ent = nullptr;
   std::vector<int64_t> h_s_off, h_d_off;  // host copies of the offsets
 };
 
@@ -183,6 +188,20 @@ void ensure_rdm_tables(sbdgpu_ctx* c);
 void free_rdm_tables(sbdgpu_ctx* c);
 // sigma.cu: the alpha-beta launch shapes (group size, threads) open to this context's FP64 sigma
 std::vector<std::pair<int, int>> ab_shapes(sbdgpu_ctx* c);
+// The alpha singles an alpha-beta kernel walks: CSR by source string ja (all
+// targets, or only those of one block of target rows, ia0 .. ia0 + rows).
+struct AlphaSingles {
+  const int64_t* off;
+  const int32_t* idx;
+  const uint32_t* info;
+  int max_s;
+  size_t ia0;
+};
+// ab_mma.cu: the alpha-beta term on the FP64 tensor pipe
+void build_ab_tiles(sbdgpu_ctx* c, SpinTables& t, const std::vector<uint64_t>& strs);
+int ab_mma_group(const sbdgpu_ctx* c, int want, size_t budget);
+void ab_mma(sbdgpu_ctx* c, const double* C, double* S, const AlphaSingles& as, int m, int nt, size_t budget);
+void preload_ab_mma(int device);
 // ozaki.cu: the FP64 same-spin terms as exact INT8 products
 bool ensure_ozaki(sbdgpu_ctx* c);
 void free_ozaki(sbdgpu_ctx* c);

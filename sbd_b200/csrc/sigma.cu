@@ -11,14 +11,16 @@
 //                        (task type 2 of the reference: alpha singles/doubles)
 //  same-spin (beta)      the same kernel on the transposed vector C^T, with the
 //                        beta tables and Ja (task type 1), added back transposed
-//  alpha-beta kernel     sigma[ia,ib] += sum_{ja in S(ia)} sum_{jb in S(ib)}
+//  alpha-beta term       sigma[ia,ib] += sum_{ja in S(ia)} sum_{jb in S(ib)}
 //                                        s_a s_b (pq|rs) C[ja,jb]   (task type 0)
 //
 // The rows kernel streams whole rows of C (coalesced) for every table entry of
-// its bra row.  The alpha-beta kernel holds one source row C[ja,:] and the
-// integral rows (pq|.) of a group of ja's singles in shared memory, streams the
-// beta singles (sliced ELL, coalesced) once per group, and adds each group's
-// contributions to sigma rows ia with FP64 atomics.
+// its bra row.  The FP64 alpha-beta term runs on the FP64 tensor pipe
+// (ab_mma.cu).  The gather kernel here serves FP32 and the bases and launch
+// shapes the tiles do not: it holds one source row C[ja,:] and the integral
+// rows (pq|.) of a group of ja's singles in shared memory, streams the beta
+// singles (sliced ELL, coalesced) once per group, and adds each group's
+// contributions to sigma rows ia with atomics.
 #include <algorithm>
 #include <vector>
 
@@ -299,18 +301,6 @@ size_t ab_smem(size_t nb, int P) {
   return ((nb * sizeof(T) + 15) & ~size_t(15)) + (size_t)P * ab_vstride<T, G>() * sizeof(T);
 }
 
-// 512 threads while two CTAs fit in shared memory, else 1024 so that one CTA
-// still keeps 32 warps resident per SM.
-// The alpha singles the kernel walks: CSR by source string ja (all targets, or
-// only those of one block of target rows, ia0 .. ia0 + rows).
-struct AlphaSingles {
-  const int64_t* off;
-  const int32_t* idx;
-  const uint32_t* info;
-  int max_s;
-  size_t ia0;
-};
-
 template <typename T, int G, int NT>
 void launch_ab_nt(sbdgpu_ctx* c, const T* C, T* S, const T* vf, size_t smem, const AlphaSingles& as) {
   const SpinTables& tb = c->tab[1];
@@ -364,7 +354,8 @@ namespace {
 // The alpha-beta term: the context's tuned group size and threads for FP64
 // when set (sbdgpu_set_tuning / sbdgpu_autotune), else the largest group of
 // alpha singles per CTA whose integral block fits in shared memory next to
-// one row of C.
+// one row of C.  FP64 groups of 16 and 8 go to the tile kernel where the basis
+// has tiles; at groups of 4 and fewer a product would be half empty.
 template <typename T>
 void alpha_beta(sbdgpu_ctx* c, const T* C, T* S, const T* vf, const AlphaSingles& as) {
   int dev_smem = 0;
@@ -375,6 +366,11 @@ void alpha_beta(sbdgpu_ctx* c, const T* C, T* S, const T* vf, const AlphaSingles
   int P = c->P;
   const bool tuned = sizeof(T) == 8 && c->ab_group > 0;
   const int g = tuned ? c->ab_group : 0, nt = tuned ? c->ab_threads : 0;
+  if constexpr (sizeof(T) == 8)
+    if (const int m = ab_mma_group(c, g, budget)) {
+      ab_mma(c, C, S, as, m, nt, budget);
+      return;
+    }
   if ((g == 0 || g == 16) && ab_smem<T, 16>(nb, P) <= budget)
     launch_ab<T, 16>(c, C, S, vf, ab_smem<T, 16>(nb, P), as, nt);
   else if ((g == 0 || g == 8) && ab_smem<T, 8>(nb, P) <= budget)
@@ -432,6 +428,7 @@ void preload_fp64_sigma(int device) {
   preload_ab<4>(device);
   preload_ab<2>(device);
   preload_ab<1>(device);
+  preload_ab_mma(device);
   preload_fp64_sigma_misc();
 }
 

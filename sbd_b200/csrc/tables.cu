@@ -133,10 +133,11 @@ __global__ void sell_fill_kernel(int n, const int64_t* __restrict__ s_off, const
 void free_tables(SpinTables& t) {
   cudaFree(t.s_off); cudaFree(t.d_off); cudaFree(t.s_idx); cudaFree(t.s_info); cudaFree(t.s_val);
   cudaFree(t.d_idx); cudaFree(t.d_val); cudaFree(t.sell_off); cudaFree(t.sell_w); cudaFree(t.sell);
+  cudaFree(t.tile_grp); cudaFree(t.tile_ent);
   t = SpinTables();
 }
 
-static void build_one(sbdgpu_ctx* c, SpinTables& t, const uint64_t* dstr, size_t n) {
+static void build_one(sbdgpu_ctx* c, SpinTables& t, const uint64_t* dstr, size_t n, bool beta) {
   cudaStream_t st = c->stream;
   t.n = n;
   int ni = (int)n;
@@ -175,7 +176,11 @@ static void build_one(sbdgpu_ctx* c, SpinTables& t, const uint64_t* dstr, size_t
   fill_kernel<<<blocks, threads, 0, st>>>(dstr, ni, c->L, t.s_off, t.d_off, c->h1, c->vf, c->P, t.s_idx,
                                           t.s_info, t.s_val, t.d_idx, t.d_val);
   SBD_CUDA(cudaGetLastError());
-  // sliced ELL of the singles
+  if (!beta) {
+    SBD_CUDA(cudaStreamSynchronize(st));
+    return;
+  }
+  // sliced ELL of the singles, which the alpha-beta kernels read for the beta strings
   t.nslice = (n + kSlice - 1) / kSlice;
   std::vector<int32_t> w(t.nslice, 0);
   std::vector<int64_t> so(t.nslice + 1, 0);
@@ -197,8 +202,9 @@ static void build_one(sbdgpu_ctx* c, SpinTables& t, const uint64_t* dstr, size_t
 
 void build_tables(sbdgpu_ctx* c) {
   if (c->tables_ready) return;
-  build_one(c, c->tab[0], c->astr, c->na);
-  build_one(c, c->tab[1], c->bstr, c->nb);
+  build_one(c, c->tab[0], c->astr, c->na, false);
+  build_one(c, c->tab[1], c->bstr, c->nb, true);
+  build_ab_tiles(c, c->tab[1], c->h_bstr);
   c->tables_ready = true;
 }
 

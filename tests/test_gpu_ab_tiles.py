@@ -1,0 +1,66 @@
+"""The FP64 alpha-beta term by tiles (csrc/ab_mma.cu) against the CPU oracle
+and the gather kernel: string counts at the edges of its groups of 16 and
+tiles of 8, alpha singles at the edges of 8 and 16 per CTA, odd rows (no
+16-byte lines), and bases that keep the gather kernel."""
+import numpy as np
+import pytest
+
+import oracle
+import sbd_b200
+from sbd_b200 import synth
+
+pytestmark = pytest.mark.gpu
+
+# sums of at most a few thousand FP64 products of O(1) terms: the bound of the sigma parity tests
+TOL = 1e-12
+
+
+def _system(norb, nea, neb, na, nb, seed, shuffle=False):
+    ints = synth.make_integrals(norb, seed)
+    rng = np.random.default_rng(seed)
+
+    def pick(ne, n):
+        s = synth.full_strings(norb, ne)
+        s = s[np.sort(rng.choice(len(s), min(n, len(s)), replace=False))]
+        return rng.permutation(s) if shuffle else s
+    return ints, pick(nea, na), pick(neb, nb)
+
+
+def _check(ints, a, b, shapes=((0, 0),)):
+    ctx = sbd_b200.context_from_integrals(ints, a, b)
+    C = np.random.default_rng(3).normal(size=ctx.n)
+    ref = oracle.Oracle(ints.norb, a, b, ints.ecore, ints.h, ints.eri).sigma(C)
+    for g, t in shapes:
+        ctx.set_tuning(g, t)
+        assert np.abs(ctx.sigma(C) - ref).max() <= TOL * np.abs(ref).max(), (g, t)
+    ctx.close()
+
+
+@pytest.mark.parametrize("nb", [1, 2, 7, 8, 9, 15, 16, 17, 31, 32, 33, 50])
+def test_beta_strings_at_group_edges(nb):
+    _check(*_system(9, 3, 3, 21, nb, 100 + nb))
+
+
+@pytest.mark.parametrize("norb,nea", [(3, 1), (5, 1), (9, 1), (10, 1), (17, 1), (18, 1), (8, 4), (10, 5)])
+def test_alpha_singles_at_block_edges(norb, nea):
+    # full spaces: nea (norb - nea) = 2, 4, 8, 9, 16, 17, 16 and 25 singles per alpha string
+    _check(*_system(norb, nea, min(2, nea), 10 ** 6, 40, norb), shapes=((0, 0), (16, 128), (8, 256), (4, 128)))
+
+
+@pytest.mark.parametrize("shuffle", [False, True])
+def test_unequal_spins_and_string_order(shuffle):
+    _check(*_system(11, 5, 3, 67, 133, 5, shuffle), shapes=((0, 0), (16, 512), (8, 128), (2, 128)))
+
+
+def test_wide_orbital_range():
+    # 2,016 off-diagonal pairs, the largest pair index
+    ints = synth.make_integrals(64, 2)
+    rng = np.random.default_rng(2)
+    s = np.array([(1 << 63) | (1 << i) for i in range(60)] + [3 << i for i in range(62)], dtype=np.uint64)
+    b = np.sort(rng.choice(s, 40, replace=False))
+    _check(ints, b[:9], b)
+
+
+def test_repeated_strings_keep_the_gather_kernel():
+    ints, a, b = _system(8, 3, 3, 20, 30, 9)
+    _check(ints, a, np.concatenate([b, b[:3]]))
