@@ -7,26 +7,30 @@
 //   states      [n][nw] uint64 in the caller's order (site q at bit q%64 of
 //               word q/64), nw = 1, 2 or 4
 //   hash table  open addressing with linear probing over a power-of-two
-//               table of at least twice the states: key words and the
-//               caller's index (-1 marks an empty slot); the target of every
-//               off-diagonal term is found in one to three probes
-//   terms       the off-diagonal list as fixed-size records: annihilation and
-//               creation masks (the sites of the first n_dag operators and of
-//               the rest), the coefficient and the operator sites in order
-//               (for the fermionic sign), sorted by annihilation mask, with one
-//               bucket record per distinct mask; the diagonal list is folded
-//               into one number per state at set-up (hdiag)
+//               table of at least twice the states: a slot holds the key words
+//               and, during a mult, the state's vector element, so that one
+//               probe returns the value itself (a slot of one-word states is 16
+//               bytes: one sector per term instead of three for index, key and
+//               element).  An empty slot's key is a configuration outside the
+//               basis and its element 0.
+//   terms       the off-diagonal list as arrays (creation mask, sign mask,
+//               coefficient) sorted by annihilation mask, with one bucket
+//               record per distinct mask; the diagonal list is folded into one
+//               number per state at set-up (hdiag)
 //
-// mult: one warp per bra state.  The warp walks the buckets (warp-uniform),
-// skips every bucket whose annihilated sites are not all occupied in the
-// state, and splits the terms of the others over its lanes.  A term applies
-// when its created sites are empty after the annihilation, which with the
-// bucket's test is the reference's sequential test (mult.h:213-240) for terms
-// whose annihilated sites are distinct and whose created sites are distinct
-// (a term that repeats a site in either part never applies there and is
-// dropped at set-up).  The lanes' sums are reduced in the warp, so no
-// atomics.  For a chemistry operator a state's occupation admits about one
-// bucket in ten.
+// mult: one warp per bra state.  Its lanes test 32 buckets at a time for
+// annihilated sites that are all occupied in the state and split the terms of
+// each bucket that passes.  A term applies when its created sites are empty
+// after the annihilation, which with the bucket's test is the reference's
+// sequential test (mult.h:213-240) for terms whose annihilated sites are
+// distinct and whose created sites are distinct (a term that repeats a site in
+// either part never applies there and is dropped at set-up).  The sign is the
+// parity of the occupied sites below each operator's site, in order: the
+// operators before it have flipped sites of their own, so the total is the
+// parity of the state under the exclusive-or of the "below" masks, times a
+// constant that goes into the coefficient.  The lanes' sums are reduced in the
+// warp, so no atomics.  Bound by the random 32-byte sectors of the hash table
+// in L2, one per Hamiltonian element.
 #include <algorithm>
 #include <chrono>
 #include <cmath>
@@ -47,10 +51,16 @@ struct sbdgpu_genop {
   size_t n = 0;
   int sign = 1;
   uint64_t* states = nullptr;
-  uint64_t* hkeys = nullptr;  // hash table: [slots][nw] key words
-  int64_t* hidx = nullptr;    // [slots] caller index, -1 = empty
+  void* slots = nullptr;      // hash table, Slot<nw> each
+  int64_t* slot_of = nullptr; // [n] slot of every state
   uint64_t hmask = 0;         // slots - 1
-  void* terms = nullptr;       // off-diagonal records, sorted by annihilation mask
+  uint64_t absent[4] = {};    // key of an empty slot: a configuration outside the basis
+  uint64_t site_or[4] = {};   // every site of a basis state
+  uint64_t term_or[4] = {};   // every site an off-diagonal term creates
+  // off-diagonal terms, sorted by annihilation mask
+  uint64_t* t_cre = nullptr;   // [n_terms][nw] created sites
+  uint64_t* t_sgn = nullptr;   // [n_terms][nw] sites whose occupations give the sign
+  double* t_coef = nullptr;    // coefficient, the sign's constant part included
   void* buckets = nullptr;     // one record per distinct annihilation mask
   size_t n_buckets = 0;
   size_t n_terms = 0;
@@ -102,23 +112,104 @@ __host__ __device__ __forceinline__ uint64_t hash_state(const uint64_t* w) {
   return h;
 }
 
-// caller index of state w, or -1
 template <int NW>
-__device__ __forceinline__ int64_t find_state(const uint64_t* __restrict__ hkeys, const int64_t* __restrict__ hidx,
-                                              uint64_t hmask, const uint64_t* w) {
+struct alignas(NW == 1 ? 16 : NW == 2 ? 32 : 64) Slot {
+  uint64_t key[NW];
+  double val;
+};
+
+// The off-diagonal terms on the device.
+template <int NW>
+struct TermList {
+  const Bucket<NW>* buckets;
+  size_t n_buckets;
+  const uint64_t* cre;
+  const uint64_t* sgn;
+  const double* coef;
+};
+
+// the vector element of state w, 0 when it is outside the basis
+template <int NW>
+__device__ __forceinline__ double element(const Slot<NW>* __restrict__ slots, uint64_t hmask, const uint64_t* absent,
+                                          const uint64_t* w) {
   uint64_t h = hash_state<NW>(w) & hmask;
   // the table is at most half full, so an empty slot ends every probe
   // sequence; the bound keeps the loop finite regardless
   for (uint64_t probe = 0; probe <= hmask; probe++) {
-    const int64_t id = __ldg(&hidx[h]);
-    if (id < 0) return -1;
-    bool eq = true;
+    uint64_t key[NW];
+    double val;
+    if constexpr (NW == 1) {
+      const ulonglong2 x = __ldg(reinterpret_cast<const ulonglong2*>(&slots[h]));
+      key[0] = x.x;
+      val = __longlong_as_double((long long)x.y);
+    } else {
 #pragma unroll
-    for (int x = 0; x < NW; x++) eq &= __ldg(&hkeys[h * NW + x]) == w[x];
-    if (eq) return id;
+      for (int x = 0; x < NW; x++) key[x] = __ldg(&slots[h].key[x]);
+      val = __ldg(&slots[h].val);
+    }
+    bool eq = true, empty = true;
+#pragma unroll
+    for (int x = 0; x < NW; x++) {
+      eq &= key[x] == w[x];
+      empty &= key[x] == absent[x];
+    }
+    if (eq) return val;
+    if (empty) return 0.0;
     h = (h + 1) & hmask;
   }
-  return -1;
+  return 0.0;
+}
+
+// slots' elements <- C
+template <int NW>
+__global__ void scatter_kernel(Slot<NW>* __restrict__ slots, const int64_t* __restrict__ slot_of,
+                               const double* __restrict__ C, size_t n) {
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
+    slots[slot_of[i]].val = C[i];
+}
+
+// Calls f(lane applies, target, coefficient with sign) for every term of every
+// bucket that applies to state v, by the whole warp (lanes past a bucket's end
+// or whose term does not apply are called with false).
+template <int NW, class F>
+__device__ __forceinline__ void for_terms(const TermList<NW>& tl, const uint64_t (&v)[NW], F&& f) {
+  const int lane = threadIdx.x & 31;
+  for (size_t b0 = 0; b0 < tl.n_buckets; b0 += 32) {
+    bool ok = b0 + lane < tl.n_buckets;
+    if (ok) {
+#pragma unroll
+      for (int x = 0; x < NW; x++) {
+        const uint64_t m = __ldg(&tl.buckets[b0 + lane].ann[x]);
+        ok &= (v[x] & m) == m;
+      }
+    }
+    for (unsigned hits = __ballot_sync(0xffffffffu, ok); hits; hits &= hits - 1) {
+      const Bucket<NW>* bk = &tl.buckets[b0 + __ffs((int)hits) - 1];
+      uint64_t left[NW];
+#pragma unroll
+      for (int x = 0; x < NW; x++) left[x] = v[x] & ~__ldg(&bk->ann[x]);
+      const int64_t t1 = __ldg(&bk->end);
+      for (int64_t t0 = __ldg(&bk->start); t0 < t1; t0 += 32) {
+        const int64_t t = t0 + lane;
+        bool on = t < t1;
+        uint64_t w[NW];
+        double c = 0.0;
+        if (on) {
+          int par = 0;
+#pragma unroll
+          for (int x = 0; x < NW; x++) {
+            const uint64_t cre = __ldg(&tl.cre[t * NW + x]);
+            on &= (left[x] & cre) == 0ull;
+            w[x] = left[x] | cre;
+            par += __popcll(v[x] & __ldg(&tl.sgn[t * NW + x]));
+          }
+          c = __ldg(&tl.coef[t]);
+          c = par & 1 ? -c : c;
+        }
+        f(on, w, c);
+      }
+    }
+  }
 }
 
 // parity of the occupied sites below q
@@ -165,14 +256,18 @@ __device__ __forceinline__ bool apply_term(const Term<NW>& t, const uint64_t* v,
 }
 
 // W[i] += hdiag[i] C[i] + sum over off-diagonal terms of coef * sign * C[j]:
-// one warp per state, its lanes over the terms of each applicable bucket
+// one warp per state.  The 349M elements of the 245,025-state FCIDUMP operator
+// took 16.1 ms with index, key and element in three sectors, the sign from the
+// operators one by one and the buckets tested one after another.
 constexpr int kMultWarps = kThreads / 32;
 template <int NW>
+struct Words {
+  uint64_t w[NW];
+};
+template <int NW>
 __global__ void __launch_bounds__(kThreads) mult_kernel(const uint64_t* __restrict__ states, size_t n,
-                                                       const uint64_t* __restrict__ hkeys,
-                                                       const int64_t* __restrict__ hidx, uint64_t hmask,
-                                                       const Bucket<NW>* __restrict__ buckets, size_t n_buckets,
-                                                       const Term<NW>* __restrict__ terms, int sign,
+                                                       const Slot<NW>* __restrict__ slots, uint64_t hmask,
+                                                       Words<NW> absent, TermList<NW> tl,
                                                        const double* __restrict__ hdiag,
                                                        const double* __restrict__ C, double* __restrict__ W) {
   const int lane = threadIdx.x & 31;
@@ -182,23 +277,9 @@ __global__ void __launch_bounds__(kThreads) mult_kernel(const uint64_t* __restri
 #pragma unroll
     for (int x = 0; x < NW; x++) v[x] = __ldg(&states[i * NW + x]);
     double acc = 0.0;
-    for (size_t b = 0; b < n_buckets; b++) {
-      bool ok = true;
-#pragma unroll
-      for (int x = 0; x < NW; x++) {
-        const uint64_t m = __ldg(&buckets[b].ann[x]);
-        ok &= (v[x] & m) == m;
-      }
-      if (!ok) continue;  // warp-uniform: the same state in every lane
-      const int64_t t1 = __ldg(&buckets[b].end);
-      for (int64_t t = __ldg(&buckets[b].start) + lane; t < t1; t += 32) {
-        uint64_t w[NW];
-        double s;
-        if (!apply_term<NW>(terms[t], v, sign, w, &s)) continue;
-        const int64_t j = find_state<NW>(hkeys, hidx, hmask, w);
-        if (j >= 0) acc += __ldg(&terms[t].coef) * s * __ldg(&C[j]);
-      }
-    }
+    for_terms<NW>(tl, v, [&](bool on, const uint64_t (&w)[NW], double c) {
+      if (on) acc += c * element<NW>(slots, hmask, absent.w, w);
+    });
 #pragma unroll
     for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
     if (lane == 0) W[i] = W[i] + hdiag[i] * C[i] + acc;
@@ -265,6 +346,46 @@ int guarded(sbdgpu_genop* g, F&& f) {
     g->base.err = e.what();
     return SBDGPU_ERR_STATE;
   }
+}
+
+// The basis on the device: states, hash table and every state's slot.
+template <int NW>
+void build_basis(sbdgpu_genop* g, const uint64_t* states) {
+  const size_t n = g->n;
+  cudaStream_t st = g->base.stream;
+  size_t count = 1024;  // at least twice the states, a power of two
+  while (count < 2 * n) count <<= 1;
+  g->hmask = count - 1;
+  std::vector<int64_t> at(count, -1), slot_of(n);  // state of a slot, slot of a state
+  // slot of configuration w, or of the empty slot that ends its search
+  const auto find = [&](const uint64_t* w) {
+    uint64_t h = hash_state<NW>(w) & g->hmask;
+    while (at[h] >= 0 && !std::equal(w, w + NW, &states[(size_t)at[h] * NW])) h = (h + 1) & g->hmask;
+    return h;
+  };
+  for (size_t i = 0; i < n; i++) {
+    const uint64_t h = find(&states[i * NW]);
+    if (at[h] >= 0) throw Error{SBDGPU_ERR_ARG, "repeated basis state"};
+    at[h] = (int64_t)i;
+    slot_of[i] = (int64_t)h;
+    for (int x = 0; x < NW; x++) g->site_or[x] |= states[i * NW + x];
+  }
+  uint64_t none[NW];
+  std::fill(none, none + NW, ~0ull);
+  while (at[find(none)] >= 0) none[0]--;
+  std::memcpy(g->absent, none, sizeof(none));
+  std::vector<Slot<NW>> table(count);
+  for (size_t h = 0; h < count; h++) {
+    std::memcpy(table[h].key, at[h] >= 0 ? &states[(size_t)at[h] * NW] : none, sizeof(none));
+    table[h].val = 0.0;
+  }
+  g->states = (uint64_t*)sbdgpu::dev_alloc(sizeof(uint64_t) * n * NW);
+  g->slots = sbdgpu::dev_alloc(sizeof(Slot<NW>) * count);
+  g->slot_of = (int64_t*)sbdgpu::dev_alloc(sizeof(int64_t) * n);
+  SBD_CUDA(cudaMemcpyAsync(g->states, states, sizeof(uint64_t) * n * NW, cudaMemcpyHostToDevice, st));
+  SBD_CUDA(cudaMemcpyAsync(g->slots, table.data(), sizeof(Slot<NW>) * count, cudaMemcpyHostToDevice, st));
+  SBD_CUDA(cudaMemcpyAsync(g->slot_of, slot_of.data(), sizeof(int64_t) * n, cudaMemcpyHostToDevice, st));
+  SBD_CUDA(cudaStreamSynchronize(st));  // the host copies leave scope
 }
 
 // One list's terms as host records.  Off-diagonal terms that repeat a site
@@ -338,10 +459,35 @@ void set_terms_nw(sbdgpu_genop* g, size_t n_diag, const int64_t* diag_off, const
     }
     bk.back().end = (int64_t)t + 1;
   }
-  cudaFree(g->terms);
+  // creation masks, sign masks (below-masks of the operators' sites) and
+  // coefficients with the constant part of the sign: the operators before one
+  // have flipped their own sites, those below it count
+  std::vector<uint64_t> cre(all.size() * NW), sgn(all.size() * NW, 0);
+  std::vector<double> cf(all.size());
+  uint64_t term_or[4] = {};
+  for (size_t t = 0; t < all.size(); t++) {
+    int flips = 0;
+    for (int k = 0; g->sign && k < all[t].nops; k++) {
+      const int q = all[t].site[k];
+      for (int x = 0; x < (q >> 6); x++) sgn[t * NW + x] ^= ~0ull;
+      sgn[t * NW + (q >> 6)] ^= (1ull << (q & 63)) - 1ull;
+      for (int j = 0; j < k; j++) flips += all[t].site[j] < q;
+    }
+    cf[t] = flips & 1 ? -all[t].coef : all[t].coef;
+    for (int x = 0; x < NW; x++) {
+      cre[t * NW + x] = all[t].cre[x];
+      term_or[x] |= all[t].cre[x];
+    }
+  }
+  std::memcpy(g->term_or, term_or, sizeof(term_or));
+  cudaFree(g->t_cre);
+  cudaFree(g->t_sgn);
+  cudaFree(g->t_coef);
   cudaFree(g->self_terms);
   cudaFree(g->buckets);
-  g->terms = g->self_terms = g->buckets = nullptr;
+  g->self_terms = g->buckets = nullptr;
+  g->t_cre = g->t_sgn = nullptr;
+  g->t_coef = nullptr;
   g->n_buckets = 0;
   g->ready = false;
   DiagTerm<NW>* d_dt = nullptr;
@@ -354,8 +500,13 @@ void set_terms_nw(sbdgpu_genop* g, size_t n_diag, const int64_t* diag_off, const
     diag_kernel<NW><<<blocks_for(g->n), kThreads, 0, st>>>(g->states, g->n, d_dt, dt.size(), g->hdiag);
     SBD_CUDA(cudaGetLastError());
     if (!all.empty()) {
-      g->terms = sbdgpu::dev_alloc(sizeof(Term<NW>) * all.size());
-      SBD_CUDA(cudaMemcpyAsync(g->terms, all.data(), sizeof(Term<NW>) * all.size(), cudaMemcpyHostToDevice, st));
+      const size_t mask_bytes = sizeof(uint64_t) * NW * all.size();
+      g->t_cre = (uint64_t*)sbdgpu::dev_alloc(mask_bytes);
+      SBD_CUDA(cudaMemcpyAsync(g->t_cre, cre.data(), mask_bytes, cudaMemcpyHostToDevice, st));
+      g->t_sgn = (uint64_t*)sbdgpu::dev_alloc(mask_bytes);
+      SBD_CUDA(cudaMemcpyAsync(g->t_sgn, sgn.data(), mask_bytes, cudaMemcpyHostToDevice, st));
+      g->t_coef = (double*)sbdgpu::dev_alloc(sizeof(double) * all.size());
+      SBD_CUDA(cudaMemcpyAsync(g->t_coef, cf.data(), sizeof(double) * all.size(), cudaMemcpyHostToDevice, st));
       g->buckets = sbdgpu::dev_alloc(sizeof(Bucket<NW>) * bk.size());
       SBD_CUDA(cudaMemcpyAsync(g->buckets, bk.data(), sizeof(Bucket<NW>) * bk.size(), cudaMemcpyHostToDevice, st));
     }
@@ -377,12 +528,21 @@ void set_terms_nw(sbdgpu_genop* g, size_t n_diag, const int64_t* diag_off, const
 }
 
 template <int NW>
+TermList<NW> term_list(const sbdgpu_genop* g) {
+  return TermList<NW>{static_cast<const Bucket<NW>*>(g->buckets), g->n_buckets, g->t_cre, g->t_sgn, g->t_coef};
+}
+
+template <int NW>
 void mult_nw(sbdgpu_genop* g, const double* C, double* W) {
-  const unsigned grid = (unsigned)std::min<size_t>((g->n + kMultWarps - 1) / kMultWarps, 148 * 16);
-  mult_kernel<NW><<<grid, kThreads, 0, g->base.stream>>>(g->states, g->n, g->hkeys, g->hidx, g->hmask,
-                                                        static_cast<const Bucket<NW>*>(g->buckets), g->n_buckets,
-                                                        static_cast<const Term<NW>*>(g->terms), g->sign, g->hdiag,
-                                                        C, W);
+  Slot<NW>* slots = static_cast<Slot<NW>*>(g->slots);
+  scatter_kernel<NW><<<(unsigned)std::min<size_t>(blocks_for(g->n), 148 * 8), kThreads, 0, g->base.stream>>>(
+      slots, g->slot_of, C, g->n);
+  SBD_CUDA(cudaGetLastError());
+  Words<NW> absent;
+  std::memcpy(absent.w, g->absent, sizeof(absent.w));
+  const unsigned grid = (unsigned)std::min<size_t>((g->n + kMultWarps - 1) / kMultWarps, 148 * 64);
+  mult_kernel<NW><<<grid, kThreads, 0, g->base.stream>>>(g->states, g->n, slots, g->hmask, absent, term_list<NW>(g),
+                                                        g->hdiag, C, W);
   SBD_CUDA(cudaGetLastError());
 }
 
@@ -575,10 +735,14 @@ void davidson(sbdgpu_genop* g, const sbdgpu_opts* o, double* Wh, double* energy,
 //
 // MeasHamSquare and ExpandBasis (expand.h:10-366) look past the basis: every
 // configuration an off-diagonal term reaches from a basis state, with weight
-// coef * sign * W_i.  Here a count pass and a write pass lay those out (with
-// the basis states themselves first), a least-significant-word-first radix
-// sort of their indices (CUB) orders them by configuration, and head flags
-// mark each distinct configuration.
+// coef * sign * W_i.  Here a count pass and a write pass (one warp per state
+// over its applicable buckets, as in the mult) lay those out with the basis
+// states themselves first, a radix sort (CUB) orders them by configuration,
+// and head flags mark each distinct configuration.  One-word configurations
+// are sorted themselves, with their weights where those are wanted, over the
+// bits that occur; wider ones through their indices, least significant word
+// first.  Every state testing every term in a thread of its own took 97 % of
+// the GPU time of a 4,900-state expansion (21 ms a call).
 
 constexpr int kGenThreads = 256;
 
@@ -586,52 +750,66 @@ constexpr int kGenThreads = 256;
 // |coef sign W_i| > eps when select)
 template <int NW>
 __global__ void __launch_bounds__(kGenThreads) gen_count_kernel(const uint64_t* __restrict__ states, size_t n,
-                                                               const Term<NW>* __restrict__ terms, size_t n_terms,
-                                                               int sign, const double* __restrict__ W, double eps,
-                                                               int select, int64_t* __restrict__ counts) {
-  const size_t i = (size_t)blockIdx.x * kGenThreads + threadIdx.x;
-  if (i >= n) return;
-  uint64_t v[NW];
+                                                               TermList<NW> tl, const double* __restrict__ W,
+                                                               double eps, int select, int64_t* __restrict__ counts) {
+  const int lane = threadIdx.x & 31;
+  const size_t warps = ((size_t)gridDim.x * kGenThreads) >> 5;
+  for (size_t i = ((size_t)blockIdx.x * kGenThreads + threadIdx.x) >> 5; i < n; i += warps) {
+    uint64_t v[NW];
 #pragma unroll
-  for (int x = 0; x < NW; x++) v[x] = states[i * NW + x];
-  const double wi = W[i];
-  int64_t cnt = 1;
-  for (size_t k = 0; k < n_terms; k++) {
-    uint64_t w[NW];
-    double s;
-    if (!apply_term<NW>(terms[k], v, sign, w, &s)) continue;
-    if (!select || fabs(terms[k].coef * s * wi) > eps) cnt++;
+    for (int x = 0; x < NW; x++) v[x] = __ldg(&states[i * NW + x]);
+    const double wi = W[i];
+    int64_t cnt = 1;
+    for_terms<NW>(tl, v, [&](bool on, const uint64_t (&)[NW], double c) {
+      cnt += __popc(__ballot_sync(0xffffffffu, on && (!select || fabs(c * wi) > eps)));
+    });
+    if (lane == 0) counts[i] = cnt;
   }
-  counts[i] = cnt;
 }
 
 template <int NW>
 __global__ void __launch_bounds__(kGenThreads) gen_write_kernel(const uint64_t* __restrict__ states, size_t n,
-                                                               const Term<NW>* __restrict__ terms, size_t n_terms,
-                                                               int sign, const double* __restrict__ W,
+                                                               TermList<NW> tl, const double* __restrict__ W,
                                                                const double* __restrict__ hdiag, double eps, int select,
                                                                const int64_t* __restrict__ offs,
                                                                uint64_t* __restrict__ keys, double* __restrict__ vals) {
-  const size_t i = (size_t)blockIdx.x * kGenThreads + threadIdx.x;
-  if (i >= n) return;
-  uint64_t v[NW];
+  const int lane = threadIdx.x & 31;
+  const size_t warps = ((size_t)gridDim.x * kGenThreads) >> 5;
+  for (size_t i = ((size_t)blockIdx.x * kGenThreads + threadIdx.x) >> 5; i < n; i += warps) {
+    uint64_t v[NW];
 #pragma unroll
-  for (int x = 0; x < NW; x++) v[x] = states[i * NW + x];
-  const double wi = W[i];
-  int64_t o = offs[i];
+    for (int x = 0; x < NW; x++) v[x] = __ldg(&states[i * NW + x]);
+    const double wi = W[i];
+    int64_t o = offs[i];
+    if (lane == 0) {
 #pragma unroll
-  for (int x = 0; x < NW; x++) keys[(size_t)o * NW + x] = v[x];
-  vals[o++] = hdiag[i] * wi;  // the diagonal list's weight (expand.h:43-64)
-  for (size_t k = 0; k < n_terms; k++) {
-    uint64_t w[NW];
-    double s;
-    if (!apply_term<NW>(terms[k], v, sign, w, &s)) continue;
-    const double val = terms[k].coef * s * wi;
-    if (select && !(fabs(val) > eps)) continue;
+      for (int x = 0; x < NW; x++) keys[(size_t)o * NW + x] = v[x];
+      if (vals) vals[o] = hdiag[i] * wi;  // the diagonal list's weight (expand.h:43-64)
+    }
+    o++;
+    for_terms<NW>(tl, v, [&](bool on, const uint64_t (&w)[NW], double c) {
+      const double val = c * wi;
+      const bool put = on && (!select || fabs(val) > eps);
+      const unsigned m = __ballot_sync(0xffffffffu, put);
+      if (put) {
+        const size_t at = (size_t)o + __popc(m & ((1u << lane) - 1u));
 #pragma unroll
-    for (int x = 0; x < NW; x++) keys[(size_t)o * NW + x] = w[x];
-    vals[o++] = val;
+        for (int x = 0; x < NW; x++) keys[at * NW + x] = w[x];
+        if (vals) vals[at] = val;
+      }
+      o += __popc(m);
+    });
   }
+}
+
+__global__ void iota_kernel(int64_t* __restrict__ out, size_t m) {
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += (size_t)gridDim.x * blockDim.x)
+    out[i] = (int64_t)i;
+}
+
+// entry of sorted place i (idx null: the entries themselves are sorted)
+__device__ __forceinline__ size_t entry(const int64_t* __restrict__ idx, size_t i) {
+  return idx ? (size_t)idx[i] : i;
 }
 
 __global__ void gather_word_kernel(const uint64_t* __restrict__ keys, int nw, int word,
@@ -646,16 +824,16 @@ __global__ void head_kernel(const uint64_t* __restrict__ keys, int nw, const int
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += (size_t)gridDim.x * blockDim.x) {
     int64_t h = i == 0;
     if (i > 0)
-      for (int x = 0; x < nw; x++) h |= keys[(size_t)idx[i] * nw + x] != keys[(size_t)idx[i - 1] * nw + x];
+      for (int x = 0; x < nw; x++) h |= keys[entry(idx, i) * nw + x] != keys[entry(idx, i - 1) * nw + x];
     head[i] = h;
   }
 }
 
-// sums[seg[i]] += vals[idx[i]] (seg = inclusive scan of head - 1)
+// sums[seg[i]] += vals of sorted entry i (seg = inclusive scan of head - 1)
 __global__ void seg_sum_kernel(const int64_t* __restrict__ seg, const int64_t* __restrict__ idx,
                                const double* __restrict__ vals, double* __restrict__ sums, size_t m) {
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += (size_t)gridDim.x * blockDim.x)
-    atomicAdd(&sums[seg[i] - 1], vals[idx[i]]);
+    atomicAdd(&sums[seg[i] - 1], vals[entry(idx, i)]);
 }
 
 // out[seg[i]-1] = key of entry i for the heads
@@ -664,7 +842,7 @@ __global__ void compact_kernel(const uint64_t* __restrict__ keys, int nw, const 
                                uint64_t* __restrict__ out, size_t m) {
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += (size_t)gridDim.x * blockDim.x)
     if (head[i])
-      for (int x = 0; x < nw; x++) out[(size_t)(seg[i] - 1) * nw + x] = keys[(size_t)idx[i] * nw + x];
+      for (int x = 0; x < nw; x++) out[(size_t)(seg[i] - 1) * nw + x] = keys[entry(idx, i) * nw + x];
 }
 
 }  // namespace
@@ -672,9 +850,9 @@ __global__ void compact_kernel(const uint64_t* __restrict__ keys, int nw, const 
 
 namespace {
 
-// The expanded space of W: sorted entry indices (idx), their configuration
-// keys, weights, head flags and segment numbers (inclusive scan of the
-// heads), all on the device; returns the number of distinct configurations.
+// The expanded space of W: sorted entries (by idx, or themselves where idx is
+// null), their configuration keys, weights (null when not wanted), head flags
+// and segment numbers (inclusive scan of the heads), all on the device.
 struct Expanded {
   std::vector<void*> bufs;
   cudaStream_t s = nullptr;
@@ -694,72 +872,113 @@ struct Expanded {
   }
 };
 
+// Slices of one allocation, 256-byte aligned.
+struct Slices {
+  size_t total = 0;
+  size_t add(size_t bytes) {
+    const size_t at = total;
+    total += (bytes + 255) / 256 * 256;
+    return at;
+  }
+};
+
 template <int NW>
-void expand_nw(sbdgpu_genop* g, const double* dW, double eps, int select, Expanded& x) {
+void expand_nw(sbdgpu_genop* g, const double* dW, double eps, int select, bool weights, Expanded& x) {
   cudaStream_t st = g->base.stream;
   x.s = st;
   const size_t n = g->n;
-  const unsigned nblk = (unsigned)((n + kGenThreads - 1) / kGenThreads);
-  const Term<NW>* terms = static_cast<const Term<NW>*>(g->terms);
-  int64_t* counts = (int64_t*)x.alloc(sizeof(int64_t) * (n + 1));
-  int64_t* offs = (int64_t*)x.alloc(sizeof(int64_t) * (n + 1));
+  const unsigned nblk = (unsigned)std::min<size_t>((n * 32 + kGenThreads - 1) / kGenThreads, 148 * 64);
+  const TermList<NW> tl = term_list<NW>(g);
+  size_t tscan = 0;
+  SBD_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tscan, (int64_t*)nullptr, (int64_t*)nullptr, n + 1, st));
+  Slices a;
+  const size_t at_counts = a.add(sizeof(int64_t) * (n + 1)), at_offs = a.add(sizeof(int64_t) * (n + 1)),
+               at_tmp = a.add(tscan);
+  char* first = (char*)x.alloc(a.total);
+  int64_t* counts = (int64_t*)(first + at_counts);
+  int64_t* offs = (int64_t*)(first + at_offs);
   SBD_CUDA(cudaMemsetAsync(counts + n, 0, sizeof(int64_t), st));
-  gen_count_kernel<NW><<<nblk, kGenThreads, 0, st>>>(g->states, n, terms, g->n_terms, g->sign, dW, eps, select,
-                                                     counts);
+  gen_count_kernel<NW><<<nblk, kGenThreads, 0, st>>>(g->states, n, tl, dW, eps, select, counts);
   SBD_CUDA(cudaGetLastError());
-  size_t tb = 0;
-  SBD_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb, counts, offs, n + 1, st));
-  void* tmp = x.alloc(tb);
-  SBD_CUDA(cub::DeviceScan::ExclusiveSum(tmp, tb, counts, offs, n + 1, st));
+  SBD_CUDA(cub::DeviceScan::ExclusiveSum(first + at_tmp, tscan, counts, offs, n + 1, st));
   int64_t m = 0;
   SBD_CUDA(cudaMemcpyAsync(&m, offs + n, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
   SBD_CUDA(cudaStreamSynchronize(st));
   x.m = (size_t)m;
-  x.keys = (uint64_t*)x.alloc(sizeof(uint64_t) * x.m * NW);
-  x.vals = (double*)x.alloc(sizeof(double) * x.m);
-  gen_write_kernel<NW><<<nblk, kGenThreads, 0, st>>>(g->states, n, terms, g->n_terms, g->sign, dW, g->hdiag, eps,
-                                                     select, offs, x.keys, x.vals);
-  SBD_CUDA(cudaGetLastError());
-  // sort the entry indices by configuration, least significant word first
-  // (each radix pass is stable)
-  int64_t* ia = (int64_t*)x.alloc(sizeof(int64_t) * x.m);
-  int64_t* ib = (int64_t*)x.alloc(sizeof(int64_t) * x.m);
-  uint64_t* ka = (uint64_t*)x.alloc(sizeof(uint64_t) * x.m);
-  uint64_t* kb = (uint64_t*)x.alloc(sizeof(uint64_t) * x.m);
-  std::vector<int64_t> iota(x.m);
-  for (size_t i = 0; i < x.m; i++) iota[i] = (int64_t)i;
-  SBD_CUDA(cudaMemcpyAsync(ia, iota.data(), sizeof(int64_t) * x.m, cudaMemcpyHostToDevice, st));
-  const unsigned gb = (unsigned)std::min<size_t>((x.m + 255) / 256 + 1, 148 * 8);
-  size_t tsort = 0;
-  SBD_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tsort, ka, kb, ia, ib, x.m, 0, 64, st));
-  void* tmp2 = x.alloc(tsort);
+  // bits above the highest site in use are equal in every configuration
+  int end_bit[NW];
   for (int w = 0; w < NW; w++) {
-    gather_word_kernel<<<gb, 256, 0, st>>>(x.keys, NW, w, ia, ka, x.m);
-    SBD_CUDA(cudaGetLastError());
-    SBD_CUDA(cub::DeviceRadixSort::SortPairs(tmp2, tsort, ka, kb, ia, ib, x.m, 0, 64, st));
-    std::swap(ia, ib);
+    const uint64_t any = g->site_or[w] | g->term_or[w];
+    end_bit[w] = any ? 64 - __builtin_clzll(any) : 0;
   }
-  x.idx = ia;
-  x.head = (int64_t*)x.alloc(sizeof(int64_t) * x.m);
-  x.seg = (int64_t*)x.alloc(sizeof(int64_t) * x.m);
+  size_t tsort = 0, tseg = 0;
+  uint64_t* kn = nullptr;
+  double* vn = nullptr;
+  int64_t* in = nullptr;
+  if (NW > 1)
+    SBD_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tsort, kn, kn, in, in, x.m, 0, 64, st));
+  else if (weights)
+    SBD_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tsort, kn, kn, vn, vn, x.m, 0, 64, st));
+  else
+    SBD_CUDA(cub::DeviceRadixSort::SortKeys(nullptr, tsort, kn, kn, x.m, 0, 64, st));
+  SBD_CUDA(cub::DeviceScan::InclusiveSum(nullptr, tseg, in, in, x.m, st));
+  // one allocation: keys, weights, the sort's second buffers head
+  // flags, segment numbers and the libraries' scratch
+  Slices b;
+  const size_t at_keys = b.add(sizeof(uint64_t) * x.m * NW), at_vals = b.add(weights ? sizeof(double) * x.m : 0),
+               at_k2 = b.add(sizeof(uint64_t) * x.m), at_v2 = b.add(sizeof(double) * x.m),
+               at_k3 = b.add(NW > 1 ? sizeof(uint64_t) * x.m : 0), at_i3 = b.add(NW > 1 ? sizeof(int64_t) * x.m : 0),
+               at_head = b.add(sizeof(int64_t) * x.m), at_seg = b.add(sizeof(int64_t) * x.m),
+               at_t = b.add(std::max(tsort, tseg));
+  char* p = (char*)x.alloc(b.total);
+  x.keys = (uint64_t*)(p + at_keys);
+  x.vals = weights ? (double*)(p + at_vals) : nullptr;
+  x.head = (int64_t*)(p + at_head);
+  x.seg = (int64_t*)(p + at_seg);
+  gen_write_kernel<NW><<<nblk, kGenThreads, 0, st>>>(g->states, n, tl, dW, g->hdiag, eps, select, offs, x.keys,
+                                                     x.vals);
+  SBD_CUDA(cudaGetLastError());
+  const unsigned gb = (unsigned)std::min<size_t>((x.m + 255) / 256 + 1, 148 * 8);
+  if constexpr (NW == 1) {
+    uint64_t* k2 = (uint64_t*)(p + at_k2);
+    double* v2 = (double*)(p + at_v2);
+    if (weights) {
+      SBD_CUDA(cub::DeviceRadixSort::SortPairs(p + at_t, tsort, x.keys, k2, x.vals, v2, x.m, 0, end_bit[0], st));
+      x.vals = v2;
+    } else {
+      SBD_CUDA(cub::DeviceRadixSort::SortKeys(p + at_t, tsort, x.keys, k2, x.m, 0, end_bit[0], st));
+    }
+    x.keys = k2;
+  } else {
+    uint64_t *ka = (uint64_t*)(p + at_k2), *kb = (uint64_t*)(p + at_k3);
+    int64_t *ia = (int64_t*)(p + at_v2), *ib = (int64_t*)(p + at_i3);
+    iota_kernel<<<gb, 256, 0, st>>>(ia, x.m);
+    SBD_CUDA(cudaGetLastError());
+    // least significant word first (each radix pass is stable)
+    for (int w = 0; w < NW; w++) {
+      if (end_bit[w] == 0) continue;
+      gather_word_kernel<<<gb, 256, 0, st>>>(x.keys, NW, w, ia, ka, x.m);
+      SBD_CUDA(cudaGetLastError());
+      SBD_CUDA(cub::DeviceRadixSort::SortPairs(p + at_t, tsort, ka, kb, ia, ib, x.m, 0, end_bit[w], st));
+      std::swap(ia, ib);
+    }
+    x.idx = ia;
+  }
   head_kernel<<<gb, 256, 0, st>>>(x.keys, NW, x.idx, x.head, x.m);
   SBD_CUDA(cudaGetLastError());
-  size_t ts = 0;
-  SBD_CUDA(cub::DeviceScan::InclusiveSum(nullptr, ts, x.head, x.seg, x.m, st));
-  void* tmp3 = x.alloc(ts);
-  SBD_CUDA(cub::DeviceScan::InclusiveSum(tmp3, ts, x.head, x.seg, x.m, st));
+  SBD_CUDA(cub::DeviceScan::InclusiveSum(p + at_t, tseg, x.head, x.seg, x.m, st));
   int64_t d = 0;
   SBD_CUDA(cudaMemcpyAsync(&d, x.seg + x.m - 1, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
   SBD_CUDA(cudaStreamSynchronize(st));
   x.distinct = (size_t)d;
 }
 
-void expand_space(sbdgpu_genop* g, const double* dW, double eps, int select, Expanded& x) {
+void expand_space(sbdgpu_genop* g, const double* dW, double eps, int select, bool weights, Expanded& x) {
   if (!g->ready) throw Error{SBDGPU_ERR_STATE, "no operator: call sbdgpu_genop_set_terms first"};
   switch (g->nw) {
-    case 1: expand_nw<1>(g, dW, eps, select, x); break;
-    case 2: expand_nw<2>(g, dW, eps, select, x); break;
-    default: expand_nw<4>(g, dW, eps, select, x); break;
+    case 1: expand_nw<1>(g, dW, eps, select, weights, x); break;
+    case 2: expand_nw<2>(g, dW, eps, select, weights, x); break;
+    default: expand_nw<4>(g, dW, eps, select, weights, x); break;
   }
 }
 
@@ -785,31 +1004,11 @@ int sbdgpu_genop_create(sbdgpu_genop** out, int device, int nwords, size_t nstat
     g->n = nstates;
     g->sign = sign ? 1 : 0;
     SBD_CUDA(cudaStreamCreateWithFlags(&g->base.stream, cudaStreamNonBlocking));
-    // the hash table: at least twice the states, a power of two
-    size_t slots = 1024;
-    while (slots < 2 * nstates) slots <<= 1;
-    std::vector<uint64_t> hk(slots * nwords, 0);
-    std::vector<int64_t> hi(slots, -1);
-    const uint64_t hmask = slots - 1;
-    for (size_t i = 0; i < nstates; i++) {
-      const uint64_t* w = &states[i * nwords];
-      uint64_t h = (nwords == 1 ? hash_state<1>(w) : nwords == 2 ? hash_state<2>(w) : hash_state<4>(w)) & hmask;
-      while (hi[h] >= 0) {
-        if (std::equal(w, w + nwords, &hk[h * nwords])) throw Error{SBDGPU_ERR_ARG, "repeated basis state"};
-        h = (h + 1) & hmask;
-      }
-      hi[h] = (int64_t)i;
-      std::memcpy(&hk[h * nwords], w, sizeof(uint64_t) * nwords);
+    switch (nwords) {
+      case 1: build_basis<1>(g, states); break;
+      case 2: build_basis<2>(g, states); break;
+      default: build_basis<4>(g, states); break;
     }
-    const size_t bytes = sizeof(uint64_t) * nstates * nwords;
-    g->states = (uint64_t*)sbdgpu::dev_alloc(bytes);
-    g->hkeys = (uint64_t*)sbdgpu::dev_alloc(sizeof(uint64_t) * hk.size());
-    g->hidx = (int64_t*)sbdgpu::dev_alloc(sizeof(int64_t) * slots);
-    g->hmask = hmask;
-    SBD_CUDA(cudaMemcpyAsync(g->states, states, bytes, cudaMemcpyHostToDevice, g->base.stream));
-    SBD_CUDA(cudaMemcpyAsync(g->hkeys, hk.data(), sizeof(uint64_t) * hk.size(), cudaMemcpyHostToDevice,
-                             g->base.stream));
-    SBD_CUDA(cudaMemcpyAsync(g->hidx, hi.data(), sizeof(int64_t) * slots, cudaMemcpyHostToDevice, g->base.stream));
     SBD_CUDA(cudaStreamSynchronize(g->base.stream));
   });
   if (rc != SBDGPU_OK) {  // a bad argument, or no memory on the device
@@ -903,7 +1102,7 @@ int sbdgpu_genop_ham_square(sbdgpu_genop* g, const double* W, double* res) {
     double* dW = v.add(g->n);
     SBD_CUDA(cudaMemcpyAsync(dW, W, sizeof(double) * g->n, cudaMemcpyHostToDevice, st));
     Expanded x;
-    expand_space(g, dW, 0.0, 0, x);
+    expand_space(g, dW, 0.0, 0, true, x);
     double* sums = v.add(x.distinct);
     SBD_CUDA(cudaMemsetAsync(sums, 0, sizeof(double) * x.distinct, st));
     const unsigned gb = (unsigned)std::min<size_t>((x.m + 255) / 256 + 1, 148 * 8);
@@ -922,7 +1121,7 @@ int sbdgpu_genop_expand(sbdgpu_genop* g, const double* W, double eps_hb, uint64_
     double* dW = v.add(g->n);
     SBD_CUDA(cudaMemcpyAsync(dW, W, sizeof(double) * g->n, cudaMemcpyHostToDevice, st));
     Expanded x;
-    expand_space(g, dW, eps_hb, 1, x);
+    expand_space(g, dW, eps_hb, 1, false, x);
     *n_out = x.distinct;
     if (!out) return;
     if (capacity < x.distinct) throw Error{SBDGPU_ERR_LIMIT, "output holds fewer states than the expanded basis"};
@@ -942,10 +1141,12 @@ void sbdgpu_genop_destroy(sbdgpu_genop* g) {
   cudaSetDevice(g->base.device);
   if (g->base.stream) cudaStreamSynchronize(g->base.stream);
   cudaFree(g->states);
-  cudaFree(g->hkeys);
-  cudaFree(g->hidx);
+  cudaFree(g->slots);
+  cudaFree(g->slot_of);
   cudaFree(g->buckets);
-  cudaFree(g->terms);
+  cudaFree(g->t_cre);
+  cudaFree(g->t_sgn);
+  cudaFree(g->t_coef);
   cudaFree(g->self_terms);
   cudaFree(g->hdiag);
   cudaFree(g->base.red);
