@@ -224,7 +224,7 @@ __device__ __forceinline__ void products(const unsigned char* vsub, uint32_t lbi
 struct MmaArgs {
   const double* C;
   double* S;
-  size_t nb, ia0;
+  size_t na, nb, ia0;
   int P, npair;
   const double* vf;
   const int64_t* a_off;
@@ -234,6 +234,7 @@ struct MmaArgs {
   const uint32_t* ent;
   int ngroup;
   int bulk;  // rows of S start on 16 bytes wherever a group of beta strings does
+  const double* Ja;  // [P][na]: the beta singles' Coulomb part as well (null: not)
 };
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -329,6 +330,14 @@ __device__ __forceinline__ void tiles(const MmaArgs& a, const unsigned char* vsu
 
 // One CTA per (source alpha string ja, M of its singles): alpha single 8 b + r
 // is row r of block b.
+//
+// With Ja, one more row per ja, with ja itself as its target, takes the beta
+// singles' Coulomb parts sum_jb s_b J_rs[ja] C[ja,jb]: its integrals are J_rs[ja].
+// As a pass of its own over the beta singles, between two transposes, that
+// took 7.3 ms at 144M determinants; the row adds 1.6 % to the products.  (The
+// alpha singles' Coulomb part J_pq[ib] C[ja,ib] as the value a row's sums start
+// from cost 20 ms more, 5.4 against 4.0 ms at 16M: its loads stall the warps and
+// take shared-memory wavefronts.  It stays a pass of its own.)
 template <int M>
 __global__ void __launch_bounds__(kMmaThreads) ab_mma_kernel(const MmaArgs a) {
   extern __shared__ __align__(128) unsigned char smem[];
@@ -339,13 +348,15 @@ __global__ void __launch_bounds__(kMmaThreads) ab_mma_kernel(const MmaArgs a) {
   double* crow = stage + (size_t)(blockDim.x >> 5) * M * 16;                           // [nb + 1]
   const size_t ja = blockIdx.x;
   const int64_t k0 = a.a_off[ja] + (int64_t)blockIdx.y * M;
-  const int count = (int)min((int64_t)M, a.a_off[ja + 1] - k0);
-  if (count <= 0) return;
+  const int singles = (int)min((int64_t)M, a.a_off[ja + 1] - k0);  // negative past the last ones
+  if (singles < 0) return;
+  const int count = singles + (a.Ja && singles < M ? 1 : 0);  // the row of ja itself comes after its last single
+  if (count == 0) return;
   if (threadIdx.x < M) {
     const int g = threadIdx.x;
-    const bool on = g < count;
-    tgt[g] = on ? (int)((int64_t)a.a_idx[k0 + g] - (int64_t)a.ia0) : -1;
-    neg[g] = on ? a.a_info[k0 + g] & 0x80000000u : 0u;
+    tgt[g] = g < singles ? (int)((int64_t)a.a_idx[k0 + g] - (int64_t)a.ia0) : g < count ? (int)ja : -1;
+    const uint32_t info = g < singles ? a.a_info[k0 + g] : 0u;
+    neg[g] = info & 0x80000000u;
   }
   for (size_t i = threadIdx.x; i <= a.nb; i += blockDim.x) crow[i] = i < a.nb ? a.C[ja * a.nb + i] : 0.0;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
@@ -353,9 +364,13 @@ __global__ void __launch_bounds__(kMmaThreads) ab_mma_kernel(const MmaArgs a) {
   for (int c = 0; c < M / 4; c++) {
     const int place = 4 * c + (lane & 3);
     const int g = M == 16 ? 8 * (place & 1) + (place >> 1) : place;
-    const double* vrow = g < count ? a.vf + (size_t)((a.a_info[k0 + g] >> 12) & 0xFFFu) * a.P : nullptr;
+    const double* vrow = g < singles ? a.vf + (size_t)((a.a_info[k0 + g] >> 12) & 0xFFFu) * a.P
+                         : g < count ? a.Ja + ja
+                                     : nullptr;
+    const size_t step = g < singles ? 1 : a.na;
     for (int o = warp * 8 + (lane >> 2); o < a.npair; o += nwarp * 8)
-      *reinterpret_cast<double*>(vsub + store_offset<M>(o, place)) = vrow ? __ldg(&vrow[folded_pair(o)]) : 0.0;
+      *reinterpret_cast<double*>(vsub + store_offset<M>(o, place)) =
+          vrow ? __ldg(&vrow[(size_t)folded_pair(o) * step]) : 0.0;
   }
   __syncthreads();
   double* mine = stage + (size_t)warp * M * 16;
@@ -376,14 +391,28 @@ size_t mma_smem(const sbdgpu_ctx* c, int m, int threads) {
 }
 
 template <int M>
-void launch_mma(sbdgpu_ctx* c, const double* C, double* S, const AlphaSingles& as, int nt) {
+void launch_mma(sbdgpu_ctx* c, const double* C, double* S, const AlphaSingles& as, int nt, bool beta_j) {
   const SpinTables& tb = c->tab[1];
-  const dim3 grid((unsigned)c->na, (unsigned)((as.max_s + M - 1) / M));
+  const dim3 grid((unsigned)c->na, (unsigned)((as.max_s + (beta_j ? 1 : 0) + M - 1) / M));
   if (grid.y == 0) return;
   // whole lines of sigma for the copy engine: 16-byte starts
   const int bulk = c->nb % 2 == 0 && ((uintptr_t)S & 15) == 0;
-  const MmaArgs a{C,      S,      c->nb,   as.ia0,      c->P,        c->L * (c->L - 1) / 2, c->vf,
-                  as.off, as.idx, as.info, tb.tile_grp, tb.tile_ent, (int)tb.n_tile_grp,    bulk};
+  const MmaArgs a{C,
+                  S,
+                  c->na,
+                  c->nb,
+                  as.ia0,
+                  c->P,
+                  c->L * (c->L - 1) / 2,
+                  c->vf,
+                  as.off,
+                  as.idx,
+                  as.info,
+                  tb.tile_grp,
+                  tb.tile_ent,
+                  (int)tb.n_tile_grp,
+                  bulk,
+                  beta_j ? c->ja : nullptr};
   allow_dynamic_smem(reinterpret_cast<const void*>(ab_mma_kernel<M>), c->device);
   ab_mma_kernel<M><<<grid, nt, mma_smem(c, M, nt), c->stream>>>(a);
   SBD_CUDA(cudaGetLastError());
@@ -434,13 +463,15 @@ int ab_mma_group(const sbdgpu_ctx* c, int want, size_t budget) {
 }
 
 // The alpha-beta term by tiles, m alpha singles per CTA, nt threads (0: the
-// default).  Default threads: the fewest of 256, 512, 1024 that put 24 warps
+// default); beta_j: the beta singles' Coulomb part as well (whole vectors
+// only).  Default threads: the fewest of 256, 512, 1024 that put 24 warps
 // on an SM beside the shared memory they need, else the number that puts most
 // there; fewer while the warps outnumber the groups.  Alpha-beta ms by
 // threads: 16M determinants 6.0 (256), 4.0 (512), 4.9 (768); 1501 x 803
 // strings 0.40 (128), 0.34 (256), 0.36 (512); 144M 107 (512), 101 (640),
 // 93 (768).
-void ab_mma(sbdgpu_ctx* c, const double* C, double* S, const AlphaSingles& as, int m, int nt, size_t budget) {
+void ab_mma(sbdgpu_ctx* c, const double* C, double* S, const AlphaSingles& as, int m, int nt, size_t budget,
+            bool beta_j) {
   if (nt == 0) {
     int best = 0;
     for (int t : {256, 512, 768, 1024}) {
@@ -457,9 +488,9 @@ void ab_mma(sbdgpu_ctx* c, const double* C, double* S, const AlphaSingles& as, i
   }
   while (nt > 128 && mma_smem(c, m, nt) > budget) nt -= 128;  // a tuned number: the stages beside the row of C
   if (m == 16)
-    launch_mma<16>(c, C, S, as, nt);
+    launch_mma<16>(c, C, S, as, nt, beta_j);
   else
-    launch_mma<8>(c, C, S, as, nt);
+    launch_mma<8>(c, C, S, as, nt, beta_j);
 }
 
 void preload_ab_mma(int device) {

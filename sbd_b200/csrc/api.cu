@@ -149,8 +149,7 @@ void sigma_ref_convention(sbdgpu_ctx* c, const double* dC, double* dS, int preci
   sbdgpu::ensure_scratch(c);
   if (precision != SBDGPU_FP64) sbdgpu::ensure_fp32(c);
   SBD_CUDA(cudaEventRecord(c->ev[4], c->stream));
-  SBD_CUDA(cudaMemcpyAsync(c->io_a, dC, sizeof(double) * c->N, cudaMemcpyDeviceToDevice, c->stream));
-  sbdgpu::apply_phase(c, c->io_a);
+  sbdgpu::phase_copy(c, dC, c->io_a);
   if (precision != SBDGPU_FP64) {
     if (!c->io32) c->io32 = (float*)sbdgpu::dev_alloc(sizeof(float) * 2 * c->N);
     float* c32 = c->io32;
@@ -798,6 +797,7 @@ void sbdgpu_destroy(sbdgpu_ctx* c) {
   sbdgpu::free_dense_same(c);
   sbdgpu::free_rdm_tables(c);
   sbdgpu::free_ozaki(c);
+  sbdgpu::free_dense_fp64(c);
   sbdgpu::free_tables(c->tab[0]);
   sbdgpu::free_tables(c->tab[1]);
   cudaFree(c->astr); cudaFree(c->bstr); cudaFree(c->h1); cudaFree(c->vf); cudaFree(c->ja); cudaFree(c->jb);

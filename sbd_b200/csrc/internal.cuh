@@ -124,6 +124,10 @@ struct sbdgpu_ctx {
   } oz;
   // alpha-beta launch shape of the FP64 sigma (0: the shared-memory heuristic)
   int ab_group = 0, ab_threads = 0;
+  // dense string-only same-spin operators of small bases (same_dense.cu), one
+  // allocation at dense[0]; row strides
+  double* dense[2] = {nullptr, nullptr};
+  size_t dense_ld[2] = {0, 0};
   // RDM tables: beta singles grouped by excitation, bra row of every alpha single
   int64_t* rdm_bin_off = nullptr;
   uint32_t* rdm_bin_ent = nullptr;
@@ -160,6 +164,7 @@ void free_tables(SpinTables& t);
 void build_j_tables(sbdgpu_ctx* c);
 void compute_hii(sbdgpu_ctx* c);
 void apply_phase(sbdgpu_ctx* c, double* v);
+void phase_copy(sbdgpu_ctx* c, const double* in, double* out);  // out = phase * in, whole vectors
 void apply_phase_rows(sbdgpu_ctx* c, double* v, size_t r0, size_t nrows);  // v: rows r0.. of a vector
 template <typename T>
 void transpose(const T* in, T* out, size_t rows, size_t cols, cudaStream_t s);
@@ -200,13 +205,23 @@ struct AlphaSingles {
 // ab_mma.cu: the alpha-beta term on the FP64 tensor pipe
 void build_ab_tiles(sbdgpu_ctx* c, SpinTables& t, const std::vector<uint64_t>& strs);
 int ab_mma_group(const sbdgpu_ctx* c, int want, size_t budget);
-void ab_mma(sbdgpu_ctx* c, const double* C, double* S, const AlphaSingles& as, int m, int nt, size_t budget);
+void ab_mma(sbdgpu_ctx* c, const double* C, double* S, const AlphaSingles& as, int m, int nt, size_t budget,
+            bool beta_j);
+// same_dense.cu: the FP64 same-spin terms as one dense product
+bool dense_same_spin(const sbdgpu_ctx* c);
+void ensure_dense_fp64(sbdgpu_ctx* c);
+void free_dense_fp64(sbdgpu_ctx* c);
+void same_spin_dense_fp64(sbdgpu_ctx* c, const double* C, double* S);
+void preload_same_dense(int device);
 void preload_ab_mma(int device);
 // ozaki.cu: the FP64 same-spin terms as exact INT8 products
 bool ensure_ozaki(sbdgpu_ctx* c);
 void free_ozaki(sbdgpu_ctx* c);
 bool use_ozaki(sbdgpu_ctx* c);
-bool same_spin_ozaki_fp64(sbdgpu_ctx* c, const double* C, double* S, double* ct, double* st, bool events);
+bool same_spin_ozaki_fp64(sbdgpu_ctx* c, const double* C, double* S, double* ct, double* st, bool events,
+                          bool beta_j);
+// sigma.cu: S = hii C + the alpha singles' Coulomb part
+void alpha_coulomb(sbdgpu_ctx* c, const double* C, double* S);
 // genop.cu: record an error message on a generic-path object
 void genop_set_error(sbdgpu_genop* g, const std::string& msg);
 void occupation(sbdgpu_ctx* c, const double* dW, double* dens);

@@ -92,8 +92,7 @@ extern "C" int sbdgpu_sigma_device_noalloc(sbdgpu_ctx* c, const double* dC, doub
     double* io = base;
     double* ct = base + kNoAllocMaxDets;
     double* st = base + 2 * kNoAllocMaxDets;
-    SBD_CUDA(cudaMemcpyAsync(io, dC, sizeof(double) * c->N, cudaMemcpyDeviceToDevice, c->stream));
-    sbdgpu::apply_phase(c, io);
+    sbdgpu::phase_copy(c, dC, io);
     sbdgpu::sigma_fp64_prepared(c, io, dS, ct, st);
     sbdgpu::apply_phase(c, dS);
     SBD_CUDA(cudaStreamSynchronize(c->stream));

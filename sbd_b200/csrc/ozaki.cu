@@ -235,12 +235,10 @@ __global__ void __launch_bounds__(kT) dense_h0_kernel(size_t n, const int64_t* _
   for (int64_t k = d_off[row] + threadIdx.x; k < d_off[row + 1]; k += kT) Hr[d_idx[k]] = d_val[k];
 }
 
-// S[row][col] (=) [hii C] + sum over the bra's singles of s J_pq[col] C[ket][col] (FP64);
+// S[row][col] = sum over the bra's singles of s J_pq[col] C[ket][col] (FP64);
 // two consecutive columns per thread (ncols even)
-template <bool kWithDiag>
 __global__ void __launch_bounds__(kT) jsingles64_kernel(const double* __restrict__ C, double* __restrict__ S,
-                                                       size_t ncols, const double* __restrict__ hii,
-                                                       const int64_t* __restrict__ s_off,
+                                                       size_t ncols, const int64_t* __restrict__ s_off,
                                                        const int32_t* __restrict__ s_idx,
                                                        const uint32_t* __restrict__ s_info,
                                                        const double* __restrict__ J) {
@@ -248,11 +246,6 @@ __global__ void __launch_bounds__(kT) jsingles64_kernel(const double* __restrict
   const size_t col = 2 * ((size_t)blockIdx.y * kT + threadIdx.x);
   if (col >= ncols) return;
   double2 acc = {0.0, 0.0};
-  if (kWithDiag) {
-    const double2 h = *reinterpret_cast<const double2*>(hii + row * ncols + col);
-    const double2 x = *reinterpret_cast<const double2*>(C + row * ncols + col);
-    acc = {h.x * x.x, h.y * x.y};
-  }
   const int64_t k1 = s_off[row + 1];
 #pragma unroll 4
   for (int64_t k = s_off[row]; k < k1; k++) {
@@ -385,14 +378,15 @@ bool use_ozaki(sbdgpu_ctx* c) {
   return ensure_ozaki(c);
 }
 
-// sigma (FP64) = hii C + same-spin terms (the alpha-beta term is added
-// after); ct, st: FP64 scratch of N each.  Returns false, having written
+// sigma (FP64) = hii C + same-spin terms (the alpha-beta term is added after);
+// beta_j: the beta singles' Coulomb part too (else the alpha-beta tiles bring
+// it); ct, st: FP64 scratch of N each.  Returns false, having written
 // nothing, when cuBLAS refuses the INT8 products (the caller then uses the
 // rows kernels, and this context stops asking).
-bool same_spin_ozaki_fp64(sbdgpu_ctx* c, const double* C, double* S, double* ct, double* st, bool events) {
+bool same_spin_ozaki_fp64(sbdgpu_ctx* c, const double* C, double* S, double* ct, double* st, bool events,
+                          bool beta_j) {
   cudaStream_t s = c->stream;
   const size_t na = c->na, nb = c->nb, N = c->N;
-  const SpinTables& ta = c->tab[0];
   const SpinTables& tb = c->tab[1];
   cublasHandle_t h = static_cast<cublasHandle_t>(c->blas);
   if (((uintptr_t)C | (uintptr_t)S) & 15) return false;  // the kernels move pairs of doubles
@@ -412,8 +406,7 @@ bool same_spin_ozaki_fp64(sbdgpu_ctx* c, const double* C, double* S, double* ct,
       c->oz.failed = true;
       return false;
     }
-  jsingles64_kernel<true><<<dim3((unsigned)na, (unsigned)((nb + 2 * kT - 1) / (2 * kT))), kT, 0, s>>>(
-      C, S, nb, c->hii, ta.s_off, ta.s_idx, ta.s_info, c->jb);
+  alpha_coulomb(c, C, S);
   crt_add_kernel<<<(unsigned)na, kT, 0, s>>>(c->oz.prod, na, nb, c->oz.h0e[0], c->oz.cte, S);
   SBD_CUDA(cudaGetLastError());
   if (events) SBD_CUDA(cudaEventRecord(c->ev[1], s));
@@ -423,10 +416,13 @@ bool same_spin_ozaki_fp64(sbdgpu_ctx* c, const double* C, double* S, double* ct,
                  c->oz.cr + (size_t)l * N, (int)nb, c->oz.prod + (size_t)l * N, (int)nb))
       throw Error{SBDGPU_ERR_CUDA, "INT8 product refused after the alpha products ran"};
   crt_add_kernel<<<(unsigned)na, kT, 0, s>>>(c->oz.prod, na, nb, c->oz.ce, c->oz.h0e[1], S);
-  jsingles64_kernel<false><<<dim3((unsigned)nb, (unsigned)((na + 2 * kT - 1) / (2 * kT))), kT, 0, s>>>(
-      ct, st, na, nullptr, tb.s_off, tb.s_idx, tb.s_info, c->ja);
   SBD_CUDA(cudaGetLastError());
-  transpose_add(st, S, nb, na, s);
+  if (beta_j) {
+    jsingles64_kernel<<<dim3((unsigned)nb, (unsigned)((na + 2 * kT - 1) / (2 * kT))), kT, 0, s>>>(
+        ct, st, na, tb.s_off, tb.s_idx, tb.s_info, c->ja);
+    SBD_CUDA(cudaGetLastError());
+    transpose_add(st, S, nb, na, s);
+  }
   if (events) SBD_CUDA(cudaEventRecord(c->ev[2], s));
   return true;
 }

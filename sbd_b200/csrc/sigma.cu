@@ -22,6 +22,7 @@
 // singles (sliced ELL, coalesced) once per group, and adds each group's
 // contributions to sigma rows ia with atomics.
 #include <algorithm>
+#include <type_traits>
 #include <vector>
 
 #include "internal.cuh"
@@ -157,6 +158,62 @@ __global__ void __launch_bounds__(kRowsThreads) rows_vec_kernel(
     for (int u = 0; u < W; u++) acc[u] += v * cr[u];
   }
   *reinterpret_cast<V*>(S + (size_t)blockIdx.x * ncols + col) = VT::make(acc);
+}
+
+// S[row][col] = hii C + sum over the bra's alpha singles of s J_pq[col] C[ket][col];
+// V consecutive columns per thread (V = 2: ncols even, 16-byte aligned rows)
+template <int V>
+__global__ void __launch_bounds__(kRowsThreads) alpha_coulomb_kernel(const double* __restrict__ C,
+                                                                    double* __restrict__ S, size_t ncols,
+                                                                    const double* __restrict__ hii,
+                                                                    const int64_t* __restrict__ s_off,
+                                                                    const int32_t* __restrict__ s_idx,
+                                                                    const uint32_t* __restrict__ s_info,
+                                                                    const double* __restrict__ J) {
+  using Vec = typename std::conditional<V == 2, double2, double>::type;
+  __shared__ int2 ent[kRowsThreads];  // the row's singles: ket, integral row and sign
+  const size_t row = blockIdx.x;
+  const size_t col = V * ((size_t)blockIdx.y * kRowsThreads + threadIdx.x);
+  const bool on = col < ncols;
+  const auto get = [&](const double* p, double(&x)[V]) {
+    const Vec v = __ldg(reinterpret_cast<const Vec*>(p));
+    if constexpr (V == 2) {
+      x[0] = v.x;
+      x[1] = v.y;
+    } else {
+      x[0] = v;
+    }
+  };
+  double acc[V], h[V], x[V];
+  if (on) {
+    get(hii + row * ncols + col, h);
+    get(C + row * ncols + col, x);
+#pragma unroll
+    for (int u = 0; u < V; u++) acc[u] = h[u] * x[u];
+  }
+  const int64_t k0 = s_off[row], k1 = s_off[row + 1];
+  for (int64_t kb = k0; kb < k1; kb += kRowsThreads) {
+    const int n = (int)min((int64_t)kRowsThreads, k1 - kb);
+    __syncthreads();
+    if ((int)threadIdx.x < n) ent[threadIdx.x] = make_int2(s_idx[kb + threadIdx.x], (int)s_info[kb + threadIdx.x]);
+    __syncthreads();
+    if (!on) continue;
+#pragma unroll 8
+    for (int k = 0; k < n; k++) {
+      const int2 e = ent[k];
+      double jv[V], cv[V];
+      get(J + (size_t)(((uint32_t)e.y >> 12) & 0xFFFu) * ncols + col, jv);
+      get(C + (size_t)e.x * ncols + col, cv);
+      const double sg = e.y < 0 ? -1.0 : 1.0;
+#pragma unroll
+      for (int u = 0; u < V; u++) acc[u] = fma(sg * jv[u], cv[u], acc[u]);
+    }
+  }
+  if (!on) return;
+  if constexpr (V == 2)
+    *reinterpret_cast<double2*>(S + row * ncols + col) = make_double2(acc[0], acc[1]);
+  else
+    S[row * ncols + col] = acc[0];
 }
 
 bool aligned16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
@@ -357,7 +414,7 @@ namespace {
 // one row of C.  FP64 groups of 16 and 8 go to the tile kernel where the basis
 // has tiles; at groups of 4 and fewer a product would be half empty.
 template <typename T>
-void alpha_beta(sbdgpu_ctx* c, const T* C, T* S, const T* vf, const AlphaSingles& as) {
+void alpha_beta(sbdgpu_ctx* c, const T* C, T* S, const T* vf, const AlphaSingles& as, bool beta_j = false) {
   int dev_smem = 0;
   SBD_CUDA(cudaDeviceGetAttribute(&dev_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
   size_t budget = (size_t)dev_smem - 1024;
@@ -368,7 +425,7 @@ void alpha_beta(sbdgpu_ctx* c, const T* C, T* S, const T* vf, const AlphaSingles
   const int g = tuned ? c->ab_group : 0, nt = tuned ? c->ab_threads : 0;
   if constexpr (sizeof(T) == 8)
     if (const int m = ab_mma_group(c, g, budget)) {
-      ab_mma(c, C, S, as, m, nt, budget);
+      ab_mma(c, C, S, as, m, nt, budget, beta_j);
       return;
     }
   if ((g == 0 || g == 16) && ab_smem<T, 16>(nb, P) <= budget)
@@ -385,6 +442,13 @@ void alpha_beta(sbdgpu_ctx* c, const T* C, T* S, const T* vf, const AlphaSingles
     throw Error{SBDGPU_ERR_LIMIT, "alpha-beta kernel: one beta row and integral row exceed shared memory"};
 }
 
+// Whether the FP64 alpha-beta term of this context runs on tiles.
+bool uses_tiles(const sbdgpu_ctx* c) {
+  int dev_smem = 0;
+  SBD_CUDA(cudaDeviceGetAttribute(&dev_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
+  return ab_mma_group(c, c->ab_group, (size_t)dev_smem - 1024) > 0;
+}
+
 // The full kernel sequence of one sigma on given scratch (ct, st: na*nb of T).
 template <typename T>
 void sigma_launch(sbdgpu_ctx* c, const T* C, T* S, T* ct, T* st, const T* ja, const T* jb, const T* vf,
@@ -393,6 +457,17 @@ void sigma_launch(sbdgpu_ctx* c, const T* C, T* S, T* ct, T* st, const T* ja, co
   const SpinTables& ta = c->tab[0];
   const SpinTables& tb = c->tab[1];
   if (events) SBD_CUDA(cudaEventRecord(c->ev[0], s));
+  if constexpr (sizeof(T) == 8) {
+    if (c->dense[0] && c->oz.mode == 0 && uses_tiles(c)) {
+      alpha_coulomb(c, C, S);
+      same_spin_dense_fp64(c, C, S);
+      if (events) SBD_CUDA(cudaEventRecord(c->ev[1], s));  // both spins at once: the second phase is empty
+      if (events) SBD_CUDA(cudaEventRecord(c->ev[2], s));
+      alpha_beta(c, C, S, vf, AlphaSingles{ta.s_off, ta.s_idx, ta.s_info, ta.max_s, 0}, true);
+      if (events) SBD_CUDA(cudaEventRecord(c->ev[3], s));
+      return;
+    }
+  }
   launch_rows<T, true>(C, S, c->na, c->nb, c->hii, ta, jb, s);
   if (events) SBD_CUDA(cudaEventRecord(c->ev[1], s));
   transpose(C, ct, c->na, c->nb, s);
@@ -429,7 +504,24 @@ void preload_fp64_sigma(int device) {
   preload_ab<2>(device);
   preload_ab<1>(device);
   preload_ab_mma(device);
+  preload_same_dense(device);
+  SBD_CUDA(cudaFuncGetAttributes(&fa, reinterpret_cast<const void*>(alpha_coulomb_kernel<1>)));
+  SBD_CUDA(cudaFuncGetAttributes(&fa, reinterpret_cast<const void*>(alpha_coulomb_kernel<2>)));
   preload_fp64_sigma_misc();
+}
+
+// S = hii C + sum over the alpha singles of s J_pq[ib] C[ja,ib] (V = 2 where
+// the rows allow 16-byte loads)
+void alpha_coulomb(sbdgpu_ctx* c, const double* C, double* S) {
+  const SpinTables& t = c->tab[0];
+  const bool vec = c->nb % 2 == 0 && aligned16(C) && aligned16(S);
+  const unsigned per = kRowsThreads * (vec ? 2 : 1);
+  const dim3 g((unsigned)c->na, (unsigned)((c->nb + per - 1) / per));
+  if (vec)
+    alpha_coulomb_kernel<2><<<g, kRowsThreads, 0, c->stream>>>(C, S, c->nb, c->hii, t.s_off, t.s_idx, t.s_info, c->jb);
+  else
+    alpha_coulomb_kernel<1><<<g, kRowsThreads, 0, c->stream>>>(C, S, c->nb, c->hii, t.s_off, t.s_idx, t.s_info, c->jb);
+  SBD_CUDA(cudaGetLastError());
 }
 
 void sigma_fp64(sbdgpu_ctx* c, const double* C, double* S) {
@@ -440,9 +532,10 @@ void sigma_fp64(sbdgpu_ctx* c, const double* C, double* S) {
     return;
   }
   ensure_scratch(c);
-  if (use_ozaki(c) && same_spin_ozaki_fp64(c, C, S, c->ct, c->st, true)) {
+  const bool tiles = uses_tiles(c);
+  if (use_ozaki(c) && same_spin_ozaki_fp64(c, C, S, c->ct, c->st, true, !tiles)) {
     const SpinTables& ta = c->tab[0];
-    alpha_beta<double>(c, C, S, c->vf, AlphaSingles{ta.s_off, ta.s_idx, ta.s_info, ta.max_s, 0});
+    alpha_beta<double>(c, C, S, c->vf, AlphaSingles{ta.s_off, ta.s_idx, ta.s_info, ta.max_s, 0}, tiles);
     SBD_CUDA(cudaEventRecord(c->ev[3], c->stream));
     return;
   }
@@ -531,8 +624,7 @@ void sigma_rows_fp64(sbdgpu_ctx* c, const double* dC, double* S, size_t r0, size
   cudaStream_t s = c->stream;
   const SpinTables& ta = c->tab[0];
   const SpinTables& tb = c->tab[1];
-  SBD_CUDA(cudaMemcpyAsync(c->io_a, dC, sizeof(double) * c->N, cudaMemcpyDeviceToDevice, s));
-  apply_phase(c, c->io_a);
+  phase_copy(c, dC, c->io_a);
   if (nrows == 0) return;
   launch_rows<double, true>(c->io_a, S, nrows, nb, c->hii, ta, c->jb, s, r0, nb);
   transpose(c->io_a + r0 * nb, c->ct, nrows, nb, s);

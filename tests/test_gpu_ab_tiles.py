@@ -64,3 +64,38 @@ def test_wide_orbital_range():
 def test_repeated_strings_keep_the_gather_kernel():
     ints, a, b = _system(8, 3, 3, 20, 30, 9)
     _check(ints, a, np.concatenate([b, b[:3]]))
+
+
+@pytest.mark.parametrize("na,nb", [(1, 70), (33, 31), (64, 64), (65, 126), (126, 17)])
+def test_dense_same_spin_product_at_tile_edges(na, nb):
+    # full or nearly full spaces of 9 orbitals (126 strings of 4 electrons): the dense product of same_dense.cu,
+    # odd and even rows, 32- and 64-wide tiles; the rows kernels as the second shape
+    ints, a, b = _system(9, 4, 4, na, nb, 40 + na)
+    ctx = sbd_b200.context_from_integrals(ints, a, b)
+    C = np.random.default_rng(4).normal(size=ctx.n)
+    ref = oracle.Oracle(9, a, b, ints.ecore, ints.h, ints.eri).sigma(C)
+    for method in (0, 1):
+        ctx.set_fp64_same_spin(method)
+        assert np.abs(ctx.sigma(C) - ref).max() <= TOL * np.abs(ref).max(), method
+    ctx.close()
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_non_finite_input_stays_where_the_operator_takes_it(bad):
+    ints, a, b = _system(9, 4, 4, 60, 61, 8)
+    C = np.random.default_rng(5).normal(size=(60, 61))
+    C[7, 11] = bad
+    orc = oracle.Oracle(9, a, b, ints.ecore, ints.h, ints.eri)
+    e = np.zeros((60, 61))
+    e[7, 11] = 1.0
+    reached = orc.sigma(e.ravel()) != 0.0
+    ctx = sbd_b200.context_from_integrals(ints, a, b)
+    s = ctx.sigma(C)
+    assert not np.isfinite(s[reached]).any()
+    ra = np.array([bin(int(x ^ a[7])).count("1") for x in a])
+    rb = np.array([bin(int(x ^ b[11])).count("1") for x in b])
+    unreached = (ra[:, None] + rb[None, :] > 4).ravel()  # more than two excitations away
+    assert unreached.any() and np.isfinite(s[unreached]).all()
+    ref = orc.sigma(np.where(np.isfinite(C), C, 0.0).ravel())
+    assert np.abs(s - ref)[unreached].max() <= TOL * np.abs(ref).max()
+    ctx.close()
