@@ -29,6 +29,11 @@ void* dev_alloc(size_t bytes) {
   return p;
 }
 
+void Arena::commit() {
+  base_ = (char*)dev_alloc(total_);
+  for (auto& x : slots_) *x.first = base_ + x.second;
+}
+
 // The dynamic shared-memory limit of a kernel is one attribute per
 // (function, device), shared by every host thread.  Setting it before each
 // launch to that launch's size lets concurrent contexts undercut each other
@@ -173,6 +178,19 @@ void sigma_ref_convention(sbdgpu_ctx* c, const double* dC, double* dS, int preci
     throw Error{SBDGPU_ERR_CUDA, "tensor-core alpha-beta kernel: completion wait timed out"};
 }
 
+// k doubles from the device, waiting for the stream
+void read_back(double* out, const double* dev, int k, cudaStream_t s) {
+  SBD_CUDA(cudaMemcpyAsync(out, dev, sizeof(double) * k, cudaMemcpyDeviceToHost, s));
+  SBD_CUDA(cudaStreamSynchronize(s));
+}
+
+sbdgpu::RitzCoef ritz_coef(const double* u, int k, double e0) {
+  sbdgpu::RitzCoef r{};
+  std::copy(u, u + k, r.u);
+  r.e0 = e0;
+  return r;
+}
+
 // Mixed-precision Davidson: FP32 basis and FP32 sigma; FP64 dot products,
 // projected matrix, Ritz vector, residual, preconditioned correction and
 // Gram-Schmidt; the energy is the FP64 Rayleigh quotient <W|H W> from one FP64
@@ -198,35 +216,10 @@ void davidson_mixed(sbdgpu_ctx* c, const sbdgpu_opts* o, double* W, double* R, d
   sbdgpu::ensure_fp32(c);
   std::vector<float*> C(nb, nullptr), HC(nb, nullptr);
   double* X = nullptr;  // FP64 correction vector
-  struct Free {
-    std::vector<float*>* a;
-    std::vector<float*>* b;
-    double** x;
-    cudaStream_t s;
-    ~Free() {
-      cudaStreamSynchronize(s);  // an error path may leave kernels queued on these buffers
-      for (auto p : *a) cudaFree(p);
-      for (auto p : *b) cudaFree(p);
-      cudaFree(*x);
-    }
-  } guard{&C, &HC, &X, st};
-  for (int k = 0; k < nb; k++) {
-    C[k] = (float*)sbdgpu::dev_alloc(sizeof(float) * n);
-    HC[k] = (float*)sbdgpu::dev_alloc(sizeof(float) * n);
-  }
-  X = (double*)sbdgpu::dev_alloc(sizeof(double) * n);
   // Olsen's correction needs P applied to the Ritz vector as well
   const bool olsen = o->precond == SBDGPU_PRECOND_OLSEN;
   double* Y = nullptr;
-  struct FreeY {
-    double** y;
-    cudaStream_t s;
-    ~FreeY() {
-      cudaStreamSynchronize(s);
-      cudaFree(*y);
-    }
-  } guard_y{&Y, st};
-  if (olsen) Y = (double*)sbdgpu::dev_alloc(sizeof(double) * n);
+  double *part = nullptr, *scal = nullptr;  // block sums; overlaps and the residual norm
   const double eps_reg = 1.0e-12;
   std::vector<double> H(nb * nb, 0.0), U(nb * nb, 0.0), E(nb, 0.0);
   std::vector<double> step_times;
@@ -241,21 +234,21 @@ void davidson_mixed(sbdgpu_ctx* c, const sbdgpu_opts* o, double* W, double* R, d
   std::vector<float*> T(keep, nullptr), TH(keep, nullptr);
   std::vector<double> u_last(nb, 0.0);  // Ritz coefficients of the previous step
   int u_last_len = 0, u_last_cycle = -1;
-  struct FreeT {
-    std::vector<float*>* a;
-    std::vector<float*>* b;
-    cudaStream_t s;
-    ~FreeT() {
-      cudaStreamSynchronize(s);
-      for (auto p : *a) cudaFree(p);
-      for (auto p : *b) cudaFree(p);
-    }
-  } guard_t{&T, &TH, st};
+  sbdgpu::Arena arena(st);
+  for (int k = 0; k < nb; k++) {
+    arena.add(&C[k], n);
+    arena.add(&HC[k], n);
+  }
   if (keep > 1)
     for (int j = 0; j < keep; j++) {
-      T[j] = (float*)sbdgpu::dev_alloc(sizeof(float) * n);
-      TH[j] = (float*)sbdgpu::dev_alloc(sizeof(float) * n);
+      arena.add(&T[j], n);
+      arena.add(&TH[j], n);
     }
+  arena.add(&X, n);
+  if (olsen) arena.add(&Y, n);
+  arena.add(&part, 32 * sbdgpu::kKrylovBlocks);
+  arena.add(&scal, 64);
+  arena.commit();
   int kept = 0;  // basis vectors (with their sigma) carried into the next cycle
   // With Ritz vectors carried across restarts in FP32, one classical
   // Gram-Schmidt pass leaves the basis drifting out of orthogonality over the
@@ -268,27 +261,23 @@ void davidson_mixed(sbdgpu_ctx* c, const sbdgpu_opts* o, double* W, double* R, d
   double tol_learned_cycle = 1e300;
   double tol_thick_cycle = 1e300;
   auto add_correction = [&](int into, double e0) {
+    const double* diagonal_from = R;  // the diagonal correction goes with the first pass
     if (use_learned) {
       sbdgpu::learned_precondition(c, R, e0, eps_reg, X);
-    } else {
+      diagonal_from = nullptr;
+    } else if (olsen) {
       sbdgpu::precondition(R, c->hii, e0, eps_reg, X, n, st);
-      if (olsen) {
-        // t = P r - eps P w with eps = <w|P r> / <w|P w>: the correction is
-        // P-orthogonal to the Ritz vector w, so it does not fall back onto w
-        // where P r is nearly parallel to it
-        sbdgpu::precondition(W, c->hii, e0, eps_reg, Y, n, st);
-        const double wpw = sbdgpu::dot(c, W, Y, n);
-        if (std::fabs(wpw) > 0.0) sbdgpu::axpy(X, Y, -sbdgpu::dot(c, W, X, n) / wpw, n, st);
-      }
+      // t = P r - eps P w with eps = <w|P r> / <w|P w>: the correction is
+      // P-orthogonal to the Ritz vector w, so it does not fall back onto w
+      // where P r is nearly parallel to it
+      sbdgpu::precondition(W, c->hii, e0, eps_reg, Y, n, st);
+      const double wpw = sbdgpu::dot(c, W, Y, n);
+      if (std::fabs(wpw) > 0.0) sbdgpu::axpy(X, Y, -sbdgpu::dot(c, W, X, n) / wpw, n, st);
+      diagonal_from = nullptr;
     }
-    for (int pass = 0; pass < gs_passes; pass++)
-      for (int kb = 0; kb < into; kb++) {
-        double olap = sbdgpu::dot_f(c, C[kb], X, C[kb], n);  // <X|C_kb> with X in FP64
-        sbdgpu::axpy_df(X, C[kb], -olap, n, st);
-      }
-    double nc = std::sqrt(sbdgpu::dot(c, X, X, n));
-    sbdgpu::scale(X, 1.0 / nc, n, st);
-    sbdgpu::convert(X, C[into], n, st);
+    // <X|C_kb> with X in FP64
+    sbdgpu::krylov_correction<float>(diagonal_from, c->hii, e0, nullptr, X, C.data(), into, C[into], n, gs_passes, part,
+                                     st);
   };
   for (int it = 0; it < o->max_it && cont; it++) {
     int ib0 = kept;
@@ -300,18 +289,16 @@ void davidson_mixed(sbdgpu_ctx* c, const sbdgpu_opts* o, double* W, double* R, d
         sbdgpu::sigma_fp32_tc(c, C[ib], HC[ib]);
       else
         sbdgpu::sigma_fp32(c, C[ib], HC[ib]);
-      for (int jb = 0; jb <= ib; jb++) {
-        H[jb + nb * ib] = sbdgpu::dot_f(c, C[jb], nullptr, HC[ib], n);
-        H[ib + nb * jb] = H[jb + nb * ib];
-      }
+      sbdgpu::krylov_dots<float>(C.data(), ib + 1, HC[ib], n, part, scal, st);
+      read_back(&H[nb * ib], scal, ib + 1, st);
+      for (int jb = 0; jb <= ib; jb++) H[ib + nb * jb] = H[jb + nb * ib];
       for (int jb = 0; jb <= ib; jb++)
         for (int kb = 0; kb <= ib; kb++) U[jb + nb * kb] = H[jb + nb * kb];
       sbdgpu::jacobi_eig(ib + 1, U.data(), nb, E.data());
-      sbdgpu::ritz_update_f(C.data(), HC.data(), U.data(), ib + 1, E[0], W, R, n, c);
-      double nw = std::sqrt(sbdgpu::dot(c, W, W, n));
-      sbdgpu::scale(W, 1.0 / nw, n, st);
-      double tol = std::sqrt(sbdgpu::dot(c, R, R, n));
-      sbdgpu::scale(R, 1.0 / tol, n, st);
+      sbdgpu::krylov_ritz<float>(C.data(), HC.data(), ib + 1, ritz_coef(U.data(), ib + 1, E[0]), nullptr, nullptr, W, R,
+                                 n, part, scal + 32, st);
+      double tol = 0.0;
+      read_back(&tol, scal + 32, 1, st);
       if (trace_e && steps < max_trace) trace_e[steps] = E[0];
       if (trace_tol && steps < max_trace) trace_tol[steps] = tol;
       steps++;
@@ -394,11 +381,11 @@ void davidson_mixed(sbdgpu_ctx* c, const sbdgpu_opts* o, double* W, double* R, d
           std::swap(C[j], T[j]);
           std::swap(HC[j], TH[j]);
         }
-        for (int j = 0; j < kk; j++)
-          for (int i = 0; i <= j; i++) {
-            H[i + nb * j] = sbdgpu::dot_f(c, C[i], nullptr, HC[j], n);
-            H[j + nb * i] = H[i + nb * j];
-          }
+        for (int j = 0; j < kk; j++) {
+          sbdgpu::krylov_dots<float>(C.data(), j + 1, HC[j], n, part, scal, st);
+          read_back(&H[nb * j], scal, j + 1, st);
+          for (int i = 0; i <= j; i++) H[j + nb * i] = H[i + nb * j];
+        }
         add_correction(kk, E[0]);
         kept = kk;
       }
@@ -408,7 +395,6 @@ void davidson_mixed(sbdgpu_ctx* c, const sbdgpu_opts* o, double* W, double* R, d
         u_last_len = ib + 1;
         u_last_cycle = it;
       }
-      SBD_CUDA(cudaStreamSynchronize(st));
       auto t1 = std::chrono::steady_clock::now();
       step_times.push_back(std::chrono::duration<double>(t1 - t0).count());
       double avg = 0.0;
@@ -602,23 +588,19 @@ int sbdgpu_davidson(sbdgpu_ctx* c, const sbdgpu_opts* o, double* Wh, double* ene
     sbdgpu::compute_hii(c);
     sbdgpu::ensure_scratch(c);
     std::vector<double*> C(nb, nullptr), HC(nb, nullptr);
-    double *W = nullptr, *R = nullptr;
-    struct Free {
-      std::vector<double*>* a;
-      std::vector<double*>* b;
-      double** w;
-      double** r;
-      cudaStream_t s;
-      ~Free() {
-        cudaStreamSynchronize(s);  // an error path may leave kernels queued on these buffers
-        for (auto p : *a) cudaFree(p);
-        for (auto p : *b) cudaFree(p);
-        cudaFree(*w);
-        cudaFree(*r);
+    double *W = nullptr, *R = nullptr, *part = nullptr, *scal = nullptr;
+    sbdgpu::Arena arena(st);
+    arena.add(&W, n);
+    arena.add(&R, n);
+    if (o->precision == SBDGPU_FP64) {
+      for (int k = 0; k < nb; k++) {
+        arena.add(&C[k], n);
+        arena.add(&HC[k], n);
       }
-    } guard{&C, &HC, &W, &R, st};
-    W = (double*)sbdgpu::dev_alloc(sizeof(double) * n);
-    R = (double*)sbdgpu::dev_alloc(sizeof(double) * n);
+      arena.add(&part, 32 * sbdgpu::kKrylovBlocks);  // block sums
+      arena.add(&scal, 64);                          // overlaps and the residual norm
+    }
+    arena.commit();
     SBD_CUDA(cudaMemcpyAsync(W, Wh, sizeof(double) * n, cudaMemcpyHostToDevice, st));
     sbdgpu::apply_phase(c, W);
     if (o->precision != SBDGPU_FP64) {
@@ -632,11 +614,6 @@ int sbdgpu_davidson(sbdgpu_ctx* c, const sbdgpu_opts* o, double* Wh, double* ene
       if (n_steps) *n_steps = steps;
       return;
     }
-    for (int k = 0; k < nb; k++) {
-      C[k] = (double*)sbdgpu::dev_alloc(sizeof(double) * n);
-      HC[k] = (double*)sbdgpu::dev_alloc(sizeof(double) * n);
-    }
-    const double eps_reg = 1.0e-12;
     std::vector<double> H(nb * nb, 0.0), U(nb * nb, 0.0), E(nb, 0.0);
     std::vector<double> step_times;
     auto t_start = std::chrono::steady_clock::now();
@@ -647,18 +624,16 @@ int sbdgpu_davidson(sbdgpu_ctx* c, const sbdgpu_opts* o, double* Wh, double* ene
       for (int ib = 0; ib < nb; ib++) {
         auto t0 = std::chrono::steady_clock::now();
         sbdgpu::sigma_fp64(c, C[ib], HC[ib]);
-        for (int jb = 0; jb <= ib; jb++) {
-          H[jb + nb * ib] = sbdgpu::dot(c, C[jb], HC[ib], n);
-          H[ib + nb * jb] = H[jb + nb * ib];
-        }
+        sbdgpu::krylov_dots<double>(C.data(), ib + 1, HC[ib], n, part, scal, st);
+        read_back(&H[nb * ib], scal, ib + 1, st);
+        for (int jb = 0; jb <= ib; jb++) H[ib + nb * jb] = H[jb + nb * ib];
         for (int jb = 0; jb <= ib; jb++)
           for (int kb = 0; kb <= ib; kb++) U[jb + nb * kb] = H[jb + nb * kb];
         sbdgpu::jacobi_eig(ib + 1, U.data(), nb, E.data());
-        sbdgpu::ritz_update(C.data(), HC.data(), U.data(), ib + 1, E[0], W, R, n, st);
-        double nw = std::sqrt(sbdgpu::dot(c, W, W, n));
-        sbdgpu::scale(W, 1.0 / nw, n, st);
-        double tol = std::sqrt(sbdgpu::dot(c, R, R, n));
-        sbdgpu::scale(R, 1.0 / tol, n, st);
+        sbdgpu::krylov_ritz<double>(C.data(), HC.data(), ib + 1, ritz_coef(U.data(), ib + 1, E[0]), nullptr, nullptr, W,
+                                    R, n, part, scal + 32, st);
+        double tol = 0.0;
+        read_back(&tol, scal + 32, 1, st);
         if (trace_e && steps < max_trace) trace_e[steps] = E[0];
         if (trace_tol && steps < max_trace) trace_tol[steps] = tol;
         steps++;
@@ -672,16 +647,9 @@ int sbdgpu_davidson(sbdgpu_ctx* c, const sbdgpu_opts* o, double* Wh, double* ene
           cont = false;
           break;
         }
-        if (ib < nb - 1) {
-          sbdgpu::precondition(R, c->hii, E[0], eps_reg, C[ib + 1], n, st);
-          for (int kb = 0; kb < ib + 1; kb++) {
-            double olap = sbdgpu::dot(c, C[kb], C[ib + 1], n);
-            sbdgpu::axpy(C[ib + 1], C[kb], -olap, n, st);
-          }
-          double nc = std::sqrt(sbdgpu::dot(c, C[ib + 1], C[ib + 1], n));
-          sbdgpu::scale(C[ib + 1], 1.0 / nc, n, st);
-        }
-        SBD_CUDA(cudaStreamSynchronize(st));
+        if (ib < nb - 1)
+          sbdgpu::krylov_correction<double>(R, c->hii, E[0], nullptr, C[ib + 1], C.data(), ib + 1, C[ib + 1], n, 1, part,
+                                            st);
         auto t1 = std::chrono::steady_clock::now();
         step_times.push_back(std::chrono::duration<double>(t1 - t0).count());
         double avg = 0.0;

@@ -5,9 +5,9 @@
 // the GPU for every dot product.  For small problems those waits, not the
 // kernels, take the time.  Here every quantity of a step stays on the device:
 //
-//   dots        the same two-stage reductions, written to a per-problem
-//               scalar block instead of copied out
-//   eigenproblem one thread per problem runs the cyclic Jacobi on the
+//   dots        reductions whose sums stay in the problem's block of device
+//               memory (krylov.cu)
+//   eigenproblem one warp per problem runs the cyclic Jacobi on the
 //               (m <= 32) projected matrix (the reference uses LAPACK dsyev,
 //               framework/hp_numeric.h:500-517)
 //   Ritz vector, residual, the diagonal correction, Gram-Schmidt and the
@@ -17,8 +17,8 @@
 // its orthogonalisation, the sigma, the projected row, the eigenproblem, the
 // Ritz update and the norms -- is a fixed sequence of launches on the
 // problem's stream with fixed pointers.  Each (problem, Krylov index) step is
-// captured once into a CUDA graph and then replayed: one launch per problem
-// per step.  One host thread drives all problems in rounds: it launches one
+// captured into a CUDA graph when it runs for the second time and then
+// replayed: one launch per problem per step.  One host thread drives all problems in rounds: it launches one
 // step graph per unconverged problem, then waits once for the round and reads
 // each problem's residual norm (8 bytes, copied to pinned memory inside the
 // graph).  The vectors of all problems come from one device allocation made
@@ -41,7 +41,6 @@ namespace sbdgpu {
 namespace {
 
 constexpr int kMaxNb = 32;
-constexpr int kVT = 256;
 
 // scalar block of one problem (doubles)
 constexpr int kH = 0;                       // projected matrix, column-major [kMaxNb][kMaxNb]
@@ -50,63 +49,66 @@ constexpr int kE = kU + kMaxNb * kMaxNb;    // eigenvalues
 constexpr int kDot = kE + kMaxNb;           // scratch dot results
 constexpr int kTol = kDot + 8;              // residual norm
 constexpr int kEn = kTol + 1;               // final energy
-constexpr int kScal = kEn + 7;
-
-struct PtrPackD {
-  const double* p[kMaxNb];
-};
-
-unsigned grid_n(size_t n) { return (unsigned)std::min<size_t>((n + kVT - 1) / kVT, 148 * 8); }
+constexpr int kPart = kEn + 7;              // block sums of the vector kernels
+constexpr int kScal = kPart + 32 * kKrylovBlocks;
 
 // Cyclic Jacobi (the host solver's algorithm, api.cu jacobi_eig) by one warp:
-// lane 0 forms each rotation, the lanes apply it to rows / columns k = lane.
-// H: the upper triangle of the leading m x m block of the projected matrix
-// (column-major, leading dimension kMaxNb); U, E: eigenvectors and
-// eigenvalues in ascending order.  The matrices live in shared memory.
+// every lane forms each rotation, lane k applies it to row k (and by symmetry
+// column k) of the matrix and to row k of the eigenvectors; the 2 x 2 block has
+// a closed form.  H: the upper triangle of the leading m x m block of the
+// projected matrix (column-major, leading dimension kMaxNb); U, E: eigenvectors
+// and eigenvalues in ascending order.  A serial chain of rotations, each one
+// division, two square roots' worth of latency and a shared-memory round trip:
+// stops once the off-diagonal part is below 1e-20 of the diagonal's norm,
+// where a further sweep changes no bit of the eigenvalues (the eigenvalues
+// move by its square).  At m = 1 .. 10: 134 us on average with lane 0 forming
+// the rotations and sweeps down to 1e-150.
 __global__ void __launch_bounds__(32) eig_kernel(double* sc, int m) {
-  __shared__ double M[kMaxNb * kMaxNb];
-  __shared__ double V[kMaxNb * kMaxNb];
-  __shared__ double rot[2];
+  __shared__ double M[kMaxNb * (kMaxNb + 1)];
+  __shared__ double V[kMaxNb * (kMaxNb + 1)];
   __shared__ int order[kMaxNb];
   const int k = threadIdx.x;
+  constexpr int ld = kMaxNb + 1;
   const double* H = sc + kH;
   for (int j = 0; j < m; j++)
     if (k < m) {
-      M[k + j * m] = k <= j ? H[k + j * kMaxNb] : H[j + k * kMaxNb];
-      V[k + j * m] = k == j ? 1.0 : 0.0;
+      M[k + j * ld] = k <= j ? H[k + j * kMaxNb] : H[j + k * kMaxNb];
+      V[k + j * ld] = k == j ? 1.0 : 0.0;
     }
   __syncwarp();
   for (int sweep = 0; sweep < 100; sweep++) {
-    double off = 0.0;
-    for (int j = 0; j < m; j++)
-      if (k < j) off += M[k + j * m] * M[k + j * m];
-    for (int o = 16; o; o >>= 1) off += __shfl_xor_sync(0xffffffffu, off, o);
-    if (off < 1e-300) break;
+    double off = 0.0, dia = 0.0;
+    if (k < m) {
+      for (int j = k + 1; j < m; j++) off += M[k + j * ld] * M[k + j * ld];
+      dia = M[k + k * ld] * M[k + k * ld];
+    }
+    for (int o = 16; o; o >>= 1) {
+      off += __shfl_xor_sync(0xffffffffu, off, o);
+      dia += __shfl_xor_sync(0xffffffffu, dia, o);
+    }
+    if (off < 1e-300 || off <= 1e-40 * dia) break;
     for (int p = 0; p < m; p++)
       for (int q = p + 1; q < m; q++) {
-        const double apq = M[p + q * m];  // the same value in every lane
+        const double apq = M[p + q * ld];  // the same value in every lane
         if (fabs(apq) < 1e-300) continue;
-        if (k == 0) {
-          const double theta = 0.5 * (M[q + q * m] - M[p + p * m]) / apq;
-          const double t = (theta >= 0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
-          rot[0] = 1.0 / sqrt(t * t + 1.0);
-          rot[1] = t * rot[0];
-        }
-        __syncwarp();
-        const double cs = rot[0], sn = rot[1];
+        const double app = M[p + p * ld], aqq = M[q + q * ld];
+        const double theta = 0.5 * (aqq - app) / apq;
+        const double t = (theta >= 0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
+        const double cs = rsqrt(t * t + 1.0), sn = t * cs;
+        __syncwarp();  // the block is read
         if (k < m) {
-          const double a = M[k + p * m], b = M[k + q * m];
-          M[k + p * m] = cs * a - sn * b;
-          M[k + q * m] = sn * a + cs * b;
-        }
-        __syncwarp();
-        if (k < m) {
-          const double a = M[p + k * m], b = M[q + k * m];
-          M[p + k * m] = cs * a - sn * b;
-          M[q + k * m] = sn * a + cs * b;
-          const double va = V[k + p * m], vb = V[k + q * m];
-          V[k + p * m] = cs * va - sn * vb;
-          V[k + q * m] = sn * va + cs * vb;
+          if (k == p) {
+            M[p + p * ld] = app - t * apq;
+            M[q + q * ld] = aqq + t * apq;
+            M[p + q * ld] = M[q + p * ld] = 0.0;
+          } else if (k != q) {
+            const double a = M[k + p * ld], b = M[k + q * ld];
+            M[k + p * ld] = M[p + k * ld] = cs * a - sn * b;
+            M[k + q * ld] = M[q + k * ld] = sn * a + cs * b;
+          }
+          const double va = V[k + p * ld], vb = V[k + q * ld];
+          V[k + p * ld] = cs * va - sn * vb;
+          V[k + q * ld] = sn * va + cs * vb;
         }
         __syncwarp();
       }
@@ -114,7 +116,7 @@ __global__ void __launch_bounds__(32) eig_kernel(double* sc, int m) {
   if (k == 0) {
     for (int i = 0; i < m; i++) order[i] = i;
     for (int i = 1; i < m; i++)  // insertion sort by eigenvalue
-      for (int j = i; j > 0 && M[order[j] * (m + 1)] < M[order[j - 1] * (m + 1)]; j--) {
+      for (int j = i; j > 0 && M[order[j] * (ld + 1)] < M[order[j - 1] * (ld + 1)]; j--) {
         const int x = order[j];
         order[j] = order[j - 1];
         order[j - 1] = x;
@@ -123,56 +125,10 @@ __global__ void __launch_bounds__(32) eig_kernel(double* sc, int m) {
   __syncwarp();
   for (int c = 0; c < m; c++) {
     const int s = order[c];
-    if (k == 0) sc[kE + c] = M[s + s * m];
-    if (k < m) sc[kU + k + c * kMaxNb] = V[k + s * m];
+    if (k == 0) sc[kE + c] = M[s + s * ld];
+    if (k < m) sc[kU + k + c * kMaxNb] = V[k + s * ld];
   }
 }
-
-// W = sum_k u_k C_k, R = E0 W - sum_k u_k HC_k (u = lowest eigenvector)
-__global__ void ritz_dev_kernel(PtrPackD c, PtrPackD hc, int nk, const double* __restrict__ sc,
-                                double* __restrict__ W, double* __restrict__ R, size_t n) {
-  __shared__ double u[kMaxNb];
-  __shared__ double e0;
-  if (threadIdx.x < nk) u[threadIdx.x] = sc[kU + threadIdx.x];
-  if (threadIdx.x == 0) e0 = sc[kE];
-  __syncthreads();
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    double w = 0.0, r = 0.0;
-    for (int k = 0; k < nk; k++) {
-      w += c.p[k][i] * u[k];
-      r -= hc.p[k][i] * u[k];
-    }
-    W[i] = w;
-    R[i] = r + e0 * w;
-  }
-}
-
-// x *= 1 / sqrt(*d)
-__global__ void scale_rsqrt_kernel(double* __restrict__ x, const double* __restrict__ d, size_t n) {
-  const double a = 1.0 / sqrt(*d);
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-    x[i] *= a;
-}
-
-// y -= (*a) x
-__global__ void axpy_neg_kernel(double* __restrict__ y, const double* __restrict__ x, const double* __restrict__ a,
-                                size_t n) {
-  const double s = -*a;
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-    y[i] += x[i] * s;
-}
-
-// out = R / (E0 - H_ii), regularised as davidson.h:855-862, E0 = the lowest eigenvalue
-__global__ void precond_dev_kernel(const double* __restrict__ R, const double* __restrict__ hii,
-                                   const double* __restrict__ sc, double* __restrict__ out, size_t n) {
-  const double e0 = sc[kE], eps_reg = 1.0e-12;
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    const double den = e0 - hii[i];
-    out[i] = fabs(den) > eps_reg ? R[i] / den : R[i] / (den - eps_reg);
-  }
-}
-
-__global__ void sqrt_to_kernel(const double* __restrict__ d, double* __restrict__ out) { *out = sqrt(*d); }
 
 // One problem of the batch: its context, vectors (slices of the batch's
 // allocation), scalar block, pinned residual norm and step graphs.
@@ -186,6 +142,7 @@ struct Prob {
   double* sc = nullptr;
   double* host = nullptr;  // pinned: [tol, energy]
   std::vector<cudaGraphExec_t> step;  // step graph per Krylov index
+  std::vector<char> ran;              // whether the index has run before
   int it = 0, ib = 0, steps = 0;
   bool done = false;
 };
@@ -198,45 +155,27 @@ void enqueue_step(Prob& p, int ib) {
   sbdgpu_ctx* c = p.c;
   cudaStream_t st = c->stream;
   const size_t n = p.n;
-  double* dot = p.sc + kDot;
-  if (ib == 0) {
+  double* part = p.sc + kPart;
+  if (ib == 0)
     SBD_CUDA(cudaMemcpyAsync(p.C[0], p.W, sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
-  } else {
-    precond_dev_kernel<<<grid_n(n), kVT, 0, st>>>(p.R, c->hii, p.sc, p.C[ib], n);
-    SBD_CUDA(cudaGetLastError());
-    for (int kb = 0; kb < ib; kb++) {  // modified Gram-Schmidt, davidson.h:864-875
-      dot_device(c, p.C[kb], p.C[ib], n, dot);
-      axpy_neg_kernel<<<grid_n(n), kVT, 0, st>>>(p.C[ib], p.C[kb], dot, n);
-    }
-    dot_device(c, p.C[ib], p.C[ib], n, dot);
-    scale_rsqrt_kernel<<<grid_n(n), kVT, 0, st>>>(p.C[ib], dot, n);
-    SBD_CUDA(cudaGetLastError());
-  }
+  else  // modified Gram-Schmidt, davidson.h:864-875
+    krylov_correction<double>(p.R, c->hii, 0.0, p.sc + kE, p.C[ib], p.C.data(), ib, p.C[ib], n, 1, part, st);
   sigma_fp64_prepared(c, p.C[ib], p.HC[ib], c->ct, c->st);
-  for (int jb = 0; jb <= ib; jb++) dot_device(c, p.C[jb], p.HC[ib], n, p.sc + kH + jb + kMaxNb * ib);
+  krylov_dots<double>(p.C.data(), ib + 1, p.HC[ib], n, part, p.sc + kH + kMaxNb * ib, st);
   eig_kernel<<<1, 32, 0, st>>>(p.sc, ib + 1);
-  PtrPackD pc{}, ph{};
-  for (int k = 0; k <= ib; k++) {
-    pc.p[k] = p.C[k];
-    ph.p[k] = p.HC[k];
-  }
-  ritz_dev_kernel<<<grid_n(n), kVT, 0, st>>>(pc, ph, ib + 1, p.sc, p.W, p.R, n);
   SBD_CUDA(cudaGetLastError());
-  dot_device(c, p.W, p.W, n, dot);
-  scale_rsqrt_kernel<<<grid_n(n), kVT, 0, st>>>(p.W, dot, n);
-  dot_device(c, p.R, p.R, n, dot + 1);
-  sqrt_to_kernel<<<1, 1, 0, st>>>(dot + 1, p.sc + kTol);
-  scale_rsqrt_kernel<<<grid_n(n), kVT, 0, st>>>(p.R, dot + 1, n);
-  SBD_CUDA(cudaGetLastError());
+  krylov_ritz<double>(p.C.data(), p.HC.data(), ib + 1, RitzCoef{}, p.sc + kU, p.sc + kE, p.W, p.R, n, part, p.sc + kTol,
+                      st);
   SBD_CUDA(cudaMemcpyAsync(p.host, p.sc + kTol, sizeof(double), cudaMemcpyDeviceToHost, st));
 }
 
-// Replays the step's graph, capturing it on first use.  If the capture or
-// the instantiation is refused, the problem's steps are launched directly
-// from then on.
+// Replays the step's graph.  A step's first run is launched directly: capturing
+// and instantiating its graph costs several times the launches, which only a
+// later cycle's replays win back.  If the capture or the instantiation is
+// refused, the problem's steps are launched directly from then on.
 void launch_step(Prob& p, int ib, bool& graphs) {
   cudaStream_t st = p.c->stream;
-  if (graphs && !p.step[ib]) {
+  if (graphs && !p.step[ib] && p.ran[ib]) {
     cudaGraph_t g = nullptr;
     cudaGraphExec_t ex = nullptr;
     bool ok = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
@@ -257,6 +196,7 @@ void launch_step(Prob& p, int ib, bool& graphs) {
       p.step[ib] = ex;
     }
   }
+  p.ran[ib] = 1;
   if (graphs && p.step[ib])
     SBD_CUDA(cudaGraphLaunch(p.step[ib], st));
   else
@@ -276,7 +216,7 @@ void davidson_batch_fp64(int nprob, sbdgpu_ctx* const* ctxs, const sbdgpu_opts* 
     P[i].c = c;
     P[i].n = c->N;
     P[i].nb = nb;
-    total += (size_t)(2 * nb + 2) * ((c->N + 1) & ~size_t(1)) + kScal;  // vectors start on 16 bytes
+    total += (size_t)(2 * nb + 2) * ((c->N + 1) & ~size_t(1)) + kScal;  // vectors start on 16 bytes (kScal is even)
   }
   preload_fp64_sigma(ctxs[0]->device);
   // every vector of every problem in one allocation, made before the first round
@@ -317,6 +257,7 @@ void davidson_batch_fp64(int nprob, sbdgpu_ctx* const* ctxs, const sbdgpu_opts* 
     off += kScal;
     p.host = pinned + 2 * i;
     p.step.assign(nb, nullptr);
+    p.ran.assign(nb, 0);
     SBD_CUDA(cudaMemsetAsync(p.sc, 0, sizeof(double) * kScal, p.c->stream));
     SBD_CUDA(cudaMemcpyAsync(p.W, Wh[i], sizeof(double) * p.n, cudaMemcpyHostToDevice, p.c->stream));
     apply_phase(p.c, p.W);

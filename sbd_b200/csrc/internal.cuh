@@ -174,13 +174,9 @@ void ensure_fp32(sbdgpu_ctx* c);
 double dot(sbdgpu_ctx* c, const double* x, const double* y, size_t n);
 void dot_device(sbdgpu_ctx* c, const double* x, const double* y, size_t n, double* out);  // needs ensure_scratch
 void scale(double* x, double a, size_t n, cudaStream_t s);
-double dot_f(sbdgpu_ctx* c, const float* x, const double* xd, const float* y, size_t n);
-void axpy_df(double* y, const float* x, double a, size_t n, cudaStream_t s);
 void lincomb_f(float* const* in, const double* U, int nk, float* out, size_t n, sbdgpu_ctx* c);
 void convert(const double* in, float* out, size_t n, cudaStream_t s);
 void convert(const float* in, double* out, size_t n, cudaStream_t s);
-void ritz_update_f(float* const* C, float* const* HC, const double* U, int nk, double e0, double* W, double* R,
-                   size_t n, sbdgpu_ctx* c);
 void axpy(double* y, const double* x, double a, size_t n, cudaStream_t s);
 void ritz_update(double* const* C, double* const* HC, const double* U, int nk, double e0, double* W,
                  double* R, size_t n, cudaStream_t s);
@@ -226,6 +222,50 @@ void alpha_coulomb(sbdgpu_ctx* c, const double* C, double* S);
 void genop_set_error(sbdgpu_genop* g, const std::string& msg);
 void occupation(sbdgpu_ctx* c, const double* dW, double* dens);
 void alpha_weights(sbdgpu_ctx* c, const double* dW, double* D);
+
+// krylov.cu: Davidson vector kernels (basis vectors of type B)
+constexpr int kKrylovBlocks = 592;  // 4 x 148 SMs
+template <typename B>
+struct BasisPack {
+  const B* p[32];
+};
+struct RitzCoef {
+  double u[32];
+  double e0;
+};
+template <typename B>
+void krylov_correction(const double* R, const double* hii, double e0, const double* e0_dev, double* x,
+                       const B* const* C, int k, B* out, size_t n, int passes, double* part, cudaStream_t s);
+template <typename B>
+void krylov_dots(const B* const* C, int k, const B* y, size_t n, double* part, double* out, cudaStream_t s);
+template <typename B>
+void krylov_ritz(const B* const* C, const B* const* HC, int nk, const RitzCoef& u, const double* u_dev,
+                 const double* e0_dev, double* W, double* R, size_t n, double* part, double* tol, cudaStream_t s);
+
+// One device allocation in slices, freed when it leaves scope, after the
+// stream's work on it.
+class Arena {
+ public:
+  explicit Arena(cudaStream_t s) : stream_(s) {}
+  Arena(const Arena&) = delete;
+  Arena& operator=(const Arena&) = delete;
+  ~Arena() {
+    if (base_) cudaStreamSynchronize(stream_);  // an error path may leave kernels queued on it
+    cudaFree(base_);
+  }
+  template <typename T>
+  void add(T** where, size_t count) {  // *where is set by commit()
+    slots_.push_back({reinterpret_cast<void**>(where), total_});
+    total_ += (sizeof(T) * count + 255) / 256 * 256;
+  }
+  void commit();
+
+ private:
+  cudaStream_t stream_;
+  char* base_ = nullptr;
+  size_t total_ = 0;
+  std::vector<std::pair<void**, size_t>> slots_;
+};
 
 // tc_ab.cu
 bool tc_ab_supported(const sbdgpu_ctx* c);

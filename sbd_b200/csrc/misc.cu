@@ -154,27 +154,6 @@ __global__ void axpy_kernel(double* y, const double* x, double a, size_t n) {
     y[i] += x[i] * a;
 }
 
-__global__ void dot_partial_f(const float* __restrict__ x, const float* __restrict__ y, const double* __restrict__ xd,
-                              size_t n, double* __restrict__ part) {
-  __shared__ double sh[kRedThreads / 32];
-  double acc = 0.0;
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-    acc += (xd ? xd[i] : (double)x[i]) * (double)y[i];
-  for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = acc;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double s = 0.0;
-    for (int w = 0; w < kRedThreads / 32; w++) s += sh[w];
-    part[blockIdx.x] = s;
-  }
-}
-
-__global__ void axpy_df_kernel(double* y, const float* x, double a, size_t n) {
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-    y[i] += (double)x[i] * a;
-}
-
 __global__ void convert_kernel_df(const double* __restrict__ in, float* __restrict__ out, size_t n) {
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
     out[i] = (float)in[i];
@@ -188,20 +167,6 @@ __global__ void convert_kernel_fd(const float* __restrict__ in, double* __restri
 struct PtrPackF {
   const float* p[32];
 };
-
-// mixed path: W = sum_k U_k C_k ; R = E0*W - sum_k U_k HC_k, FP32 basis, FP64 result
-__global__ void ritz_kernel_f(PtrPackF c, PtrPackF hc, const double* __restrict__ u, int nk, double e0,
-                              double* __restrict__ W, double* __restrict__ R, size_t n) {
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    double w = 0.0, r = 0.0;
-    for (int k = 0; k < nk; k++) {
-      w += (double)c.p[k][i] * u[k];
-      r -= (double)hc.p[k][i] * u[k];
-    }
-    W[i] = w;
-    R[i] = r + e0 * w;
-  }
-}
 
 // out = sum_k u_k in_k (FP32 vectors, FP64 accumulation)
 __global__ void lincomb_kernel_f(PtrPackF in, const double* __restrict__ u, int nk, float* __restrict__ out,
@@ -405,22 +370,6 @@ void dot_device(sbdgpu_ctx* c, const double* x, const double* y, size_t n, doubl
   SBD_CUDA(cudaGetLastError());
 }
 
-double dot_f(sbdgpu_ctx* c, const float* x, const double* xd, const float* y, size_t n) {
-  ensure_scratch(c);
-  dot_partial_f<<<kRedBlocks, kRedThreads, 0, c->stream>>>(x, y, xd, n, c->red);
-  dot_final<<<1, 1024, 0, c->stream>>>(c->red, kRedBlocks, c->red + kRedBlocks);
-  SBD_CUDA(cudaGetLastError());
-  double r = 0.0;
-  SBD_CUDA(cudaMemcpyAsync(&r, c->red + kRedBlocks, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-  SBD_CUDA(cudaStreamSynchronize(c->stream));
-  return r;
-}
-
-void axpy_df(double* y, const float* x, double a, size_t n, cudaStream_t s) {
-  axpy_df_kernel<<<grid_for(n), 256, 0, s>>>(y, x, a, n);
-  SBD_CUDA(cudaGetLastError());
-}
-
 void convert(const double* in, float* out, size_t n, cudaStream_t s) {
   convert_kernel_df<<<grid_for(n), 256, 0, s>>>(in, out, n);
   SBD_CUDA(cudaGetLastError());
@@ -429,21 +378,6 @@ void convert(const double* in, float* out, size_t n, cudaStream_t s) {
 void convert(const float* in, double* out, size_t n, cudaStream_t s) {
   convert_kernel_fd<<<grid_for(n), 256, 0, s>>>(in, out, n);
   SBD_CUDA(cudaGetLastError());
-}
-
-void ritz_update_f(float* const* C, float* const* HC, const double* U, int nk, double e0, double* W, double* R,
-                   size_t n, sbdgpu_ctx* c) {
-  PtrPackF pc{}, ph{};
-  for (int k = 0; k < nk; k++) {
-    pc.p[k] = C[k];
-    ph.p[k] = HC[k];
-  }
-  ensure_scratch(c);
-  double* du = c->red + 600;  // 32 spare doubles after the 593 reduction slots
-  SBD_CUDA(cudaMemcpyAsync(du, U, sizeof(double) * nk, cudaMemcpyHostToDevice, c->stream));
-  ritz_kernel_f<<<grid_for(n), 256, 0, c->stream>>>(pc, ph, du, nk, e0, W, R, n);
-  SBD_CUDA(cudaGetLastError());
-  SBD_CUDA(cudaStreamSynchronize(c->stream));
 }
 
 void lincomb_f(float* const* in, const double* U, int nk, float* out, size_t n, sbdgpu_ctx* c) {
