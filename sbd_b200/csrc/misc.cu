@@ -447,25 +447,35 @@ void occupation(sbdgpu_ctx* c, const double* dW, double* dens) {
 void rdm(sbdgpu_ctx* c, const double* dW, double* one, double* two) {
   int L = c->L;
   size_t L2 = (size_t)L * L, L4 = L2 * L2;
-  double* d_one = (double*)dev_alloc(sizeof(double) * (2 * L2 + 4 * L4));
+  // bases with alpha-beta tiles (distinct strings, at most 65,535 beta ones):
+  // products on the tensor pipe, the opposite-spin diagonal included
+  const bool products = c->tab[1].tile_grp != nullptr;
+  double *d_one = nullptr, *Da = nullptr;
+  Arena arena(c->stream);
+  arena.add(&d_one, 2 * L2 + 4 * L4);
+  arena.add(&Da, c->na + c->nb + (products ? 0 : c->na * L));
+  arena.commit();
   double* d_two = d_one + 2 * L2;
   SBD_CUDA(cudaMemsetAsync(d_one, 0, sizeof(double) * (2 * L2 + 4 * L4), c->stream));
-  rdm_offdiag(c, dW, d_one, d_two);
-  // diagonal contributions (ZeroDiffCorrelation, correlation.h:15-44) from the
-  // alpha-row weights, beta-column weights and the alpha x beta occupation moment
-  double* Da = (double*)dev_alloc(sizeof(double) * (c->na + c->nb + c->na * L));
-  double* Db = Da + c->na;
-  double* X = Db + c->nb;
-  row_weights_kernel<<<(unsigned)c->na, 256, 0, c->stream>>>(dW, c->bstr, c->nb, L, Da, X);
-  col_weights_kernel<<<(unsigned)((c->nb + 255) / 256), 256, 0, c->stream>>>(dW, c->na, c->nb, Db);
-  SBD_CUDA(cudaGetLastError());
-  std::vector<double> h(c->na + c->nb + c->na * L);
+  if (products) {
+    ensure_io(c);
+    phase_copy(c, dW, c->io_b);
+    rdm_products(c, c->io_b, d_one, d_two, Da);
+  } else {
+    rdm_offdiag(c, dW, d_one, d_two);
+    // diagonal contributions (ZeroDiffCorrelation, correlation.h:15-44) from the
+    // alpha-row weights, beta-column weights and the alpha x beta occupation moment
+    double* Db = Da + c->na;
+    double* X = Db + c->nb;
+    row_weights_kernel<<<(unsigned)c->na, 256, 0, c->stream>>>(dW, c->bstr, c->nb, L, Da, X);
+    col_weights_kernel<<<(unsigned)((c->nb + 255) / 256), 256, 0, c->stream>>>(dW, c->na, c->nb, Db);
+    SBD_CUDA(cudaGetLastError());
+  }
+  std::vector<double> h(c->na + c->nb + (products ? 0 : c->na * L));
   SBD_CUDA(cudaMemcpyAsync(h.data(), Da, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, c->stream));
   SBD_CUDA(cudaMemcpyAsync(one, d_one, sizeof(double) * 2 * L2, cudaMemcpyDeviceToHost, c->stream));
   SBD_CUDA(cudaMemcpyAsync(two, d_two, sizeof(double) * 4 * L4, cudaMemcpyDeviceToHost, c->stream));
   SBD_CUDA(cudaStreamSynchronize(c->stream));
-  cudaFree(d_one);
-  cudaFree(Da);
   const double* hDa = h.data();
   const double* hDb = hDa + c->na;
   const double* hX = hDb + c->nb;
@@ -475,7 +485,8 @@ void rdm(sbdgpu_ctx* c, const double* dW, double* one, double* two) {
     for (int p = 0; p < L; p++) {
       if (!((a >> p) & 1)) continue;
       na1[p] += hDa[ia];
-      for (int r = 0; r < L; r++) M[p * L + r] += hX[ia * L + r];
+      if (!products)
+        for (int r = 0; r < L; r++) M[p * L + r] += hX[ia * L + r];
       for (int q = 0; q < L; q++)
         if (q != p && ((a >> q) & 1)) Aaa[p * L + q] += hDa[ia];
     }

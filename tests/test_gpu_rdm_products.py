@@ -1,0 +1,48 @@
+"""RDMs by products (csrc/rdm_mma.cu) against the CPU oracle at the edges of
+their blocks: four beta strings, eight columns (P = L (L + 1) / 2), 16 alpha
+rows per CTA, 64-wide tiles of the density products; repeated strings keep the
+scalar kernels."""
+import numpy as np
+import pytest
+
+import oracle
+import sbd_b200
+from sbd_b200 import synth
+
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-11  # the bound of the other RDM tests against the oracle (a normalised vector)
+
+
+def _check(norb, nea, neb, na, nb, seed, repeat=0):
+    ints = synth.make_integrals(norb, seed)
+    rng = np.random.default_rng(seed)
+
+    def pick(ne, n):
+        s = synth.full_strings(norb, ne)
+        return s[np.sort(rng.choice(len(s), min(n, len(s)), replace=False))]
+    a, b = pick(nea, na), pick(neb, nb)
+    if repeat:
+        b = np.concatenate([b, b[:repeat]])
+    ctx = sbd_b200.context_from_integrals(ints, a, b)
+    W = rng.normal(size=ctx.n)
+    W /= np.linalg.norm(W)
+    one, two = ctx.rdm(W)
+    ref1, ref2 = oracle.Oracle(norb, a, b, ints.ecore, ints.h, ints.eri).correlation(W)
+    assert np.abs(one - ref1).max() <= TOL and np.abs(two - ref2).max() <= TOL
+    ctx.close()
+
+
+@pytest.mark.parametrize("nb", [1, 3, 4, 5, 63, 65])
+def test_beta_strings(nb):
+    _check(9, 3, 3, 40, nb, 10 + nb)
+
+
+@pytest.mark.parametrize("norb,nea", [(4, 1), (7, 3), (8, 4), (11, 5), (17, 1), (18, 1)])
+def test_alpha_rows_and_columns(norb, nea):
+    # 10 to 171 columns; full alpha spaces with up to 30 singles per string
+    _check(norb, nea, 2, 70, 37, norb)
+
+
+def test_repeated_strings_keep_the_scalar_kernels():
+    _check(8, 3, 3, 20, 21, 3, repeat=2)
