@@ -7,7 +7,7 @@
 //   states      [n][nw] uint64 in the caller's order (site q at bit q%64 of
 //               word q/64), nw = 1, 2 or 4
 //   hash table  open addressing with linear probing over a power-of-two
-//               table of at least twice the states: a slot holds the key words
+//               table of at least two to four times the states: a slot holds the key words
 //               and, during a mult, the state's vector element, so that one
 //               probe returns the value itself (a slot of one-word states is 16
 //               bytes: one sector per term instead of three for index, key and
@@ -29,8 +29,7 @@
 // operators before it have flipped sites of their own, so the total is the
 // parity of the state under the exclusive-or of the "below" masks, times a
 // constant that goes into the coefficient.  The lanes' sums are reduced in the
-// warp, so no atomics.  Bound by the random 32-byte sectors of the hash table
-// in L2, one per Hamiltonian element.
+// warp, so no atomics.
 #include <algorithm>
 #include <chrono>
 #include <cmath>
@@ -96,20 +95,21 @@ struct Bucket {
   int64_t start, end;  // its terms in the sorted term array
 };
 
-__host__ __device__ __forceinline__ uint64_t mix64(uint64_t x) {  // splitmix64 finaliser
-  x ^= x >> 30;
-  x *= 0xbf58476d1ce4e5b9ull;
-  x ^= x >> 27;
-  x *= 0x94d049bb133111ebull;
-  x ^= x >> 31;
-  return x;
-}
-
+// Hash of a state, in 32-bit steps: two odd multipliers per word, then one
+// round of shifts and a multiply, enough to spread bit strings that differ in a
+// few sites (at a quarter full: 1.15 probes per search, 97 % within two).  The
+// upper half only serves tables of more than 2^32 slots.
 template <int NW>
-__host__ __device__ __forceinline__ uint64_t hash_state(const uint64_t* w) {
-  uint64_t h = 0x9e3779b97f4a7c15ull;
-  for (int x = 0; x < NW; x++) h = mix64(h ^ w[x]);
-  return h;
+__host__ __device__ __forceinline__ uint64_t hash_state(const uint64_t* w, uint64_t hmask) {
+  uint32_t h = 0;
+  for (int x = 0; x < NW; x++) {
+    h = (h ^ (h >> 16)) + (uint32_t)w[x] * 0x9E3779B1u + (uint32_t)(w[x] >> 32) * 0x85EBCA77u;
+    h ^= h >> 15;
+    h *= 0x2C1B3C6Du;
+  }
+  uint64_t r = h ^ (h >> 13);
+  if (hmask >> 32) r |= (uint64_t)((uint32_t)(w[0] >> 16) * 0xC2B2AE3Du ^ h) << 32;
+  return r & hmask;
 }
 
 template <int NW>
@@ -132,7 +132,7 @@ struct TermList {
 template <int NW>
 __device__ __forceinline__ double element(const Slot<NW>* __restrict__ slots, uint64_t hmask, const uint64_t* absent,
                                           const uint64_t* w) {
-  uint64_t h = hash_state<NW>(w) & hmask;
+  uint64_t h = hash_state<NW>(w, hmask);
   // the table is at most half full, so an empty slot ends every probe
   // sequence; the bound keeps the loop finite regardless
   for (uint64_t probe = 0; probe <= hmask; probe++) {
@@ -256,9 +256,12 @@ __device__ __forceinline__ bool apply_term(const Term<NW>& t, const uint64_t* v,
 }
 
 // W[i] += hdiag[i] C[i] + sum over off-diagonal terms of coef * sign * C[j]:
-// one warp per state.  The 349M elements of the 245,025-state FCIDUMP operator
-// took 16.1 ms with index, key and element in three sectors, the sign from the
-// operators one by one and the buckets tested one after another.
+// one warp per state.  Bound by the integer pipe (81 % busy).  The 349M elements
+// of the 245,025-state FCIDUMP operator: 16.1 ms with index, key and element in
+// three sectors, the sign from the operators one by one and the buckets tested
+// one after another; 6.6 ms with one sector, the sign by mask and 32 buckets at
+// a time; 4.8 ms with a 32-bit hash and a quarter-full table.  (Queueing the
+// targets that apply and probing for 32 at a time: 4.9 ms.)
 constexpr int kMultWarps = kThreads / 32;
 template <int NW>
 struct Words {
@@ -353,13 +356,15 @@ template <int NW>
 void build_basis(sbdgpu_genop* g, const uint64_t* states) {
   const size_t n = g->n;
   cudaStream_t st = g->base.stream;
-  size_t count = 1024;  // at least twice the states, a power of two
-  while (count < 2 * n) count <<= 1;
+  // a power of two of at least four times the states (twice above 1 GiB: the
+  // lanes of a warp wait for their longest search)
+  size_t count = 1024;
+  while (count < 4 * n && (count < 2 * n || count * sizeof(Slot<NW>) < (size_t(1) << 30))) count <<= 1;
   g->hmask = count - 1;
   std::vector<int64_t> at(count, -1), slot_of(n);  // state of a slot, slot of a state
   // slot of configuration w, or of the empty slot that ends its search
   const auto find = [&](const uint64_t* w) {
-    uint64_t h = hash_state<NW>(w) & g->hmask;
+    uint64_t h = hash_state<NW>(w, g->hmask);
     while (at[h] >= 0 && !std::equal(w, w + NW, &states[(size_t)at[h] * NW])) h = (h + 1) & g->hmask;
     return h;
   };
