@@ -25,6 +25,7 @@
 // fragment (lane = 4 n + k); an empty slot points at a zero behind the row of
 // C.
 #include <algorithm>
+#include <type_traits>
 #include <vector>
 
 #include "internal.cuh"
@@ -168,6 +169,9 @@ __device__ __forceinline__ void mma8(double (&d)[4], double a0, double b) {
       : "d"(a0), "d"(b));
 }
 
+// FP32 vectors: the row of C is converted as it is staged, products and sums
+// stay FP64, a row's sum is rounded once before it is added.
+//
 // What bounds it: the shared-memory pipe (16M determinants: 86 % of its
 // wavefronts, the FP64 tensor pipe 68 % busy).  Alpha-beta term, gather kernel
 // -> tiles: 144M determinants 198 -> 93 ms, 16M 11.2 -> 4.0 ms, 1501 x 803
@@ -221,9 +225,10 @@ __device__ __forceinline__ void products(const unsigned char* vsub, uint32_t lbi
   }
 }
 
+template <typename T>
 struct MmaArgs {
-  const double* C;
-  double* S;
+  const T* C;
+  T* S;
   size_t na, nb, ia0;
   int P, npair;
   const double* vf;
@@ -239,10 +244,16 @@ struct MmaArgs {
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
-// dst[0 .. bytes / 8) += staged values, by the copy engine (16-byte aligned
-// addresses, bytes a multiple of 16)
+// dst += staged values, by the copy engine (16-byte aligned addresses, bytes a
+// multiple of 16)
 __device__ __forceinline__ void bulk_add(double* dst, uint32_t src, uint32_t bytes) {
   asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f64 [%0], [%1], %2;" ::"l"(dst), "r"(src),
+               "r"(bytes)
+               : "memory");
+}
+
+__device__ __forceinline__ void bulk_add(float* dst, uint32_t src, uint32_t bytes) {
+  asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;" ::"l"(dst), "r"(src),
                "r"(bytes)
                : "memory");
 }
@@ -275,9 +286,9 @@ __device__ __forceinline__ void section(const E* __restrict__ p, int n, F&& step
 // copy engine where they start on 16 bytes, else by coalesced atomics.  (Added
 // straight from the accumulators' layout, 8 rows x 2 columns per lane, the
 // atomics took 29 % of the shared-memory pipe's wavefronts.)
-template <int M, int BLOCKS>
-__device__ __forceinline__ void tiles(const MmaArgs& a, const unsigned char* vsub, const unsigned char* crow,
-                                      double* stage, const int* tgt, const uint32_t* neg) {
+template <typename T, int M, int BLOCKS>
+__device__ __forceinline__ void tiles(const MmaArgs<T>& a, const unsigned char* vsub, const unsigned char* crow,
+                                      T* stage, const int* tgt, const uint32_t* neg) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
   const int r = lane >> 2, q = lane & 3;
   const uint32_t lbits = lane_bits<M>(r);
@@ -305,17 +316,18 @@ __device__ __forceinline__ void tiles(const MmaArgs& a, const unsigned char* vsu
 #pragma unroll
     for (int b = 0; b < BLOCKS; b++) {
       const uint32_t sg = neg[8 * b + r];
-      const auto val = [&](double x) { return __hiloint2double(__double2hiint(x) ^ (int)sg, __double2loint(x)); };
-      double* row = stage + (8 * b + r) * 16 + 2 * q;
-      *reinterpret_cast<double2*>(row) = make_double2(val(acc0[2 * b]), val(acc0[2 * b + 1]));
-      *reinterpret_cast<double2*>(row + 8) = make_double2(val(acc1[2 * b]), val(acc1[2 * b + 1]));
+      const auto val = [&](double x) { return (T)__hiloint2double(__double2hiint(x) ^ (int)sg, __double2loint(x)); };
+      using V = typename std::conditional<sizeof(T) == 8, double2, float2>::type;
+      T* row = stage + (8 * b + r) * 16 + 2 * q;
+      *reinterpret_cast<V*>(row) = V{val(acc0[2 * b]), val(acc0[2 * b + 1])};
+      *reinterpret_cast<V*>(row + 8) = V{val(acc1[2 * b]), val(acc1[2 * b + 1])};
     }
     if (a.bulk) {
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
       if (lane < 8 * BLOCKS && tgt[lane] >= 0)
         bulk_add(a.S + (size_t)tgt[lane] * a.nb + ib0, smem_addr(stage + lane * 16),
-                 (uint32_t)min((size_t)16, a.nb - ib0) * 8u);
+                 (uint32_t)min((size_t)16, a.nb - ib0) * (uint32_t)sizeof(T));
       asm volatile("cp.async.bulk.commit_group;" ::: "memory");
     } else {
       __syncwarp();
@@ -338,14 +350,14 @@ __device__ __forceinline__ void tiles(const MmaArgs& a, const unsigned char* vsu
 // alpha singles' Coulomb part J_pq[ib] C[ja,ib] as the value a row's sums start
 // from cost 20 ms more, 5.4 against 4.0 ms at 16M: its loads stall the warps and
 // take shared-memory wavefronts.  It stays a pass of its own.)
-template <int M>
-__global__ void __launch_bounds__(kMmaThreads) ab_mma_kernel(const MmaArgs a) {
+template <typename T, int M>
+__global__ void __launch_bounds__(kMmaThreads) ab_mma_kernel(const MmaArgs<T> a) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ int tgt[M];
   __shared__ uint32_t neg[M];
   unsigned char* vsub = smem;                                                          // [npair][M] integrals
-  double* stage = reinterpret_cast<double*>(smem + (size_t)a.npair * M * 8);           // [warps][M][16] results
-  double* crow = stage + (size_t)(blockDim.x >> 5) * M * 16;                           // [nb + 1]
+  T* stage = reinterpret_cast<T*>(smem + (size_t)a.npair * M * 8);                     // [warps][M][16] results
+  double* crow = reinterpret_cast<double*>(stage + (size_t)(blockDim.x >> 5) * M * 16);  // [nb + 1]
   const size_t ja = blockIdx.x;
   const int64_t k0 = a.a_off[ja] + (int64_t)blockIdx.y * M;
   const int singles = (int)min((int64_t)M, a.a_off[ja + 1] - k0);  // negative past the last ones
@@ -358,7 +370,7 @@ __global__ void __launch_bounds__(kMmaThreads) ab_mma_kernel(const MmaArgs a) {
     const uint32_t info = g < singles ? a.a_info[k0 + g] : 0u;
     neg[g] = info & 0x80000000u;
   }
-  for (size_t i = threadIdx.x; i <= a.nb; i += blockDim.x) crow[i] = i < a.nb ? a.C[ja * a.nb + i] : 0.0;
+  for (size_t i = threadIdx.x; i <= a.nb; i += blockDim.x) crow[i] = i < a.nb ? (double)a.C[ja * a.nb + i] : 0.0;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
   // one 32-byte chunk of eight pairs' rows per warp and step
   for (int c = 0; c < M / 4; c++) {
@@ -373,12 +385,12 @@ __global__ void __launch_bounds__(kMmaThreads) ab_mma_kernel(const MmaArgs a) {
           vrow ? __ldg(&vrow[(size_t)folded_pair(o) * step]) : 0.0;
   }
   __syncthreads();
-  double* mine = stage + (size_t)warp * M * 16;
+  T* mine = stage + (size_t)warp * M * 16;
   const unsigned char* cr = reinterpret_cast<const unsigned char*>(crow);
   if (M == 16 && count > 8)
-    tiles<M, M / 8>(a, vsub, cr, mine, tgt, neg);
+    tiles<T, M, M / 8>(a, vsub, cr, mine, tgt, neg);
   else
-    tiles<M, 1>(a, vsub, cr, mine, tgt, neg);
+    tiles<T, M, 1>(a, vsub, cr, mine, tgt, neg);
 }
 
 }  // namespace
@@ -386,18 +398,18 @@ __global__ void __launch_bounds__(kMmaThreads) ab_mma_kernel(const MmaArgs a) {
 namespace {
 
 // dynamic shared memory: integrals, per-warp stages, the row of C
-size_t mma_smem(const sbdgpu_ctx* c, int m, int threads) {
-  return sizeof(double) * ((size_t)(c->L * (c->L - 1) / 2) * m + (size_t)(threads / 32) * m * 16 + (c->nb + 1));
+size_t mma_smem(const sbdgpu_ctx* c, int m, int threads, size_t elem) {
+  return sizeof(double) * ((size_t)(c->L * (c->L - 1) / 2) * m + (c->nb + 1)) + elem * (threads / 32) * m * 16;
 }
 
-template <int M>
-void launch_mma(sbdgpu_ctx* c, const double* C, double* S, const AlphaSingles& as, int nt, bool beta_j) {
+template <typename T, int M>
+void launch_mma(sbdgpu_ctx* c, const T* C, T* S, const AlphaSingles& as, int nt, bool beta_j) {
   const SpinTables& tb = c->tab[1];
   const dim3 grid((unsigned)c->na, (unsigned)((as.max_s + (beta_j ? 1 : 0) + M - 1) / M));
   if (grid.y == 0) return;
   // whole lines of sigma for the copy engine: 16-byte starts
-  const int bulk = c->nb % 2 == 0 && ((uintptr_t)S & 15) == 0;
-  const MmaArgs a{C,
+  const int bulk = c->nb * sizeof(T) % 16 == 0 && ((uintptr_t)S & 15) == 0;
+  const MmaArgs<T> a{C,
                   S,
                   c->na,
                   c->nb,
@@ -413,8 +425,8 @@ void launch_mma(sbdgpu_ctx* c, const double* C, double* S, const AlphaSingles& a
                   (int)tb.n_tile_grp,
                   bulk,
                   beta_j ? c->ja : nullptr};
-  allow_dynamic_smem(reinterpret_cast<const void*>(ab_mma_kernel<M>), c->device);
-  ab_mma_kernel<M><<<grid, nt, mma_smem(c, M, nt), c->stream>>>(a);
+  allow_dynamic_smem(reinterpret_cast<const void*>(ab_mma_kernel<T, M>), c->device);
+  ab_mma_kernel<T, M><<<grid, nt, mma_smem(c, M, nt, sizeof(T)), c->stream>>>(a);
   SBD_CUDA(cudaGetLastError());
 }
 
@@ -458,7 +470,7 @@ void build_ab_tiles(sbdgpu_ctx* c, SpinTables& t, const std::vector<uint64_t>& s
 int ab_mma_group(const sbdgpu_ctx* c, int want, size_t budget) {
   if (!c->tab[1].tile_grp) return 0;
   for (int m : {16, 8})
-    if ((want == 0 || want == m) && mma_smem(c, m, 128) <= budget) return m;
+    if ((want == 0 || want == m) && mma_smem(c, m, 128, sizeof(double)) <= budget) return m;
   return 0;
 }
 
@@ -470,13 +482,14 @@ int ab_mma_group(const sbdgpu_ctx* c, int want, size_t budget) {
 // threads: 16M determinants 6.0 (256), 4.0 (512), 4.9 (768); 1501 x 803
 // strings 0.40 (128), 0.34 (256), 0.36 (512); 144M 107 (512), 101 (640),
 // 93 (768).
-void ab_mma(sbdgpu_ctx* c, const double* C, double* S, const AlphaSingles& as, int m, int nt, size_t budget,
+template <typename T>
+void ab_mma(sbdgpu_ctx* c, const T* C, T* S, const AlphaSingles& as, int m, int nt, size_t budget,
             bool beta_j) {
   if (nt == 0) {
     int best = 0;
     for (int t : {256, 512, 768, 1024}) {
-      if (mma_smem(c, m, t) > budget) break;
-      const int warps = (int)std::min<size_t>(228 * 1024 / (mma_smem(c, m, t) + 1024), 1024 / t) * (t / 32);
+      if (mma_smem(c, m, t, sizeof(T)) > budget) break;
+      const int warps = (int)std::min<size_t>(228 * 1024 / (mma_smem(c, m, t, sizeof(T)) + 1024), 1024 / t) * (t / 32);
       if (warps > best) {
         best = warps;
         nt = t;
@@ -486,16 +499,19 @@ void ab_mma(sbdgpu_ctx* c, const double* C, double* S, const AlphaSingles& as, i
     if (nt == 0) nt = 128;
     while (nt > 128 && (size_t)(nt / 2) >= c->tab[1].n_tile_grp * 32) nt /= 2;
   }
-  while (nt > 128 && mma_smem(c, m, nt) > budget) nt -= 128;  // a tuned number: the stages beside the row of C
+  while (nt > 128 && mma_smem(c, m, nt, sizeof(T)) > budget) nt -= 128;  // a tuned number: the stages beside the row of C
   if (m == 16)
-    launch_mma<16>(c, C, S, as, nt, beta_j);
+    launch_mma<T, 16>(c, C, S, as, nt, beta_j);
   else
-    launch_mma<8>(c, C, S, as, nt, beta_j);
+    launch_mma<T, 8>(c, C, S, as, nt, beta_j);
 }
 
+template void ab_mma<double>(sbdgpu_ctx*, const double*, double*, const AlphaSingles&, int, int, size_t, bool);
+template void ab_mma<float>(sbdgpu_ctx*, const float*, float*, const AlphaSingles&, int, int, size_t, bool);
+
 void preload_ab_mma(int device) {
-  allow_dynamic_smem(reinterpret_cast<const void*>(ab_mma_kernel<16>), device);
-  allow_dynamic_smem(reinterpret_cast<const void*>(ab_mma_kernel<8>), device);
+  allow_dynamic_smem(reinterpret_cast<const void*>(ab_mma_kernel<double, 16>), device);
+  allow_dynamic_smem(reinterpret_cast<const void*>(ab_mma_kernel<double, 8>), device);
 }
 
 }  // namespace sbdgpu

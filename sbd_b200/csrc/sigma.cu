@@ -16,8 +16,8 @@
 //
 // The rows kernel streams whole rows of C (coalesced) for every table entry of
 // its bra row.  The FP64 alpha-beta term runs on the FP64 tensor pipe
-// (ab_mma.cu).  The gather kernel here serves FP32 and the bases and launch
-// shapes the tiles do not: it holds one source row C[ja,:] and the integral
+// (ab_mma.cu), the FP32 one of large bases too.  The gather kernel here serves
+// the bases and launch shapes the tiles do not: it holds one source row C[ja,:] and the integral
 // rows (pq|.) of a group of ja's singles in shared memory, streams the beta
 // singles (sliced ELL, coalesced) once per group, and adds each group's
 // contributions to sigma rows ia with atomics.
@@ -412,7 +412,11 @@ namespace {
 // when set (sbdgpu_set_tuning / sbdgpu_autotune), else the largest group of
 // alpha singles per CTA whose integral block fits in shared memory next to
 // one row of C.  FP64 groups of 16 and 8 go to the tile kernel where the basis
-// has tiles; at groups of 4 and fewer a product would be half empty.
+// has tiles; at groups of 4 and fewer a product would be half empty.  The FP32
+// term is formed there too, in FP64 on the row of C converted, from half a
+// million determinants: 144M determinants 100 -> 85 ms, 16M 7.25 -> 4.46 ms,
+// 1501 x 803 strings 0.57 -> 0.33 ms; at 495 x 495 both take 0.05 ms.
+constexpr size_t kTilesFp32 = size_t(1) << 19;
 template <typename T>
 void alpha_beta(sbdgpu_ctx* c, const T* C, T* S, const T* vf, const AlphaSingles& as, bool beta_j = false) {
   int dev_smem = 0;
@@ -423,11 +427,12 @@ void alpha_beta(sbdgpu_ctx* c, const T* C, T* S, const T* vf, const AlphaSingles
   int P = c->P;
   const bool tuned = sizeof(T) == 8 && c->ab_group > 0;
   const int g = tuned ? c->ab_group : 0, nt = tuned ? c->ab_threads : 0;
-  if constexpr (sizeof(T) == 8)
+  if (sizeof(T) == 8 || c->N >= kTilesFp32) {
     if (const int m = ab_mma_group(c, g, budget)) {
-      ab_mma(c, C, S, as, m, nt, budget, beta_j);
+      ab_mma<T>(c, C, S, as, m, nt, budget, beta_j);
       return;
     }
+  }
   if ((g == 0 || g == 16) && ab_smem<T, 16>(nb, P) <= budget)
     launch_ab<T, 16>(c, C, S, vf, ab_smem<T, 16>(nb, P), as, nt);
   else if ((g == 0 || g == 8) && ab_smem<T, 8>(nb, P) <= budget)

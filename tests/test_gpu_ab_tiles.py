@@ -99,3 +99,20 @@ def test_non_finite_input_stays_where_the_operator_takes_it(bad):
     ref = orc.sigma(np.where(np.isfinite(C), C, 0.0).ravel())
     assert np.abs(s - ref)[unreached].max() <= TOL * np.abs(ref).max()
     ctx.close()
+
+
+@pytest.mark.parametrize("nb", [723, 726, 728])
+def test_fp32_sigma_by_tiles(nb):
+    # 731 x 723..728 determinants are past the rule's half million; rows of 4, 2 and 1 times 16 bytes
+    ints = synth.make_integrals(14, 6)
+    rng = np.random.default_rng(nb)
+    s = synth.full_strings(14, 5)
+    a, b = (s[np.sort(rng.choice(len(s), n, replace=False))] for n in (731, nb))
+    ctx = sbd_b200.context_from_integrals(ints, a, b)
+    C = rng.normal(size=ctx.n)
+    C /= np.linalg.norm(C)
+    ref = ctx.sigma(C)
+    got = ctx.sigma(C, precision=sbd_b200.MIXED)
+    # the bound of the mixed sigma's other tests against FP64
+    assert np.abs(got - ref).max() <= 2e-5 * np.abs(ref).max()
+    ctx.close()
