@@ -174,7 +174,7 @@ __device__ __forceinline__ void mma8(double (&d)[4], double a0, double b) {
 //
 // What bounds it: the shared-memory pipe (16M determinants: 86 % of its
 // wavefronts, the FP64 tensor pipe 68 % busy).  Alpha-beta term, gather kernel
-// -> tiles: 144M determinants 198 -> 93 ms, 16M 11.2 -> 4.0 ms, 1501 x 803
+// -> tiles: 144M determinants 198 -> 89 ms, 16M 11.2 -> 4.0 ms, 1501 x 803
 // strings 0.85 -> 0.34 ms, 495 x 495 0.10 -> 0.052 ms; the tensor pipe's floor
 // of the filled tiles is 54 / 2.8 ms at the first two.  24 and 32 alpha
 // singles per CTA (fewer loads of C per product) and entries fetched a batch
@@ -281,12 +281,12 @@ __device__ __forceinline__ void section(const E* __restrict__ p, int n, F&& step
   }
 }
 
-// The groups of 16 beta strings of one warp.  stage: the warp's [M][16] block
-// of results, whose rows are added to sigma as whole 128-byte lines: by the
+// The groups of 16 beta strings of one warp.  stage: the warp's [8 SB][16]
+// results of SB blocks of alpha singles, whose rows are added to sigma as whole 128-byte lines: by the
 // copy engine where they start on 16 bytes, else by coalesced atomics.  (Added
 // straight from the accumulators' layout, 8 rows x 2 columns per lane, the
 // atomics took 29 % of the shared-memory pipe's wavefronts.)
-template <typename T, int M, int BLOCKS>
+template <typename T, int M, int BLOCKS, int SB>
 __device__ __forceinline__ void tiles(const MmaArgs<T>& a, const unsigned char* vsub, const unsigned char* crow,
                                       T* stage, const int* tgt, const uint32_t* neg) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
@@ -311,30 +311,35 @@ __device__ __forceinline__ void tiles(const MmaArgs<T>& a, const unsigned char* 
     alone(p + (size_t)64 * d.y + lane, d.z, acc0);
     alone(p + (size_t)64 * d.y + (size_t)32 * d.z + lane, d.w, acc1);
     const size_t ib0 = (size_t)g * 16;
-    if (a.bulk) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // the last lines are read
-    __syncwarp();
 #pragma unroll
-    for (int b = 0; b < BLOCKS; b++) {
-      const uint32_t sg = neg[8 * b + r];
-      const auto val = [&](double x) { return (T)__hiloint2double(__double2hiint(x) ^ (int)sg, __double2loint(x)); };
-      using V = typename std::conditional<sizeof(T) == 8, double2, float2>::type;
-      T* row = stage + (8 * b + r) * 16 + 2 * q;
-      *reinterpret_cast<V*>(row) = V{val(acc0[2 * b]), val(acc0[2 * b + 1])};
-      *reinterpret_cast<V*>(row + 8) = V{val(acc1[2 * b]), val(acc1[2 * b + 1])};
-    }
-    if (a.bulk) {
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    for (int b0 = 0; b0 < BLOCKS; b0 += SB) {
+      constexpr int ROWS = 8 * (SB < BLOCKS ? SB : BLOCKS);
+      if (a.bulk) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // the last lines are read
       __syncwarp();
-      if (lane < 8 * BLOCKS && tgt[lane] >= 0)
-        bulk_add(a.S + (size_t)tgt[lane] * a.nb + ib0, smem_addr(stage + lane * 16),
-                 (uint32_t)min((size_t)16, a.nb - ib0) * (uint32_t)sizeof(T));
-      asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-    } else {
-      __syncwarp();
-      const size_t ib = ib0 + (lane & 15);
+#pragma unroll
+      for (int b = b0; b < b0 + SB && b < BLOCKS; b++) {
+        const uint32_t sg = neg[8 * b + r];
+        const auto val = [&](double x) { return (T)__hiloint2double(__double2hiint(x) ^ (int)sg, __double2loint(x)); };
+        using V = typename std::conditional<sizeof(T) == 8, double2, float2>::type;
+        T* row = stage + (8 * (b - b0) + r) * 16 + 2 * q;
+        *reinterpret_cast<V*>(row) = V{val(acc0[2 * b]), val(acc0[2 * b + 1])};
+        *reinterpret_cast<V*>(row + 8) = V{val(acc1[2 * b]), val(acc1[2 * b + 1])};
+      }
+      const int* to = tgt + 8 * b0;
+      if (a.bulk) {
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane < ROWS && to[lane] >= 0)
+          bulk_add(a.S + (size_t)to[lane] * a.nb + ib0, smem_addr(stage + lane * 16),
+                   (uint32_t)min((size_t)16, a.nb - ib0) * (uint32_t)sizeof(T));
+        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+      } else {
+        __syncwarp();
+        const size_t ib = ib0 + (lane & 15);
 #pragma unroll 4
-      for (int row = lane >> 4; row < 8 * BLOCKS; row += 2)
-        if (tgt[row] >= 0 && ib < a.nb) atomicAdd(a.S + (size_t)tgt[row] * a.nb + ib, stage[row * 16 + (lane & 15)]);
+        for (int row = lane >> 4; row < ROWS; row += 2)
+          if (to[row] >= 0 && ib < a.nb) atomicAdd(a.S + (size_t)to[row] * a.nb + ib, stage[row * 16 + (lane & 15)]);
+      }
     }
   }
   if (a.bulk) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
@@ -350,14 +355,14 @@ __device__ __forceinline__ void tiles(const MmaArgs<T>& a, const unsigned char* 
 // alpha singles' Coulomb part J_pq[ib] C[ja,ib] as the value a row's sums start
 // from cost 20 ms more, 5.4 against 4.0 ms at 16M: its loads stall the warps and
 // take shared-memory wavefronts.  It stays a pass of its own.)
-template <typename T, int M>
+template <typename T, int M, int SB>
 __global__ void __launch_bounds__(kMmaThreads) ab_mma_kernel(const MmaArgs<T> a) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ int tgt[M];
   __shared__ uint32_t neg[M];
   unsigned char* vsub = smem;                                                          // [npair][M] integrals
-  T* stage = reinterpret_cast<T*>(smem + (size_t)a.npair * M * 8);                     // [warps][M][16] results
-  double* crow = reinterpret_cast<double*>(stage + (size_t)(blockDim.x >> 5) * M * 16);  // [nb + 1]
+  T* stage = reinterpret_cast<T*>(smem + (size_t)a.npair * M * 8);                     // [warps][8 SB][16] results
+  double* crow = reinterpret_cast<double*>(stage + (size_t)(blockDim.x >> 5) * SB * 128);  // [nb + 1]
   const size_t ja = blockIdx.x;
   const int64_t k0 = a.a_off[ja] + (int64_t)blockIdx.y * M;
   const int singles = (int)min((int64_t)M, a.a_off[ja + 1] - k0);  // negative past the last ones
@@ -385,12 +390,12 @@ __global__ void __launch_bounds__(kMmaThreads) ab_mma_kernel(const MmaArgs<T> a)
           vrow ? __ldg(&vrow[(size_t)folded_pair(o) * step]) : 0.0;
   }
   __syncthreads();
-  T* mine = stage + (size_t)warp * M * 16;
+  T* mine = stage + (size_t)warp * SB * 128;
   const unsigned char* cr = reinterpret_cast<const unsigned char*>(crow);
   if (M == 16 && count > 8)
-    tiles<T, M, M / 8>(a, vsub, cr, mine, tgt, neg);
+    tiles<T, M, M / 8, SB>(a, vsub, cr, mine, tgt, neg);
   else
-    tiles<T, M, 1>(a, vsub, cr, mine, tgt, neg);
+    tiles<T, M, 1, SB>(a, vsub, cr, mine, tgt, neg);
 }
 
 }  // namespace
@@ -398,11 +403,11 @@ __global__ void __launch_bounds__(kMmaThreads) ab_mma_kernel(const MmaArgs<T> a)
 namespace {
 
 // dynamic shared memory: integrals, per-warp stages, the row of C
-size_t mma_smem(const sbdgpu_ctx* c, int m, int threads, size_t elem) {
-  return sizeof(double) * ((size_t)(c->L * (c->L - 1) / 2) * m + (c->nb + 1)) + elem * (threads / 32) * m * 16;
+size_t mma_smem(const sbdgpu_ctx* c, int m, int threads, size_t elem, int sb) {
+  return sizeof(double) * ((size_t)(c->L * (c->L - 1) / 2) * m + (c->nb + 1)) + elem * (threads / 32) * sb * 128;
 }
 
-template <typename T, int M>
+template <typename T, int M, int SB>
 void launch_mma(sbdgpu_ctx* c, const T* C, T* S, const AlphaSingles& as, int nt, bool beta_j) {
   const SpinTables& tb = c->tab[1];
   const dim3 grid((unsigned)c->na, (unsigned)((as.max_s + (beta_j ? 1 : 0) + M - 1) / M));
@@ -425,8 +430,8 @@ void launch_mma(sbdgpu_ctx* c, const T* C, T* S, const AlphaSingles& as, int nt,
                   (int)tb.n_tile_grp,
                   bulk,
                   beta_j ? c->ja : nullptr};
-  allow_dynamic_smem(reinterpret_cast<const void*>(ab_mma_kernel<T, M>), c->device);
-  ab_mma_kernel<T, M><<<grid, nt, mma_smem(c, M, nt, sizeof(T)), c->stream>>>(a);
+  allow_dynamic_smem(reinterpret_cast<const void*>(ab_mma_kernel<T, M, SB>), c->device);
+  ab_mma_kernel<T, M, SB><<<grid, nt, mma_smem(c, M, nt, sizeof(T), SB), c->stream>>>(a);
   SBD_CUDA(cudaGetLastError());
 }
 
@@ -470,48 +475,59 @@ void build_ab_tiles(sbdgpu_ctx* c, SpinTables& t, const std::vector<uint64_t>& s
 int ab_mma_group(const sbdgpu_ctx* c, int want, size_t budget) {
   if (!c->tab[1].tile_grp) return 0;
   for (int m : {16, 8})
-    if ((want == 0 || want == m) && mma_smem(c, m, 128, sizeof(double)) <= budget) return m;
+    if ((want == 0 || want == m) && mma_smem(c, m, 128, sizeof(double), 1) <= budget) return m;
   return 0;
 }
 
 // The alpha-beta term by tiles, m alpha singles per CTA, nt threads (0: the
 // default); beta_j: the beta singles' Coulomb part as well (whole vectors
-// only).  Default threads: the fewest of 256, 512, 1024 that put 24 warps
-// on an SM beside the shared memory they need, else the number that puts most
-// there; fewer while the warps outnumber the groups.  Alpha-beta ms by
-// threads: 16M determinants 6.0 (256), 4.0 (512), 4.9 (768); 1501 x 803
-// strings 0.40 (128), 0.34 (256), 0.36 (512); 144M 107 (512), 101 (640),
-// 93 (768).
+// only).  Default threads: those that put most warps on an SM beside the shared
+// memory they need (at equal warps the smaller CTA), fewer while the warps
+// outnumber the groups; results are staged for one block of alpha singles at a
+// time where that lets more warps in.  Alpha-beta ms: 16M determinants 6.0 at
+// 256 threads, 4.6 at 512, 5.6 at 768; 1501 x 803 strings 0.40 at 128, 0.34 at
+// 256, 0.37 at 512; 144M 93 at 768 with both blocks staged, 97 and 88.6 at 768
+// and 1,024 with one (FP32 vectors: 82 at 768, 77 at 1,024).
 template <typename T>
-void ab_mma(sbdgpu_ctx* c, const T* C, T* S, const AlphaSingles& as, int m, int nt, size_t budget,
-            bool beta_j) {
+void ab_mma(sbdgpu_ctx* c, const T* C, T* S, const AlphaSingles& as, int m, int nt, size_t budget, bool beta_j) {
+  int sb = m / 8;
   if (nt == 0) {
     int best = 0;
-    for (int t : {256, 512, 768, 1024}) {
-      if (mma_smem(c, m, t, sizeof(T)) > budget) break;
-      const int warps = (int)std::min<size_t>(228 * 1024 / (mma_smem(c, m, t, sizeof(T)) + 1024), 1024 / t) * (t / 32);
-      if (warps > best) {
-        best = warps;
-        nt = t;
+    for (int b = m / 8; b >= 1; b--)
+      for (int t : {256, 512, 768, 1024}) {
+        const size_t smem = mma_smem(c, m, t, sizeof(T), b);
+        if (smem > budget) break;
+        const int warps = (int)std::min<size_t>(228 * 1024 / (smem + 1024), 1024 / t) * (t / 32);
+        if (warps > best) {
+          best = warps;
+          nt = t;
+          sb = b;
+        }
       }
-      if (warps >= 24) break;
+    if (nt == 0) {
+      nt = 128;
+      sb = 1;
     }
-    if (nt == 0) nt = 128;
     while (nt > 128 && (size_t)(nt / 2) >= c->tab[1].n_tile_grp * 32) nt /= 2;
+  } else {  // a tuned number: as many stages as fit beside the row of C
+    if (mma_smem(c, m, nt, sizeof(T), sb) > budget) sb = 1;
+    while (nt > 128 && mma_smem(c, m, nt, sizeof(T), sb) > budget) nt -= 128;
   }
-  while (nt > 128 && mma_smem(c, m, nt, sizeof(T)) > budget) nt -= 128;  // a tuned number: the stages beside the row of C
-  if (m == 16)
-    launch_mma<T, 16>(c, C, S, as, nt, beta_j);
+  if (m == 16 && sb == 2)
+    launch_mma<T, 16, 2>(c, C, S, as, nt, beta_j);
+  else if (m == 16)
+    launch_mma<T, 16, 1>(c, C, S, as, nt, beta_j);
   else
-    launch_mma<T, 8>(c, C, S, as, nt, beta_j);
+    launch_mma<T, 8, 1>(c, C, S, as, nt, beta_j);
 }
 
 template void ab_mma<double>(sbdgpu_ctx*, const double*, double*, const AlphaSingles&, int, int, size_t, bool);
 template void ab_mma<float>(sbdgpu_ctx*, const float*, float*, const AlphaSingles&, int, int, size_t, bool);
 
 void preload_ab_mma(int device) {
-  allow_dynamic_smem(reinterpret_cast<const void*>(ab_mma_kernel<double, 16>), device);
-  allow_dynamic_smem(reinterpret_cast<const void*>(ab_mma_kernel<double, 8>), device);
+  allow_dynamic_smem(reinterpret_cast<const void*>(ab_mma_kernel<double, 16, 2>), device);
+  allow_dynamic_smem(reinterpret_cast<const void*>(ab_mma_kernel<double, 16, 1>), device);
+  allow_dynamic_smem(reinterpret_cast<const void*>(ab_mma_kernel<double, 8, 1>), device);
 }
 
 }  // namespace sbdgpu

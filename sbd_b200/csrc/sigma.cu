@@ -414,7 +414,7 @@ namespace {
 // one row of C.  FP64 groups of 16 and 8 go to the tile kernel where the basis
 // has tiles; at groups of 4 and fewer a product would be half empty.  The FP32
 // term is formed there too, in FP64 on the row of C converted, from half a
-// million determinants: 144M determinants 100 -> 85 ms, 16M 7.25 -> 4.46 ms,
+// million determinants: 144M determinants 100 -> 77 ms, 16M 7.25 -> 4.46 ms,
 // 1501 x 803 strings 0.57 -> 0.33 ms; at 495 x 495 both take 0.05 ms.
 constexpr size_t kTilesFp32 = size_t(1) << 19;
 template <typename T>
