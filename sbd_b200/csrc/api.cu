@@ -57,12 +57,19 @@ void allow_dynamic_smem(const void* func, int device) {
 
 void ensure_scratch(sbdgpu_ctx* c) {
   if (!c->red) c->red = (double*)dev_alloc(sizeof(double) * 1024);
+}
+
+void ensure_ct(sbdgpu_ctx* c) {
   if (!c->ct) c->ct = (double*)dev_alloc(sizeof(double) * c->N);
   if (!c->st) c->st = (double*)dev_alloc(sizeof(double) * c->N);
 }
 
-void ensure_io(sbdgpu_ctx* c) {
+void ensure_io_a(sbdgpu_ctx* c) {
   if (!c->io_a) c->io_a = (double*)dev_alloc(sizeof(double) * c->N);
+}
+
+void ensure_io(sbdgpu_ctx* c) {
+  ensure_io_a(c);
   if (!c->io_b) c->io_b = (double*)dev_alloc(sizeof(double) * c->N);
 }
 
@@ -148,7 +155,7 @@ void check_precision(int precision) {
 
 void sigma_ref_convention(sbdgpu_ctx* c, const double* dC, double* dS, int precision = SBDGPU_FP64) {
   // dC, dS in the reference (interleaved) sign convention
-  ensure_io(c);
+  sbdgpu::ensure_io_a(c);
   sbdgpu::build_tables(c);
   sbdgpu::compute_hii(c);
   sbdgpu::ensure_scratch(c);

@@ -213,6 +213,8 @@ void davidson_batch_fp64(int nprob, sbdgpu_ctx* const* ctxs, const sbdgpu_opts* 
     build_tables(c);
     compute_hii(c);
     ensure_scratch(c);
+    ensure_dense_fp64(c);  // its sigma takes no integer products
+    if (sigma_fp64_needs_ct(c)) ensure_ct(c);
     P[i].c = c;
     P[i].n = c->N;
     P[i].nb = nb;
@@ -398,6 +400,7 @@ extern "C" int sbdgpu_autotune(sbdgpu_ctx* c, int reps, int* ab_group, int* ab_t
     sbdgpu::build_tables(c);
     sbdgpu::compute_hii(c);
     sbdgpu::ensure_scratch(c);
+    sbdgpu::ensure_ct(c);
     sbdgpu::ensure_io(c);
     sbdgpu::preload_fp64_sigma(c->device);
     cudaStream_t st = c->stream;

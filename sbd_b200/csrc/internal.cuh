@@ -63,10 +63,12 @@ struct SpinTables {
   int64_t* sell_off = nullptr;  // [nslice+1]
   int32_t* sell_w = nullptr;    // [nslice]
   uint32_t* sell = nullptr;
-  // n8 x k4 tiles of the singles for the FP64 tensor pipe (ab_mma.cu): per 16
-  // bras {first entry / 32, k4 steps of both tiles, of the first, of the second}
+  // n8 x k4 tiles of the singles for the FP64 tensor pipe (ab_mma.cu): per two
+  // tiles {first entry / 32, k4 steps of both tiles, of the first, of the
+  // second} and {first bra, the tiles' lengths}
   size_t n_tile_grp = 0;
   int4* tile_grp = nullptr;
+  int2* tile_pos = nullptr;  // in tile_grp's allocation
   uint32_t* tile_ent = nullptr;
   std::vector<int64_t> h_s_off, h_d_off;  // host copies of the offsets
 };
@@ -215,6 +217,7 @@ void preload_ab_mma(int device);
 // ozaki.cu: the FP64 same-spin terms as exact INT8 products
 bool ensure_ozaki(sbdgpu_ctx* c);
 void free_ozaki(sbdgpu_ctx* c);
+bool wants_ozaki(const sbdgpu_ctx* c);
 bool use_ozaki(sbdgpu_ctx* c);
 bool same_spin_ozaki_fp64(sbdgpu_ctx* c, const double* C, double* S, double* ct, double* st, bool events,
                           bool beta_j);
@@ -289,6 +292,7 @@ void davidson_roots(sbdgpu_ctx* c, const sbdgpu_opts* o, int nroots, double* Wh,
 void preload_fp64_sigma(int device);
 void preload_fp64_sigma_misc();  // misc.cu
 void sigma_fp64(sbdgpu_ctx* c, const double* C, double* S);
+bool sigma_fp64_needs_ct(const sbdgpu_ctx* c);  // for its ct and st
 void sigma_fp64_prepared(sbdgpu_ctx* c, const double* C, double* S, double* ct, double* st);
 void sigma_fp32(sbdgpu_ctx* c, const float* C, float* S);
 void sigma_fp32_tc(sbdgpu_ctx* c, const float* C, float* S);
@@ -312,8 +316,10 @@ void learned_get(sbdgpu_ctx* c, float* w, int* n);
 void learned_set(sbdgpu_ctx* c, const float* w, int n);
 
 // api.cu
-void ensure_scratch(sbdgpu_ctx* c);
-void ensure_io(sbdgpu_ctx* c);
+void ensure_scratch(sbdgpu_ctx* c);  // the reductions'
+void ensure_ct(sbdgpu_ctx* c);       // ct and st
+void ensure_io_a(sbdgpu_ctx* c);
+void ensure_io(sbdgpu_ctx* c);  // io_a and io_b
 void jacobi_eig(int n, double* A, int lda, double* w);
 void* dev_alloc(size_t bytes);
 void allow_dynamic_smem(const void* func, int device);

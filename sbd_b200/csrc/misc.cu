@@ -280,7 +280,9 @@ void compute_hii(sbdgpu_ctx* c) {
   dim3 g((unsigned)c->na, (unsigned)((c->nb + 255) / 256));
   hii_kernel<<<g, 256, 0, c->stream>>>(c->astr, c->na, c->nb, Ea, Eb, c->jb, c->P, c->ecore, c->hii);
   SBD_CUDA(cudaGetLastError());
-  ensure_dense_fp64(c);  // with the set-up, so that the no-allocation sigma finds it
+  // with the set-up, so that the no-allocation sigma finds it (its bases are too
+  // small for the integer products)
+  if (!wants_ozaki(c)) ensure_dense_fp64(c);
   SBD_CUDA(cudaStreamSynchronize(c->stream));
   cudaFree(Ea);
   c->hii_ready = true;

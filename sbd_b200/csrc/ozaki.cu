@@ -130,26 +130,31 @@ __device__ __forceinline__ void store_all_residues(std::index_sequence<L...>, co
   (store_residues4<(int)L>(hu, lo, out, n, at), ...);
 }
 
-// symmetric residues modulo the primes of round(X * 2^e_row), int8,
-// [kMods][rows*cols]; one block per row, four consecutive entries per thread
-// (cols a multiple of 4)
-__global__ void __launch_bounds__(kT) residue_kernel(const double* __restrict__ X, size_t rows, size_t cols,
-                                                    const int* __restrict__ e, int8_t* __restrict__ out) {
-  const size_t n = rows * cols, row = blockIdx.x;
+// symmetric residues modulo the primes of round(X * 2^e_row), int8, planes of
+// `plane` bytes with rows of ld (a multiple of 16, zeros past cols); one block
+// per row of the rows x cols matrix X, four consecutive entries per thread
+// (vec: its rows are 16-byte aligned)
+__global__ void __launch_bounds__(kT) residue_kernel(const double* __restrict__ X, size_t cols, size_t ld, size_t plane,
+                                                    bool vec, const int* __restrict__ e, int8_t* __restrict__ out) {
+  const size_t row = blockIdx.x;
   const int er = e[row];
   const double scale = er == kNonFinite ? 0.0 : pow2(er);  // e <= kMaxExp; >= kBits - 1024
   const double* xr = X + row * cols;
-  for (size_t c = 4 * (size_t)threadIdx.x; c < cols; c += 4 * kT) {
-    double x[4];
+  for (size_t c = 4 * (size_t)threadIdx.x; c < ld; c += 4 * kT) {
+    double x[4] = {0.0, 0.0, 0.0, 0.0};
     if (er == kNonFinite) {
-      x[0] = x[1] = x[2] = x[3] = 0.0;  // residues 0: the reconstruction writes NaN for this row
-    } else {
+      // residues 0: the reconstruction writes NaN for this row
+    } else if (vec && c + 4 <= cols) {
       const double2 x01 = *reinterpret_cast<const double2*>(xr + c);
       const double2 x23 = *reinterpret_cast<const double2*>(xr + c + 2);
       x[0] = x01.x;
       x[1] = x01.y;
       x[2] = x23.x;
       x[3] = x23.y;
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; j++)
+        if (c + j < cols) x[j] = xr[c + j];
     }
     unsigned hu[4], lo[4];
 #pragma unroll
@@ -158,7 +163,7 @@ __global__ void __launch_bounds__(kT) residue_kernel(const double* __restrict__ 
       hu[j] = (unsigned)((y >> 25) + (1LL << 24));     // in [0, 2^25)
       lo[j] = (unsigned)(y & 0x1FFFFFFLL);
     }
-    store_all_residues(std::make_index_sequence<kMods>{}, hu, lo, out, n, row * cols + c);
+    store_all_residues(std::make_index_sequence<kMods>{}, hu, lo, out, plane, row * ld + c);
   }
 }
 
@@ -182,18 +187,18 @@ __device__ __forceinline__ double u128_to_double(unsigned __int128 x) {
   return (double)(unsigned long long)(x >> 64) * 18446744073709551616.0 + (double)(unsigned long long)x;
 }
 
-// S[row][col] += (integer product, from its residues) * 2^-(e_row + e_col);
-// one block per row
-__global__ void __launch_bounds__(kT) crt_add_kernel(const int32_t* __restrict__ P, size_t rows, size_t cols,
-                                                    const int* __restrict__ e_row, const int* __restrict__ e_col,
+// S[row][col] += (integer product, from its residues in planes of `plane`
+// entries with rows of ld) * 2^-(e_row + e_col); one block per row
+__global__ void __launch_bounds__(kT) crt_add_kernel(const int32_t* __restrict__ P, size_t plane, size_t ld,
+                                                    size_t cols, const int* __restrict__ e_row, const int* __restrict__ e_col,
                                                     double* __restrict__ S) {
-  const size_t n = rows * cols, row = blockIdx.x;
+  const size_t row = blockIdx.x;
   const int er = e_row[row];
   const unsigned __int128 M = ((unsigned __int128)c_Mhi << 64) | c_Mlo;
   for (size_t c = threadIdx.x; c < cols; c += kT) {
     const size_t i = row * cols + c;
     unsigned long long a[4] = {0, 0, 0, 0};
-    crt_all(std::make_index_sequence<kMods>{}, P, n, i, a);
+    crt_all(std::make_index_sequence<kMods>{}, P, plane, row * ld + c, a);
     // carries: acc = sum_l r_l w_l < kMods * 251 * M < 2^128
     a[1] += a[0] >> 32;
     a[2] += a[1] >> 32;
@@ -282,6 +287,11 @@ void upload_crt_constants() {
   SBD_CUDA(cudaMemcpyToSymbol(c_Minv, &minv, sizeof(minv)));
 }
 
+// Rows and depths of the INT8 products are padded to multiples of 16 with zero
+// residues: cuBLAS falls to a kernel an order of magnitude slower on leading
+// dimensions that are not (3,000 x 3,000 strings: 7.5 ms for both spins' terms).
+constexpr size_t pad16(size_t n) { return (n + 15) & ~size_t(15); }
+
 // INT8 GEMM, column-major: out (m x n, int32) = op(A) op(B); false when
 // cuBLAS does not offer it
 bool gemm_i8(cublasHandle_t h, cublasOperation_t ta, cublasOperation_t tb, int m, int n, int k, const int8_t* A,
@@ -299,8 +309,9 @@ bool gemm_i8(cublasHandle_t h, cublasOperation_t ta, cublasOperation_t tb, int m
 bool ensure_ozaki(sbdgpu_ctx* c) {
   if (c->oz.ready) return true;
   if (c->oz.failed) return false;
-  const size_t na = c->na, nb = c->nb, N = c->N, nmax = std::max(na, nb);
-  const size_t bytes = (size_t)kMods * (na * na + nb * nb) + 2 * (size_t)kMods * N + 4 * (size_t)kMods * N +
+  const size_t na = c->na, nb = c->nb, nmax = std::max(na, nb);
+  const size_t pa = pad16(na), pb = pad16(nb), plane = pa * pb;
+  const size_t bytes = (size_t)kMods * (pa * pa + pb * pb) + 2 * (size_t)kMods * plane + 4 * (size_t)kMods * plane +
                        sizeof(double) * nmax * nmax;
   size_t free_b = 0, total_b = 0;
   SBD_CUDA(cudaMemGetInfo(&free_b, &total_b));
@@ -310,6 +321,7 @@ bool ensure_ozaki(sbdgpu_ctx* c) {
   }
   build_tables(c);
   ensure_scratch(c);
+  ensure_ct(c);
   upload_crt_constants();
   cudaStream_t st = c->stream;
   double* tmp = (double*)dev_alloc(sizeof(double) * nmax * nmax);
@@ -320,8 +332,10 @@ bool ensure_ozaki(sbdgpu_ctx* c) {
       dense_h0_kernel<<<(unsigned)n, kT, 0, st>>>(n, t.s_off, t.s_idx, t.s_val, t.d_off, t.d_idx, t.d_val, tmp);
       c->oz.h0e[spin] = (int*)dev_alloc(sizeof(int) * n);
       row_exp_kernel<<<(unsigned)n, kT, 0, st>>>(tmp, n, c->oz.h0e[spin]);
-      c->oz.h0r[spin] = (int8_t*)dev_alloc((size_t)kMods * n * n);
-      residue_kernel<<<(unsigned)n, kT, 0, st>>>(tmp, n, n, c->oz.h0e[spin], c->oz.h0r[spin]);
+      const size_t p = pad16(n);
+      c->oz.h0r[spin] = (int8_t*)dev_alloc((size_t)kMods * p * p);
+      if (p != n) SBD_CUDA(cudaMemsetAsync(c->oz.h0r[spin], 0, (size_t)kMods * p * p, st));
+      residue_kernel<<<(unsigned)n, kT, 0, st>>>(tmp, n, p, p * p, n % 2 == 0, c->oz.h0e[spin], c->oz.h0r[spin]);
       SBD_CUDA(cudaGetLastError());
       SBD_CUDA(cudaStreamSynchronize(st));
     }
@@ -332,11 +346,15 @@ bool ensure_ozaki(sbdgpu_ctx* c) {
   }
   cudaFree(tmp);
   try {
-    c->oz.cr = (int8_t*)dev_alloc((size_t)kMods * N);
-    c->oz.ctr = (int8_t*)dev_alloc((size_t)kMods * N);
+    c->oz.cr = (int8_t*)dev_alloc((size_t)kMods * plane);
+    c->oz.ctr = (int8_t*)dev_alloc((size_t)kMods * plane);
+    if (plane != c->N) {  // the rows past the last string stay zero
+      SBD_CUDA(cudaMemsetAsync(c->oz.cr, 0, (size_t)kMods * plane, st));
+      SBD_CUDA(cudaMemsetAsync(c->oz.ctr, 0, (size_t)kMods * plane, st));
+    }
     c->oz.ce = (int*)dev_alloc(sizeof(int) * na);
     c->oz.cte = (int*)dev_alloc(sizeof(int) * nb);
-    c->oz.prod = (int32_t*)dev_alloc(sizeof(int32_t) * (size_t)kMods * N);
+    c->oz.prod = (int32_t*)dev_alloc(sizeof(int32_t) * (size_t)kMods * plane);
     if (!c->blas) {
       cublasHandle_t h = nullptr;
       if (cublasCreate(&h) != CUBLAS_STATUS_SUCCESS) throw Error{SBDGPU_ERR_CUDA, "cublasCreate failed"};
@@ -369,14 +387,22 @@ void free_ozaki(sbdgpu_ctx* c) {
   c->oz.ready = false;
 }
 
-// Whether the FP64 sigma takes its same-spin terms from the integer products:
-// the context's choice (c->oz.mode: 0 automatic, 1 never), at least 1,024
-// strings per spin, leading dimensions the INT8 GEMMs take (multiples of 4)
-// and room in device memory.
-bool use_ozaki(sbdgpu_ctx* c) {
-  if (c->oz.mode == 1 || c->oz.failed || c->na < 1024 || c->nb < 1024 || c->na % 4 || c->nb % 4) return false;
-  return ensure_ozaki(c);
+// Whether the FP64 sigma takes its same-spin terms from the integer products by
+// its size and the context's choice (c->oz.mode: 0 automatic, 1 never): at
+// least 1,024 strings per spin; where the counts are not multiples of 4 only
+// beside alpha-beta tiles (the singles' pass for the beta strings moves pairs
+// of columns), and not while the dense FP64 product is faster: both take 1.4 ms
+// per sigma at 1,600 x 1,600 strings, at 2,000 x 2,000 the integers take 2.1
+// and the dense product 2.5.
+bool wants_ozaki(const sbdgpu_ctx* c) {
+  if (c->oz.mode == 1 || c->oz.failed || c->na < 1024 || c->nb < 1024) return false;
+  if (c->na % 4 == 0 && c->nb % 4 == 0) return true;
+  return c->tab[1].tile_grp &&
+         !(dense_same_spin(c) && (double)c->na * c->nb * (c->na + c->nb) < 8.2e9);
 }
+
+// As wants_ozaki, with room in device memory.
+bool use_ozaki(sbdgpu_ctx* c) { return wants_ozaki(c) && ensure_ozaki(c); }
 
 // sigma (FP64) = hii C + same-spin terms (the alpha-beta term is added after);
 // beta_j: the beta singles' Coulomb part too (else the alpha-beta tiles bring
@@ -386,36 +412,38 @@ bool use_ozaki(sbdgpu_ctx* c) {
 bool same_spin_ozaki_fp64(sbdgpu_ctx* c, const double* C, double* S, double* ct, double* st, bool events,
                           bool beta_j) {
   cudaStream_t s = c->stream;
-  const size_t na = c->na, nb = c->nb, N = c->N;
+  const size_t na = c->na, nb = c->nb, pa = pad16(na), pb = pad16(nb), plane = pa * pb;
   const SpinTables& tb = c->tab[1];
   cublasHandle_t h = static_cast<cublasHandle_t>(c->blas);
-  if (((uintptr_t)C | (uintptr_t)S) & 15) return false;  // the kernels move pairs of doubles
+  // jsingles64_kernel moves pairs of doubles
+  if (beta_j && (na % 2 || nb % 2 || (((uintptr_t)C | (uintptr_t)S) & 15))) return false;
   SBD_CUDA(cudaGetLastError());
   if (events) SBD_CUDA(cudaEventRecord(c->ev[0], s));
   // scaled residues of C (rows: for the beta product) and of C^T (for the alpha product)
   transpose(C, ct, na, nb, s);
   row_exp_kernel<<<(unsigned)na, kT, 0, s>>>(C, nb, c->oz.ce);
   row_exp_kernel<<<(unsigned)nb, kT, 0, s>>>(ct, na, c->oz.cte);
-  residue_kernel<<<(unsigned)na, kT, 0, s>>>(C, na, nb, c->oz.ce, c->oz.cr);
-  residue_kernel<<<(unsigned)nb, kT, 0, s>>>(ct, nb, na, c->oz.cte, c->oz.ctr);
+  residue_kernel<<<(unsigned)na, kT, 0, s>>>(C, nb, pb, plane, nb % 2 == 0 && ((uintptr_t)C & 15) == 0, c->oz.ce,
+                                             c->oz.cr);
+  residue_kernel<<<(unsigned)nb, kT, 0, s>>>(ct, na, pa, plane, na % 2 == 0, c->oz.cte, c->oz.ctr);
   SBD_CUDA(cudaGetLastError());
   // alpha: sigma^T (nb x na, column-major) = (C^T)(H0a^T), one INT8 product per prime
   for (int l = 0; l < kMods; l++)
-    if (!gemm_i8(h, CUBLAS_OP_T, CUBLAS_OP_N, (int)nb, (int)na, (int)na, c->oz.ctr + (size_t)l * N, (int)na,
-                 c->oz.h0r[0] + (size_t)l * na * na, (int)na, c->oz.prod + (size_t)l * N, (int)nb)) {
+    if (!gemm_i8(h, CUBLAS_OP_T, CUBLAS_OP_N, (int)pb, (int)pa, (int)pa, c->oz.ctr + (size_t)l * plane, (int)pa,
+                 c->oz.h0r[0] + (size_t)l * pa * pa, (int)pa, c->oz.prod + (size_t)l * plane, (int)pb)) {
       c->oz.failed = true;
       return false;
     }
   alpha_coulomb(c, C, S);
-  crt_add_kernel<<<(unsigned)na, kT, 0, s>>>(c->oz.prod, na, nb, c->oz.h0e[0], c->oz.cte, S);
+  crt_add_kernel<<<(unsigned)na, kT, 0, s>>>(c->oz.prod, plane, pb, nb, c->oz.h0e[0], c->oz.cte, S);
   SBD_CUDA(cudaGetLastError());
   if (events) SBD_CUDA(cudaEventRecord(c->ev[1], s));
   // beta: sigma^T = H0b (C^T), with H0b's rows and C's rows scaled
   for (int l = 0; l < kMods; l++)
-    if (!gemm_i8(h, CUBLAS_OP_T, CUBLAS_OP_N, (int)nb, (int)na, (int)nb, c->oz.h0r[1] + (size_t)l * nb * nb, (int)nb,
-                 c->oz.cr + (size_t)l * N, (int)nb, c->oz.prod + (size_t)l * N, (int)nb))
+    if (!gemm_i8(h, CUBLAS_OP_T, CUBLAS_OP_N, (int)pb, (int)pa, (int)pb, c->oz.h0r[1] + (size_t)l * pb * pb, (int)pb,
+                 c->oz.cr + (size_t)l * plane, (int)pb, c->oz.prod + (size_t)l * plane, (int)pb))
       throw Error{SBDGPU_ERR_CUDA, "INT8 product refused after the alpha products ran"};
-  crt_add_kernel<<<(unsigned)na, kT, 0, s>>>(c->oz.prod, na, nb, c->oz.ce, c->oz.h0e[1], S);
+  crt_add_kernel<<<(unsigned)na, kT, 0, s>>>(c->oz.prod, plane, pb, nb, c->oz.ce, c->oz.h0e[1], S);
   SBD_CUDA(cudaGetLastError());
   if (beta_j) {
     jsingles64_kernel<<<dim3((unsigned)nb, (unsigned)((na + 2 * kT - 1) / (2 * kT))), kT, 0, s>>>(

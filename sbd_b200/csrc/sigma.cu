@@ -454,6 +454,10 @@ bool uses_tiles(const sbdgpu_ctx* c) {
   return ab_mma_group(c, c->ab_group, (size_t)dev_smem - 1024) > 0;
 }
 
+// Whether its same-spin terms are the dense product (else, or before that, the
+// integer products): no transposes, no ct and st.
+bool dense_path(const sbdgpu_ctx* c) { return c->dense[0] && c->oz.mode == 0 && uses_tiles(c); }
+
 // The full kernel sequence of one sigma on given scratch (ct, st: na*nb of T).
 template <typename T>
 void sigma_launch(sbdgpu_ctx* c, const T* C, T* S, T* ct, T* st, const T* ja, const T* jb, const T* vf,
@@ -463,7 +467,7 @@ void sigma_launch(sbdgpu_ctx* c, const T* C, T* S, T* ct, T* st, const T* ja, co
   const SpinTables& tb = c->tab[1];
   if (events) SBD_CUDA(cudaEventRecord(c->ev[0], s));
   if constexpr (sizeof(T) == 8) {
-    if (c->dense[0] && c->oz.mode == 0 && uses_tiles(c)) {
+    if (dense_path(c)) {
       alpha_coulomb(c, C, S);
       same_spin_dense_fp64(c, C, S);
       if (events) SBD_CUDA(cudaEventRecord(c->ev[1], s));  // both spins at once: the second phase is empty
@@ -538,6 +542,7 @@ void sigma_fp64(sbdgpu_ctx* c, const double* C, double* S) {
   }
   ensure_scratch(c);
   const bool tiles = uses_tiles(c);
+  if (wants_ozaki(c) || !dense_path(c)) ensure_ct(c);
   if (use_ozaki(c) && same_spin_ozaki_fp64(c, C, S, c->ct, c->st, true, !tiles)) {
     const SpinTables& ta = c->tab[0];
     alpha_beta<double>(c, C, S, c->vf, AlphaSingles{ta.s_off, ta.s_idx, ta.s_info, ta.max_s, 0}, tiles);
@@ -547,6 +552,8 @@ void sigma_fp64(sbdgpu_ctx* c, const double* C, double* S) {
   sigma_launch<double>(c, C, S, c->ct, c->st, c->ja, c->jb, c->vf, true);
 }
 
+bool sigma_fp64_needs_ct(const sbdgpu_ctx* c) { return !dense_path(c); }
+
 void sigma_fp64_prepared(sbdgpu_ctx* c, const double* C, double* S, double* ct, double* st) {
   sigma_launch<double>(c, C, S, ct, st, c->ja, c->jb, c->vf, false);
 }
@@ -555,6 +562,7 @@ void sigma_fp32(sbdgpu_ctx* c, const float* C, float* S) {
   build_tables(c);
   compute_hii(c);
   ensure_scratch(c);
+  ensure_ct(c);
   ensure_fp32(c);
   // the FP64 scratch vectors hold the FP32 transposes (half their size)
   float* ct = reinterpret_cast<float*>(c->ct);
@@ -624,7 +632,8 @@ void sigma_rows_fp64(sbdgpu_ctx* c, const double* dC, double* S, size_t r0, size
   build_tables(c);
   compute_hii(c);
   ensure_scratch(c);
-  ensure_io(c);
+  ensure_ct(c);
+  ensure_io_a(c);
   const size_t nrows = r1 - r0, nb = c->nb;
   cudaStream_t s = c->stream;
   const SpinTables& ta = c->tab[0];
@@ -647,6 +656,7 @@ void sigma_fp32_tc(sbdgpu_ctx* c, const float* C, float* S) {
   build_tables(c);
   compute_hii(c);
   ensure_scratch(c);
+  ensure_ct(c);
   ensure_fp32(c);
   build_tc_buckets(c);
   if (!tc_ab_supported(c)) throw Error{SBDGPU_ERR_LIMIT, "tensor-core alpha-beta kernel: basis or norb too large"};

@@ -116,3 +116,21 @@ def test_fp32_sigma_by_tiles(nb):
     # the bound of the mixed sigma's other tests against FP64
     assert np.abs(got - ref).max() <= 2e-5 * np.abs(ref).max()
     ctx.close()
+
+
+@pytest.mark.parametrize("na,nb", [(1025, 1039), (1100, 1102), (1041, 1024)])
+def test_integer_products_of_any_string_counts(na, nb):
+    # counts that are padded to multiples of 16, against the rows kernels
+    ints, a, b = _system(18, 5, 5, na, nb, 70 + na)
+    ctx = sbd_b200.context_from_integrals(ints, a, b)
+    C = np.random.default_rng(6).normal(size=ctx.n)
+    ctx.set_fp64_same_spin(1)
+    ref = ctx.sigma(C)
+    ctx.set_fp64_same_spin(0)
+    for x, r in ((C, ref), (np.where(np.arange(ctx.n) == 5, np.inf, C), None)):
+        got = ctx.sigma(x)
+        if r is not None:
+            assert np.abs(got - r).max() <= TOL * np.abs(r).max()
+        else:
+            assert not np.isfinite(got[5]) and np.isfinite(got).sum() > ctx.n // 2
+    ctx.close()
