@@ -441,8 +441,24 @@ __device__ __forceinline__ void tiles(const MmaArgs<T>& a, const unsigned char* 
     // the tiles' strings side by side: at.x .. at.x + len0 + len1
     const int len0 = at.y & 0xFF, len1 = at.y >> 8, len = len0 + len1;
     const bool bulk = a.bulk && (at.x * sizeof(T)) % 16 == 0 && (len * sizeof(T)) % 16 == 0;
+    if constexpr (SB == 0) {  // no room for stages: straight from the accumulators
 #pragma unroll
-    for (int b0 = 0; b0 < BLOCKS; b0 += SB) {
+      for (int b = 0; b < BLOCKS; b++) {
+        const int to = tgt[8 * b + r];
+        if (to < 0) continue;
+        const uint32_t sg = neg[8 * b + r];
+        const auto val = [&](double x) { return (T)__hiloint2double(__double2hiint(x) ^ (int)sg, __double2loint(x)); };
+        T* row = a.S + (size_t)to * a.nb + at.x;
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+          if (2 * q + u < len0) atomicAdd(row + 2 * q + u, val(acc0[2 * b + u]));
+          if (2 * q + u < len1) atomicAdd(row + len0 + 2 * q + u, val(acc1[2 * b + u]));
+        }
+      }
+      continue;
+    }
+#pragma unroll
+    for (int b0 = 0; b0 < BLOCKS; b0 += SB > 0 ? SB : BLOCKS) {
       constexpr int ROWS = 8 * (SB < BLOCKS ? SB : BLOCKS);
       if (a.bulk) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // the last lines are read
       __syncwarp();
@@ -471,7 +487,7 @@ __device__ __forceinline__ void tiles(const MmaArgs<T>& a, const unsigned char* 
       }
     }
   }
-  if (a.bulk) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+  if (SB > 0 && a.bulk) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
 
 // One CTA per (source alpha string ja, M of its singles): alpha single 8 b + r
@@ -644,12 +660,20 @@ void build_ab_tiles(sbdgpu_ctx* c, SpinTables& t, const std::vector<uint64_t>& s
   SBD_CUDA(cudaStreamSynchronize(st));
 }
 
+// Without stages the kernel may use all that the opt-in limit leaves beside its
+// own 128 bytes (budget is the limit less 1 KiB): eight singles beside 20,000
+// beta strings at norb 48, where 490 ms replace the 1,180 ms of the gather
+// kernel at four singles (400M determinants; FP32: 446 ms).  Where stages fit
+// they stay the better choice: 93 against 125 ms at 144M.
+constexpr size_t kUnstagedExtra = 1024 - 128;
+
 // Alpha singles per CTA of the tile kernel for a wanted number (0: the larger
 // that fits); 0 when this basis has no tiles or they do not fit.
 int ab_mma_group(const sbdgpu_ctx* c, int want, size_t budget) {
   if (!c->tab[1].tile_grp) return 0;
   for (int m : {16, 8})
     if ((want == 0 || want == m) && mma_smem(c, m, 128, sizeof(double), 1) <= budget) return m;
+  if (want == 0 && mma_smem(c, 8, 0, 0, 0) <= budget + kUnstagedExtra) return 8;
   return 0;
 }
 
@@ -679,8 +703,9 @@ void ab_mma(sbdgpu_ctx* c, const T* C, T* S, const AlphaSingles& as, int m, int 
         }
       }
     if (nt == 0) {
-      nt = 128;
-      sb = 1;
+      const bool staged = mma_smem(c, m, 128, sizeof(T), 1) <= budget;
+      nt = staged ? 128 : 1024;
+      sb = staged ? 1 : 0;
     }
     while (nt > 128 && (size_t)(nt / 2) >= c->tab[1].n_tile_grp * 32) nt /= 2;
   } else {  // a tuned number: as many stages as fit beside the row of C
@@ -691,8 +716,10 @@ void ab_mma(sbdgpu_ctx* c, const T* C, T* S, const AlphaSingles& as, int m, int 
     launch_mma<T, 16, 2>(c, C, S, as, nt, beta_j);
   else if (m == 16)
     launch_mma<T, 16, 1>(c, C, S, as, nt, beta_j);
-  else
+  else if (sb == 1)
     launch_mma<T, 8, 1>(c, C, S, as, nt, beta_j);
+  else
+    launch_mma<T, 8, 0>(c, C, S, as, nt, beta_j);
 }
 
 template void ab_mma<double>(sbdgpu_ctx*, const double*, double*, const AlphaSingles&, int, int, size_t, bool);
@@ -702,6 +729,7 @@ void preload_ab_mma(int device) {
   allow_dynamic_smem(reinterpret_cast<const void*>(ab_mma_kernel<double, 16, 2>), device);
   allow_dynamic_smem(reinterpret_cast<const void*>(ab_mma_kernel<double, 16, 1>), device);
   allow_dynamic_smem(reinterpret_cast<const void*>(ab_mma_kernel<double, 8, 1>), device);
+  allow_dynamic_smem(reinterpret_cast<const void*>(ab_mma_kernel<double, 8, 0>), device);
 }
 
 }  // namespace sbdgpu

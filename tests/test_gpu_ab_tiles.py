@@ -134,3 +134,19 @@ def test_integer_products_of_any_string_counts(na, nb):
         else:
             assert not np.isfinite(got[5]) and np.isfinite(got).sum() > ctx.n // 2
     ctx.close()
+
+
+def test_tiles_without_stages():
+    # 48 orbitals and 19,990 beta strings leave no shared memory for staged results beside eight singles' integrals
+    # and the row of C; one string more than 20,015 keeps the gather kernel
+    ints = synth.make_integrals(48, 3)
+    b = synth.selected_strings(48, 4, 20100, np.diag(ints.h), 4)
+    a = b[[0, 1, 2, 5, 9]]
+    for nb in (19990, 20016):
+        ctx = sbd_b200.context_from_integrals(ints, a, b[:nb])
+        C = np.random.default_rng(nb).normal(size=ctx.n)
+        got = ctx.sigma(C)
+        ctx.set_tuning(4, 512)  # the gather kernel
+        ref = ctx.sigma(C)
+        assert np.abs(got - ref).max() <= TOL * np.abs(ref).max()
+        ctx.close()
