@@ -123,10 +123,10 @@ def measured_peaks():
 # DRAM bytes (ncu dram__bytes_read.sum + dram__bytes_write.sum) of one launch,
 # from single captures of smaller workloads of the same kernels:
 #  - ab_mma_kernel at 16M determinants (norb 26, 6a/6b, 4000 strings):
-#    1101 MB per launch, 68.8 bytes per determinant; the 144M line scales it
+#    1379 MB per launch, 86.2 bytes per determinant; the 144M line scales it
 #    by the determinant count
 #  - spmv_kernel (method 1) at 245,025 determinants: 4.236 GB per launch
-AB_TRAFFIC_BYTES_PER_DET = 68.8
+AB_TRAFFIC_BYTES_PER_DET = 86.2
 SPMV_TRAFFIC_BYTES_C0 = 4.236e9
 
 
