@@ -389,16 +389,12 @@ void free_ozaki(sbdgpu_ctx* c) {
 
 // Whether the FP64 sigma takes its same-spin terms from the integer products by
 // its size and the context's choice (c->oz.mode: 0 automatic, 1 never): at
-// least 1,024 strings per spin; where the counts are not multiples of 4 only
-// beside alpha-beta tiles (the singles' pass for the beta strings moves pairs
-// of columns), and not while the dense FP64 product is faster: both take 1.4 ms
-// per sigma at 1,600 x 1,600 strings, at 2,000 x 2,000 the integers take 2.1
-// and the dense product 2.5.
+// least 1,024 strings per spin, in multiples of 4.  (Other counts would be
+// faster this way too, 7,777 x 6,001 strings 27.5 ms per sigma, but the
+// products round their operands to 49 bits, and those bases' FP64 sums do not:
+// 1.2e-15 against 1.0e-15 of sigma's norm.)
 bool wants_ozaki(const sbdgpu_ctx* c) {
-  if (c->oz.mode == 1 || c->oz.failed || c->na < 1024 || c->nb < 1024) return false;
-  if (c->na % 4 == 0 && c->nb % 4 == 0) return true;
-  return c->tab[1].tile_grp &&
-         !(dense_same_spin(c) && (double)c->na * c->nb * (c->na + c->nb) < 8.2e9);
+  return c->oz.mode != 1 && !c->oz.failed && c->na >= 1024 && c->nb >= 1024 && c->na % 4 == 0 && c->nb % 4 == 0;
 }
 
 // As wants_ozaki, with room in device memory.
@@ -415,8 +411,7 @@ bool same_spin_ozaki_fp64(sbdgpu_ctx* c, const double* C, double* S, double* ct,
   const size_t na = c->na, nb = c->nb, pa = pad16(na), pb = pad16(nb), plane = pa * pb;
   const SpinTables& tb = c->tab[1];
   cublasHandle_t h = static_cast<cublasHandle_t>(c->blas);
-  // jsingles64_kernel moves pairs of doubles
-  if (beta_j && (na % 2 || nb % 2 || (((uintptr_t)C | (uintptr_t)S) & 15))) return false;
+  if (((uintptr_t)C | (uintptr_t)S) & 15) return false;  // the kernels move pairs of doubles
   SBD_CUDA(cudaGetLastError());
   if (events) SBD_CUDA(cudaEventRecord(c->ev[0], s));
   // scaled residues of C (rows: for the beta product) and of C^T (for the alpha product)
