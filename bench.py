@@ -731,7 +731,8 @@ def run_gpu(args):
         return 0
     hbm_peak, peak_kind = measured_peaks()
     ab_ms = parts[2] / args.steps
-    same_spin = ("rows" if args.fp64_same_spin == 1 else "int8" if min(ctx.na, ctx.nb) >= 1024 else "dense")
+    same_spin = ("rows" if args.fp64_same_spin == 1
+                 else "int8" if min(ctx.na, ctx.nb) >= 1024 and ctx.na % 4 == 0 and ctx.nb % 4 == 0 else "dense")
     kernel_names = [f"alpha same-spin and diagonal ({same_spin})", f"beta same-spin ({same_spin})",
                     "ab_mma_kernel (alpha-beta)"]
     dom = int(np.argmax(parts))
@@ -767,346 +768,6 @@ def run_gpu(args):
         "e2e": {"value": world * 1000.0 / t_e2e, "unit": UNIT, "h2d_bytes_per_step": 8 * n,
                 "d2h_bytes_per_step": 8 * n},
         "gpu_launches": LAUNCHES_PER_SIGMA[same_spin] * args.steps * 2,
-        "roofline": {"bound": "hbm", "kernel": "spmv_kernel (stored Hamiltonian)", "achieved": achieved,
-                         "peak": hbm_peak, "unit": "GB/s", "frac": achieved / hbm_peak, "peak_source": peak_kind,
-                         "algorithmic_bytes": bytes_per, "traffic": SPMV_TRAFFIC_BYTES_C0},
-            "note": "12 bytes per stored element (uint32 ket, FP64 value) + row offsets + hii, C, sigma"}
-
-
-def genop_block(args, dev):
-    """The generic second-quantised path (sbdgpu_genop_*): the FCIDUMP
-    Hamiltonian of the 245,025-determinant system (norb 12, 4a/4b, full
-    space) as a GeneralOp on 24 sites, its on-the-fly mult per second, and its
-    Davidson energy against the tensor-product-basis path's."""
-    import os
-    import tempfile
-    import torch
-    import sbd_b200
-    from sbd_b200 import synth
-    ints, ne, strs = synth.make_workload("c0_L12_4e_full", seed=0)
-    L = ints.norb
-    states = np.array([int(a) | (int(b) << L) for a in strs for b in strs], dtype=np.uint64)
-    g = sbd_b200.GenOp(states, sign=True, device=dev)
-    with tempfile.TemporaryDirectory() as td:
-        p = os.path.join(td, "FCIDUMP")
-        synth.write_fcidump(p, ints, 2 * ne)
-        g.set_fcidump(p)
-    n = len(states)
-    C = torch.randn(n, dtype=torch.float64, device=f"cuda:{dev}")
-    Wd = torch.zeros_like(C)
-    for _ in range(3):
-        g.mult_device(C.data_ptr(), Wd.data_ptr())
-    # the object runs on its own stream: time over a device-wide synchronize
-    torch.cuda.synchronize()
-    reps = 20
-    t = time.perf_counter()
-    for _ in range(reps):
-        g.mult_device(C.data_ptr(), Wd.data_ptr())
-    torch.cuda.synchronize()
-    ms = (time.perf_counter() - t) * 1000.0 / reps
-    ctx = sbd_b200.context_from_integrals(ints, strs, strs, device=dev)
-    W0 = np.zeros(n)
-    W0[0] = 1.0
-    e_tpb, _, te_tpb, _ = ctx.davidson(W0, 200, 10, 1e-8)
-    t = time.perf_counter()
-    e_gen, _, te, tt = g.davidson(W0, 200, 10, 1e-8)
-    t_gen = time.perf_counter() - t
-    ctx.close()
-    g.close()
-    return {"workload": "c0_L12_4e_full as GeneralOp (24 sites)", "states": n, "mult_ms": ms, "mult_per_s": 1000.0 / ms, "davidson_steps": len(te),
-            "davidson_s": t_gen, "e_generic": e_gen, "e_tpb": e_tpb, "abs_diff": abs(e_gen - e_tpb),
-            "note": "mult timed over 20 launches between device synchronizations; no reference arm: the reference's generic mult cannot find most basis "
-                    "states (Basis::IndexSearch bisects over the first nwords states only)"}
-
-
-def config4_block(args, dev, learned):
-    """The 400M-determinant workload (norb 48, 10a/10b, 20,000 x 20,000
-    selected strings): FP64, FP32 and tensor-core sigma builds per second, and
-    time-to-E0 within 1e-6 Eh for plain FP64, mixed precision with the
-    diagonal correction and with the learned one (the network trained on the
-    16M-determinant system).  FP64 vectors are 3.2 GB each."""
-    import torch
-    import sbd_b200
-    from sbd_b200 import synth
-    ints, ne, strs = synth.make_workload("c4_L48_10e_20000", seed=0)
-    ctx = sbd_b200.context_from_integrals(ints, strs, strs, device=dev)
-    n = ctx.n
-    C = torch.randn(n, dtype=torch.float64, device=f"cuda:{dev}",
-                    generator=torch.Generator(device=f"cuda:{dev}").manual_seed(3))
-    C /= torch.linalg.norm(C)
-    S = torch.empty_like(C)
-    out = {"workload": "c4_L48_10e_20000", "determinants": n}
-    for name, prec in (("fp64", sbd_b200.FP64), ("mixed_fp32", sbd_b200.MIXED), ("mixed_tc", sbd_b200.MIXED_TC)):
-        ms = []
-        for i in range(2 + 3):
-            ctx.sigma_device(C.data_ptr(), S.data_ptr(), precision=prec)
-            if i >= 2:
-                ms.append(ctx.last_sigma_ms())
-        out[name] = {"sigma_per_s": 1000.0 * len(ms) / sum(m[3] for m in ms),
-                     "phases_ms": [sum(m[k] for m in ms) / len(ms) for k in range(3)]}
-    del C, S
-    torch.cuda.empty_cache()
-    W0 = np.zeros(n)
-    W0[0] = 1.0
-    t = time.perf_counter()
-    e_ref, _, te, tt = ctx.davidson(W0, 100, 10, args.e0_tol, precision=sbd_b200.FP64)
-    t_all = time.perf_counter() - t
-    hit = np.nonzero(te - e_ref < 1e-6)[0]
-    k = int(hit[0]) + 1 if len(hit) else len(te)
-    t_plain = t_all * k / len(te)
-    out["plain"] = {"steps_total": len(te), "steps_to_1e-6": k, "s_to_1e-6": t_plain, "e": e_ref,
-                    "final_residual": float(tt[-1])}
-    t = time.perf_counter()
-    e_m, _, tm, ttm = ctx.davidson(W0, 100, 10, args.mixed_tol, precision=sbd_b200.MIXED, restart_keep=3,
-                                   restart_prev=1)
-    t_m = time.perf_counter() - t
-    out["mixed"] = {"steps": len(tm), "s": t_m, "abs_err": abs(e_m - e_ref), "within_1e-6": abs(e_m - e_ref) < 1e-6,
-                    "speedup": t_plain / t_m}
-    if learned is not None:
-        ctx.precond_set(learned[0])
-        t = time.perf_counter()
-        e_l, _, tl, ttl = ctx.davidson(W0, 100, 10, args.mixed_tol, precision=sbd_b200.MIXED, restart_keep=3,
-                                       restart_prev=1, precond=sbd_b200.PRECOND_LEARNED)
-        t_l = time.perf_counter() - t
-        out["learned"] = {"steps": len(tl), "s": t_l, "abs_err": abs(e_l - e_ref),
-                          "within_1e-6": abs(e_l - e_ref) < 1e-6, "speedup": t_plain / t_l,
-                          "speedup_vs_mixed_diagonal": t_m / t_l, "network": learned[1]}
-    ctx.close()
-    return out
-
-
-def rdm_block(args, dev):
-    """1/2-RDMs (sbdgpu_rdm) of a seeded normalised vector on args.rdm_workload,
-    wall-clock including the host copies of the 4 L^4 two-body array."""
-    import sbd_b200
-    from sbd_b200 import synth
-    ints, ne, strs = synth.make_workload(args.rdm_workload, seed=0)
-    ctx = sbd_b200.context_from_integrals(ints, strs, strs, device=dev)
-    W = np.random.default_rng(5).normal(size=ctx.n)
-    W /= np.linalg.norm(W)
-    ctx.hii()  # tables and diagonal outside the timing
-    t = time.perf_counter()
-    one, two = ctx.rdm(W)
-    sec = time.perf_counter() - t
-    ctx.close()
-    return {"workload": args.rdm_workload, "determinants": int(len(strs)) ** 2, "seconds": sec,
-            "trace_alpha": float(np.trace(one[:ints.norb ** 2].reshape(ints.norb, ints.norb)))}
-
-
-def roots_block(args, dev):
-    """Block Davidson for the lowest args.roots roots (FP64) on the
-    16M-determinant system (norb 26, 6a/6b, 4000 x 4000 strings): wall time,
-    cycles, sigma builds, residual norms, and root 0 against the single-root
-    FP64 Davidson of the same system."""
-    import sbd_b200
-    from sbd_b200 import synth
-    ints, ne, strs = synth.make_workload(args.roots_workload, seed=0)
-    ctx = sbd_b200.context_from_integrals(ints, strs, strs, device=dev)
-    k = args.roots
-    nb = min(32, max(2 * k, 3 * k))
-    W0 = np.zeros(ctx.n)
-    W0[0] = 1.0
-    t = time.perf_counter()
-    e1, w1, te, _ = ctx.davidson(W0, 200, 10, args.roots_tol)
-    t_one = time.perf_counter() - t
-    # the block run starts from the single-root ground state and the
-    # lowest-H_ii determinants: from determinants alone its first collapse can
-    # drop the ground state's symmetry sector (see DESIGN)
-    Wb = np.zeros((k, ctx.n))
-    Wb[0] = w1
-    t = time.perf_counter()
-    E, W, r, it, ns = ctx.davidson_roots(k, 400, nb, args.roots_tol, W0=Wb)
-    t_block = time.perf_counter() - t
-    ctx.close()
-    return {"workload": args.roots_workload, "roots": k, "max_nb": nb, "eps": args.roots_tol, "seconds": t_block,
-            "cycles": it, "sigma_builds": ns, "energies": [float(x) for x in E],
-            "residuals": [float(x) for x in r],
-            "note": "each Ritz value lies within its residual norm of an eigenvalue (symmetric H); block run started "
-                    "from the single-root ground state and the lowest-H_ii determinants",
-            "root0_minus_single_root": float(E[0] - e1),
-            "single_root_seconds": t_one, "single_root_steps": len(te)}
-
-
-def batch_block(args, dev):
-    """args.batch independent problems drawn as the batching workload
-    describes (norb uniform in 10-20, electrons per spin in 3-6, 200-2000
-    selected strings per spin capped at C(norb, ne), seeded integrals per
-    problem): lowest-root FP64 Davidson one problem after another against one
-    sbdgpu_davidson_batch call on the same contexts (set-up done before
-    either), as problems/s, with the largest energy difference."""
-    import math
-    import sbd_b200
-    from sbd_b200 import synth
-    rng = np.random.default_rng(2024)
-    ctxs, sizes = [], []
-    for i in range(args.batch):
-        L = int(rng.integers(10, 21))
-        ne = int(rng.integers(3, 7))
-        cnt = min(int(rng.integers(200, 2001)), math.comb(L, ne))
-        ints, ne, strs = synth.make_small(L, ne, cnt, 1000 + i)
-        c = sbd_b200.context_from_integrals(ints, strs, strs, device=dev)
-        c.hii()  # tables and diagonal, outside both timings
-        ctxs.append(c)
-        sizes.append(c.n)
-    # the same seeded start for both arms: the aufbau determinant plus a 1 %
-    # random part, so that every run reaches the lowest state whatever its
-    # spin-flip symmetry (from the closed-shell determinant alone, rounding
-    # decides whether a run leaves the spin-flip-even sector)
-    W0s = []
-    for i, c in enumerate(ctxs):
-        w = np.random.default_rng(5000 + i).normal(size=c.n)
-        w *= 0.01 / np.linalg.norm(w)
-        w[0] += 1.0
-        W0s.append(w / np.linalg.norm(w))
-    # the committed launch shapes of the alpha-beta kernel, in both arms
-    from sbd_b200 import autotune
-    table = autotune.load()
-    tuned = sum(1 for c in ctxs if autotune.apply(c, table))
-    max_it = 300
-    t = time.perf_counter()
-    e_seq, s_seq = [], []
-    for c, w in zip(ctxs, W0s):
-        e1, _, te, _ = c.davidson(w, max_it, 10, args.batch_tol)
-        e_seq.append(e1)
-        s_seq.append(len(te))
-    t_seq = time.perf_counter() - t
-    t = time.perf_counter()
-    e_bat, _, steps = sbd_b200.davidson_batch(ctxs, W0s, max_it, 10, args.batch_tol)
-    t_bat = time.perf_counter() - t
-    for c in ctxs:
-        c.close()
-    diff = np.abs(np.array(e_bat) - np.array(e_seq))
-    return {"problems": args.batch, "determinants_min": int(min(sizes)), "determinants_max": int(max(sizes)),
-            "determinants_total": int(sum(sizes)), "eps": args.batch_tol,
-            "sequential_problems_per_s": args.batch / t_seq, "batch_problems_per_s": args.batch / t_bat,
-            "speedup": t_seq / t_bat, "max_abs_energy_diff": float(diff.max()),
-            "problems_differing_by_more_than_1e-6": int((diff > 1e-6).sum()),
-            "steps_total": int(sum(steps)), "steps_max": int(max(steps)),
-            "sequential_steps_total": int(sum(s_seq)),
-            "problems_at_step_cap": int(sum(1 for x in steps if x >= max_it * 10)),
-            "tuned_contexts": tuned, "tuning_classes": len(table),
-            "note": "batch: device-resident Davidson, one replayed CUDA graph per problem step, one host wait per "
-                    "round; sequential: sbdgpu_davidson per problem (one host round trip per dot product)"}
-
-
-def run_gpu(args):
-    import torch
-    import sbd_b200
-    from sbd_b200 import synth
-
-    rank, world, local = dist_env()
-    dev = local if world > 1 else 0
-    torch.cuda.set_device(dev)
-    pg = None
-    if world > 1:
-        import datetime
-        import torch.distributed as dist
-        dist.init_process_group("nccl", timeout=datetime.timedelta(seconds=600))
-        pg = dist
-    ints, ne, strs = synth.make_workload(args.workload, seed=0)
-    ctx = sbd_b200.context_from_integrals(ints, strs, strs, device=dev)
-    ctx.set_fp64_same_spin(args.fp64_same_spin)
-    st = table_stats(ctx)
-    alg = algorithmic(ctx, st)
-    n = ctx.n
-    C = torch.randn(n, dtype=torch.float64, device=f"cuda:{dev}", generator=torch.Generator(device=f"cuda:{dev}").manual_seed(1))
-    C /= torch.linalg.norm(C)
-    S = torch.empty_like(C)
-    torch.cuda.synchronize()
-    for _ in range(args.warmup):
-        ctx.sigma_device(C.data_ptr(), S.data_ptr())
-    if pg:
-        pg.barrier()
-    torch.cuda.synchronize()
-    sampler = ClockSampler(dev)
-    sampler.start()
-    tot, ab, parts = 0.0, 0.0, [0.0, 0.0, 0.0]
-    for _ in range(args.steps):
-        ctx.sigma_device(C.data_ptr(), S.data_ptr())
-        ms = ctx.last_sigma_ms()
-        tot += ms[3]
-        for k in range(3):
-            parts[k] += ms[k]
-    torch.cuda.synchronize()
-    # the mixed-precision sigma (FP32 vectors) on the same resident vector
-    mixed_ms = []
-    for i in range(args.warmup + args.steps):
-        ctx.sigma_device(C.data_ptr(), S.data_ptr(), precision=sbd_b200.MIXED)
-        if i >= args.warmup:
-            mixed_ms.append(ctx.last_sigma_ms())
-    tc_ms = []
-    for i in range(args.warmup + args.steps):
-        ctx.sigma_device(C.data_ptr(), S.data_ptr(), precision=sbd_b200.MIXED_TC)
-        if i >= args.warmup:
-            tc_ms.append(ctx.last_sigma_ms())
-    torch.cuda.synchronize()
-    if pg:
-        pg.barrier()
-    # end to end: pinned host buffers through the C ABI
-    Ch = torch.empty(n, dtype=torch.float64, pin_memory=True)
-    Ch.copy_(C.cpu())
-    Sh = torch.empty(n, dtype=torch.float64, pin_memory=True)
-    e2e_ms = 0.0
-    Cnp = Ch.numpy()
-    Snp = Sh.numpy()
-    import ctypes
-    for _ in range(args.steps):
-        rc = sbd_b200.lib().sbdgpu_sigma(ctx._h, Cnp.ctypes.data_as(ctypes.POINTER(ctypes.c_double)),
-                                         Snp.ctypes.data_as(ctypes.POINTER(ctypes.c_double)), 0)
-        ctx._check(rc)
-        e2e_ms += ctx.last_sigma_ms()[4]
-    torch.cuda.synchronize()
-    sampler.stop()
-    if pg:
-        pg.barrier()
-    t_step = tot / args.steps
-    t_e2e = e2e_ms / args.steps
-    if pg:
-        t_step, t_e2e = max_over_ranks([t_step, t_e2e], pg, f"cuda:{dev}")
-    if rank != 0:
-        ctx.close()
-        if pg:
-            pg.destroy_process_group()
-        return 0
-    hbm_peak, peak_kind = measured_peaks()
-    ab_ms = parts[2] / args.steps
-    same_spin = ("rows" if args.fp64_same_spin == 1 else "int8" if min(ctx.na, ctx.nb) >= 1024 else "dense")
-    kernel_names = [f"alpha same-spin and diagonal ({same_spin})", f"beta same-spin ({same_spin})",
-                    "ab_mma_kernel (alpha-beta)"]
-    dom = int(np.argmax(parts))
-    dom_ms = parts[dom] / args.steps
-    dom_bytes = [8.0 * n * 3 + st[0][0] * 16 + st[0][1] * 12, 8.0 * n * 6 + st[1][0] * 16 + st[1][1] * 12,
-                 alg["ab_bytes"]][dom]
-    achieved = dom_bytes / (dom_ms * 1e-3) / 1e9
-    traffic = args.traffic
-    if traffic is None and dom == 2:
-        traffic = AB_TRAFFIC_BYTES_PER_DET * n
-    smem_floor = None
-    if dom == 2:
-        props = torch.cuda.get_device_properties(dev)
-        group = ab_default_group(ctx.nb, ctx.norb * (ctx.norb + 1) // 2,
-                                 getattr(props, "shared_memory_per_block_optin", 232448))
-        clk = sampler.summary().get("sm_mhz") or 1965.0
-        if group:
-            smem_floor = ab_smem_floor(st, group, props.multi_processor_count, clk)
-            smem_floor["measured_ms"] = ab_ms
-            smem_floor["frac"] = smem_floor["floor_ms"] / ab_ms
-            smem_floor["note"] = "floor of the one-integral-per-product gather that the tiles replace"
-    ab_flops = 2.0 * st[0][0] * st[1][0]
-    fp64_floor = {"flops": ab_flops, "tflops_peak": FP64_TENSOR_TFLOPS,
-                  "floor_ms": ab_flops / FP64_TENSOR_TFLOPS / 1e9, "measured_ms": ab_ms,
-                  "frac": ab_flops / FP64_TENSOR_TFLOPS / 1e9 / ab_ms}
-    line = {
-        "metric": METRIC, "value": world * 1000.0 / t_step, "unit": UNIT, "n_gpus": world, "steps": args.steps,
-        "warmup": args.warmup, "ms_per_step": t_step, "higher_is_better": True, "scaling": "weak",
-        "vs_baseline": None, "dtype": "f64", "data": "synthetic (seeded integrals and strings)",
-        "config": {"workload": args.workload, "determinants": n, "norb": ints.norb, "electrons": f"{ne}a/{ne}b",
-                   "strings_per_spin": ctx.na, "parallelism": f"replicas x{world}" if world > 1 else "single GPU",
-                   "l2": "inputs (1.15 GB per vector) larger than L2; no flush"},
-        "e2e": {"value": world * 1000.0 / t_e2e, "unit": UNIT, "h2d_bytes_per_step": 8 * n,
-                "d2h_bytes_per_step": 8 * n},
-        "gpu_launches": (LAUNCHES_PER_SIGMA_INT8 if args.fp64_same_spin == 0 and min(ctx.na, ctx.nb) >= 1024
-                         and ctx.na % 4 == 0 and ctx.nb % 4 == 0 else LAUNCHES_PER_SIGMA) * args.steps * 2,
         "roofline": {"bound": "hbm", "kernel": kernel_names[dom], "achieved": achieved, "peak": hbm_peak,
                      "unit": "GB/s", "frac": achieved / hbm_peak, "peak_source": peak_kind,
                      "traffic": traffic,
