@@ -647,7 +647,7 @@ def batch_block(args, dev):
             "problems_at_step_cap": int(sum(1 for x in steps if x >= max_it * 10)),
             "tuned_contexts": tuned, "tuning_classes": len(table),
             "note": "batch: device-resident Davidson, one replayed CUDA graph per problem step, one host wait per "
-                    "round; sequential: sbdgpu_davidson per problem (one host round trip per dot product)"}
+                    "round; sequential: sbdgpu_davidson per problem (two host round trips per step)"}
 
 
 def run_gpu(args):

@@ -233,9 +233,9 @@ int sbdgpu_occupation(sbdgpu_ctx* ctx, const double* W, double* density);
 int sbdgpu_alpha_weights(sbdgpu_ctx* ctx, const double* W, double* D);
 
 /* CUDA-event times in milliseconds of the last sigma build, on the context's
- * stream: ms5[0] diagonal + alpha same-spin kernel, [1] beta same-spin
- * (transposes included), [2] alpha-beta kernel, [3] the whole build on device
- * vectors (sign phases included), [4] for sbdgpu_sigma only: end to end from
+ * stream: ms5[0] diagonal + alpha same-spin kernel (both spins' where they are
+ * one dense product), [1] beta same-spin (transposes included), [2] alpha-beta
+ * kernel, [3] the whole build on device vectors (sign phases included), [4] for sbdgpu_sigma only: end to end from
  * the start of the host-to-device copy to the end of the device-to-host copy
  * (0 after a device-vector call).  No counterpart in the reference, which
  * prints wall-clock timers (chemistry/tpb/mult.h:435-446, 619-646). */
@@ -285,9 +285,10 @@ int sbdgpu_mlp_loss_grad(int device, const float* w, int B, const float* X, cons
 /* Launch shape of the FP64 alpha-beta kernel (an extension): ab_group alpha
  * singles per CTA (16, 8, 4, 2 or 1, where the integral block fits in shared
  * memory beside a row of C) and ab_threads threads per CTA (128, 256, 512 or
- * 1024); (0, 0) restores the default (the largest group that fits; 512
- * threads while two CTAs fit an SM, else 1024, halved down to 128 while the
- * warps outnumber the 32-string slices of beta strings).  A shape that does not fit the
+ * 1024).  Groups of 16 and 8 run as products on the FP64 tensor pipe where the
+ * basis allows it, smaller ones as a gather.  (0, 0) restores the default (the
+ * largest group that fits, the threads that put most warps on an SM, fewer
+ * while the warps outnumber the work of a CTA).  A shape that does not fit the
  * basis is refused. */
 int sbdgpu_set_tuning(sbdgpu_ctx* ctx, int ab_group, int ab_threads);
 
@@ -300,9 +301,11 @@ int sbdgpu_autotune(sbdgpu_ctx* ctx, int reps, int* ab_group, int* ab_threads, f
  * default) = as exact INT8 tensor-core products of the dense string-only
  * operator (residues modulo 15 primes, CRT reconstruction; FP64-accurate: the
  * scaled operands are rounded to 49-bit integers) where both spins have at
- * least 1,024 strings (multiples of 4) and the residues fit in device memory,
- * else the rows kernels; method 1 = the rows kernels always (and the device
- * memory of the integer products is released). */
+ * least 1,024 strings (multiples of 4) and the residues fit in device memory;
+ * as one dense FP64 product of both spins for other bases of at most 4,096
+ * strings whose operators are dense enough; else the rows kernels; method 1 =
+ * the rows kernels always (and the device memory of the integer products is
+ * released). */
 int sbdgpu_set_fp64_same_spin(sbdgpu_ctx* ctx, int method);
 
 const char* sbdgpu_last_error(sbdgpu_ctx* ctx);

@@ -22,8 +22,9 @@
 // their pair's class modulo 4, so that four pairs of different classes lie in
 // different banks; the pairs of a section are dealt to its steps by class and
 // by the banks of their kets.  One 32-bit entry per slot, in the order of the B
-// fragment (lane = 4 n + k); an empty slot points at a zero behind the row of
-// C.
+// fragment (lane = 4 n + k).  Behind the row of C stand 16 zeros, one per bank
+// pair; the empty slots of a half-warp point at one that none of its kets
+// collides with.
 #include <algorithm>
 #include <type_traits>
 #include <vector>
@@ -35,6 +36,7 @@ namespace sbdgpu {
 namespace {
 
 constexpr int kMmaThreads = 1024;
+constexpr int kZeros = 16;     // zeros behind the row of C, one in each pair of banks
 constexpr int kMaxWords = 63;  // bitmap words of the off-diagonal pairs: 64 * 63 / 2 = 2016
 
 __device__ __forceinline__ int od_pair(uint32_t info) {  // off-diagonal pair index of a single
@@ -196,7 +198,7 @@ __global__ void __launch_bounds__(32) tile_fill_kernel(int n, int words, const i
   // Deal the pairs of a section to its steps: the first one left, then three
   // times the one whose integral row differs in class from the step's others
   // and whose kets share fewest banks with theirs (per tile and half-warp of
-  // four strings; the zero of the empty slots counts once).
+  // four strings).
   for (int s = 0; s < 3; s++) {
     const int b0 = base[s], cnt = base[s + 1] - b0;
     uint64_t load[4] = {0, 0, 0, 0};  // 4-bit counts of 16 bank pairs by (tile, half)
@@ -224,14 +226,9 @@ __global__ void __launch_bounds__(32) tile_fill_kernel(int n, int words, const i
       const PairPlan p = plan[b0 + pick];
       classes |= 1u << (p.pair & 3);
       for (int h = 0; h < 4; h++) {
-        bool empty = false;
-        for (int x = 0; x < 4; x++) {
+        for (int x = 0; x < 4; x++)
           if ((p.set >> (4 * h + x)) & 1)
             load[h] += 1ull << (4 * ((p.bank[h >> 1] >> (4 * (4 * (h & 1) + x))) & 15));
-          else
-            empty = true;
-        }
-        if (empty && ((load[h] >> (4 * (n & 15))) & 15) == 0) load[h] += 1ull << (4 * (n & 15));
       }
       __syncwarp();
       if (lane == 0) plan[b0 + pick].place = (int16_t)at;
@@ -267,6 +264,27 @@ __global__ void __launch_bounds__(32) tile_fill_kernel(int n, int words, const i
     out[slot(s, at, nn, t)] =
         s == 0 && t == 1 ? second_word((uint32_t)ket, neg) : first_word((uint32_t)ket, o, neg);
   });
+  __syncwarp();
+  // The empty slots of a half-warp read the zero whose bank none of its kets has
+  // (one zero for all: 16M determinants 4.38 -> 4.31 ms, 144M 87.1 -> 85.1, FP32
+  // vectors 74.4 -> 72.6).
+  for (int u = lane; u < 2 * (2 * d.y + d.z + d.w); u += 32) {
+    const bool both = u < 4 * d.y;
+    uint32_t* w = both ? out + (u >> 2) * 64 + (u & 1) * 32 + ((u >> 1) & 1) : out + (size_t)u * 16;
+    const int stride = both ? 2 : 1;
+    uint32_t used = 0, empty = 0;
+    for (int i = 0; i < 16; i++) {
+      const uint32_t ket = (w[i * stride] >> 3) & 0xFFFFu;
+      if (ket == (uint32_t)n)
+        empty |= 1u << i;
+      else
+        used |= 1u << (ket & 15);
+    }
+    if (!empty) continue;
+    const uint32_t shift = (uint32_t)(__ffs(~used) - 1 - n) & 15u;
+    for (int i = 0; i < 16; i++)
+      if ((empty >> i) & 1) w[i * stride] += shift << 3;
+  }
 }
 
 // D (16 x 8) += A (16 x 4) B (4 x 8), FP64
@@ -285,11 +303,12 @@ __device__ __forceinline__ void mma8(double (&d)[4], double a0, double b) {
 // FP32 vectors: the row of C is converted as it is staged, products and sums
 // stay FP64, a row's sum is rounded once before it is added.
 //
-// What bounds it: the shared-memory pipe (16M determinants: 86 % of its
-// wavefronts, the FP64 tensor pipe 68 % busy).  Alpha-beta term, gather kernel
-// -> tiles: 144M determinants 198 -> 89 ms, 16M 11.2 -> 4.0 ms, 1501 x 803
-// strings 0.85 -> 0.34 ms, 495 x 495 0.10 -> 0.052 ms; the tensor pipe's floor
-// of the filled tiles is 54 / 2.8 ms at the first two.  24 and 32 alpha
+// What bounds it: the shared-memory pipe (16M determinants: 87 % of its
+// wavefronts, the FP64 tensor pipe 62 % busy).  Alpha-beta term with the beta
+// singles' Coulomb part, gather kernel (without it) -> tiles: 144M determinants
+// 198 -> 84 ms, 16M 11.2 -> 4.3 ms, 1501 x 803 strings 0.85 -> 0.34 ms,
+// 495 x 495 0.10 -> 0.07 ms; the products alone take 48 / 2.1 ms of the tensor
+// pipe at the first two.  24 and 32 alpha
 // singles per CTA (fewer loads of C per product) and entries fetched a batch
 // ahead were no faster: fewer warps fit, and the loads were not what waited.
 //
@@ -507,7 +526,7 @@ __global__ void __launch_bounds__(kMmaThreads) ab_mma_kernel(const MmaArgs<T> a)
   __shared__ uint32_t neg[M];
   unsigned char* vsub = smem;                                                          // [npair][M] integrals
   T* stage = reinterpret_cast<T*>(smem + (size_t)a.npair * M * 8);                     // [warps][8 SB][16] results
-  double* crow = reinterpret_cast<double*>(stage + (size_t)(blockDim.x >> 5) * SB * 128);  // [nb + 1]
+  double* crow = reinterpret_cast<double*>(stage + (size_t)(blockDim.x >> 5) * SB * 128);  // [nb + kZeros]
   const size_t ja = blockIdx.x;
   const int64_t k0 = a.a_off[ja] + (int64_t)blockIdx.y * M;
   const int singles = (int)min((int64_t)M, a.a_off[ja + 1] - k0);  // negative past the last ones
@@ -520,7 +539,7 @@ __global__ void __launch_bounds__(kMmaThreads) ab_mma_kernel(const MmaArgs<T> a)
     const uint32_t info = g < singles ? a.a_info[k0 + g] : 0u;
     neg[g] = info & 0x80000000u;
   }
-  for (size_t i = threadIdx.x; i <= a.nb; i += blockDim.x) crow[i] = i < a.nb ? (double)a.C[ja * a.nb + i] : 0.0;
+  for (size_t i = threadIdx.x; i < a.nb + kZeros; i += blockDim.x) crow[i] = i < a.nb ? (double)a.C[ja * a.nb + i] : 0.0;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
   // one 32-byte chunk of eight pairs' rows per warp and step
   for (int c = 0; c < M / 4; c++) {
@@ -549,7 +568,7 @@ namespace {
 
 // dynamic shared memory: integrals, per-warp stages, the row of C
 size_t mma_smem(const sbdgpu_ctx* c, int m, int threads, size_t elem, int sb) {
-  return sizeof(double) * ((size_t)(c->L * (c->L - 1) / 2) * m + (c->nb + 1)) + elem * (threads / 32) * sb * 128;
+  return sizeof(double) * ((size_t)(c->L * (c->L - 1) / 2) * m + (c->nb + kZeros)) + elem * (threads / 32) * sb * 128;
 }
 
 template <typename T, int M, int SB>
@@ -588,7 +607,7 @@ void launch_mma(sbdgpu_ctx* c, const T* C, T* S, const AlphaSingles& as, int nt,
 // for the zero: such bases keep the gather kernel.
 void build_ab_tiles(sbdgpu_ctx* c, SpinTables& t, const std::vector<uint64_t>& strs) {
   const size_t n = strs.size();
-  if (n == 0 || n > 65535) return;
+  if (n == 0 || n + kZeros > 65536) return;
   std::vector<uint64_t> sorted(strs);
   std::sort(sorted.begin(), sorted.end());
   if (std::adjacent_find(sorted.begin(), sorted.end()) != sorted.end()) return;

@@ -1,9 +1,9 @@
 // Many independent problems at once: a device-resident Davidson.
 //
-// The single-problem Davidson (api.cu) keeps the projected matrix, its
-// eigenvectors and every norm and overlap on the host, so each step waits on
-// the GPU for every dot product.  For small problems those waits, not the
-// kernels, take the time.  Here every quantity of a step stays on the device:
+// The single-problem Davidson (api.cu) keeps the projected matrix and its
+// eigenvectors on the host, so each step waits on the GPU twice and issues its
+// launches one by one.  For small problems those waits, not the kernels, take
+// the time.  Here every quantity of a step stays on the device:
 //
 //   dots        reductions whose sums stay in the problem's block of device
 //               memory (krylov.cu)
@@ -18,10 +18,10 @@
 // Ritz update and the norms -- is a fixed sequence of launches on the
 // problem's stream with fixed pointers.  Each (problem, Krylov index) step is
 // captured into a CUDA graph when it runs for the second time and then
-// replayed: one launch per problem per step.  One host thread drives all problems in rounds: it launches one
-// step graph per unconverged problem, then waits once for the round and reads
-// each problem's residual norm (8 bytes, copied to pinned memory inside the
-// graph).  The vectors of all problems come from one device allocation made
+// replayed: one launch per problem per step.  One host thread drives all
+// problems in rounds: it launches one step graph per unconverged problem, then
+// waits once for the round and reads each problem's residual norm (8 bytes,
+// copied to pinned memory inside the graph).  The vectors of all problems come from one device allocation made
 // before the first round.  The algorithm is the reference's
 // (chemistry/tpb/davidson.h:661-923): collapse restart to the Ritz vector,
 // the diagonal correction regularised by 1e-12, modified Gram-Schmidt, and the

@@ -1,5 +1,6 @@
 // Off-diagonal part of the one- and two-particle RDMs (Correlation,
-// chemistry/tpb/correlation.h:194-443; the diagonal part is in misc.cu).
+// chemistry/tpb/correlation.h:194-443; the diagonal part is in misc.cu), for the
+// bases without alpha-beta tiles; the others take products (rdm_mma.cu).
 //
 // The reference walks every determinant and each of its connected
 // determinants and adds OneDiff/TwoDiffCorrelation terms (correlation.h:

@@ -138,7 +138,7 @@ def test_integer_products_of_padded_string_counts(na, nb):
 
 def test_tiles_without_stages():
     # 48 orbitals and 19,990 beta strings leave no shared memory for staged results beside eight singles' integrals
-    # and the row of C; one string more than 20,015 keeps the gather kernel
+    # and the row of C; more than 20,000 keep the gather kernel
     ints = synth.make_integrals(48, 3)
     b = synth.selected_strings(48, 4, 20100, np.diag(ints.h), 4)
     a = b[[0, 1, 2, 5, 9]]
