@@ -307,8 +307,7 @@ __device__ __forceinline__ void mma8(double (&d)[4], double a0, double b) {
 // wavefronts, the FP64 tensor pipe 62 % busy).  Alpha-beta term with the beta
 // singles' Coulomb part, gather kernel (without it) -> tiles: 144M determinants
 // 198 -> 84 ms, 16M 11.2 -> 4.3 ms, 1501 x 803 strings 0.85 -> 0.34 ms,
-// 495 x 495 0.10 -> 0.07 ms; the products alone take 48 / 2.1 ms of the tensor
-// pipe at the first two.  24 and 32 alpha
+// 495 x 495 0.10 -> 0.07 ms.  24 and 32 alpha
 // singles per CTA (fewer loads of C per product) and entries fetched a batch
 // ahead were no faster: fewer warps fit, and the loads were not what waited.
 //
@@ -474,35 +473,35 @@ __device__ __forceinline__ void tiles(const MmaArgs<T>& a, const unsigned char* 
           if (2 * q + u < len1) atomicAdd(row + len0 + 2 * q + u, val(acc1[2 * b + u]));
         }
       }
-      continue;
-    }
+    } else {
 #pragma unroll
-    for (int b0 = 0; b0 < BLOCKS; b0 += SB > 0 ? SB : BLOCKS) {
-      constexpr int ROWS = 8 * (SB < BLOCKS ? SB : BLOCKS);
-      if (a.bulk) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // the last lines are read
-      __syncwarp();
+      for (int b0 = 0; b0 < BLOCKS; b0 += SB) {
+        constexpr int ROWS = 8 * (SB < BLOCKS ? SB : BLOCKS);
+        if (a.bulk) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // the last lines are read
+        __syncwarp();
 #pragma unroll
-      for (int b = b0; b < b0 + SB && b < BLOCKS; b++) {
-        const uint32_t sg = neg[8 * b + r];
-        const auto val = [&](double x) { return (T)__hiloint2double(__double2hiint(x) ^ (int)sg, __double2loint(x)); };
-        T* row = stage + (8 * (b - b0) + r) * 16;
-        put2(row, 2 * q, len0, val(acc0[2 * b]), val(acc0[2 * b + 1]));
-        put2(row + len0, 2 * q, len1, val(acc1[2 * b]), val(acc1[2 * b + 1]));
-      }
-      const int* to = tgt + 8 * b0;
-      if (bulk) {
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncwarp();
-        if (lane < ROWS && to[lane] >= 0)
-          bulk_add(a.S + (size_t)to[lane] * a.nb + at.x, smem_addr(stage + lane * 16),
-                   (uint32_t)len * (uint32_t)sizeof(T));
-        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-      } else {
-        __syncwarp();
-        const int col = lane & 15;
+        for (int b = b0; b < b0 + SB && b < BLOCKS; b++) {
+          const uint32_t sg = neg[8 * b + r];
+          const auto val = [&](double x) { return (T)__hiloint2double(__double2hiint(x) ^ (int)sg, __double2loint(x)); };
+          T* row = stage + (8 * (b - b0) + r) * 16;
+          put2(row, 2 * q, len0, val(acc0[2 * b]), val(acc0[2 * b + 1]));
+          put2(row + len0, 2 * q, len1, val(acc1[2 * b]), val(acc1[2 * b + 1]));
+        }
+        const int* to = tgt + 8 * b0;
+        if (bulk) {
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          __syncwarp();
+          if (lane < ROWS && to[lane] >= 0)
+            bulk_add(a.S + (size_t)to[lane] * a.nb + at.x, smem_addr(stage + lane * 16),
+                     (uint32_t)len * (uint32_t)sizeof(T));
+          asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        } else {
+          __syncwarp();
+          const int col = lane & 15;
 #pragma unroll 4
-        for (int row = lane >> 4; row < ROWS; row += 2)
-          if (to[row] >= 0 && col < len) atomicAdd(a.S + (size_t)to[row] * a.nb + at.x + col, stage[row * 16 + col]);
+          for (int row = lane >> 4; row < ROWS; row += 2)
+            if (to[row] >= 0 && col < len) atomicAdd(a.S + (size_t)to[row] * a.nb + at.x + col, stage[row * 16 + col]);
+        }
       }
     }
   }

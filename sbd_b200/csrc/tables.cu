@@ -141,19 +141,16 @@ static void build_one(sbdgpu_ctx* c, SpinTables& t, const uint64_t* dstr, size_t
   cudaStream_t st = c->stream;
   t.n = n;
   int ni = (int)n;
-  int *cs = nullptr, *cd = nullptr;
-  cs = (int*)dev_alloc(sizeof(int) * (n + 1));
-  cd = (int*)dev_alloc(sizeof(int) * (n + 1));
+  int* counts = (int*)dev_alloc(sizeof(int) * (2 * n + 1));  // singles, then doubles
   int threads = 256;
   int blocks = (int)((n * 32 + threads - 1) / threads);
-  count_kernel<<<blocks, threads, 0, st>>>(dstr, ni, cs, cd);
+  count_kernel<<<blocks, threads, 0, st>>>(dstr, ni, counts, counts + n);
   SBD_CUDA(cudaGetLastError());
-  std::vector<int> hs(n), hd(n);
-  SBD_CUDA(cudaMemcpyAsync(hs.data(), cs, sizeof(int) * n, cudaMemcpyDeviceToHost, st));
-  SBD_CUDA(cudaMemcpyAsync(hd.data(), cd, sizeof(int) * n, cudaMemcpyDeviceToHost, st));
+  std::vector<int> h(2 * n + 1);
+  SBD_CUDA(cudaMemcpyAsync(h.data(), counts, sizeof(int) * 2 * n, cudaMemcpyDeviceToHost, st));
   SBD_CUDA(cudaStreamSynchronize(st));
-  cudaFree(cs);
-  cudaFree(cd);
+  cudaFree(counts);
+  const int *hs = h.data(), *hd = hs + n;
   t.h_s_off.assign(n + 1, 0);
   t.h_d_off.assign(n + 1, 0);
   for (size_t i = 0; i < n; i++) {
@@ -162,7 +159,7 @@ static void build_one(sbdgpu_ctx* c, SpinTables& t, const uint64_t* dstr, size_t
   }
   t.ns = (uint64_t)t.h_s_off[n];
   t.nd = (uint64_t)t.h_d_off[n];
-  t.max_s = n ? *std::max_element(hs.begin(), hs.end()) : 0;
+  t.max_s = n ? *std::max_element(hs, hs + n) : 0;
   t.s_off = (int64_t*)dev_alloc(sizeof(int64_t) * (n + 1));
   t.d_off = (int64_t*)dev_alloc(sizeof(int64_t) * (n + 1));
   SBD_CUDA(cudaMemcpyAsync(t.s_off, t.h_s_off.data(), sizeof(int64_t) * (n + 1), cudaMemcpyHostToDevice, st));
@@ -176,10 +173,7 @@ static void build_one(sbdgpu_ctx* c, SpinTables& t, const uint64_t* dstr, size_t
   fill_kernel<<<blocks, threads, 0, st>>>(dstr, ni, c->L, t.s_off, t.d_off, c->h1, c->vf, c->P, t.s_idx,
                                           t.s_info, t.s_val, t.d_idx, t.d_val);
   SBD_CUDA(cudaGetLastError());
-  if (!beta) {
-    SBD_CUDA(cudaStreamSynchronize(st));
-    return;
-  }
+  if (!beta) return;
   // sliced ELL of the singles, which the alpha-beta kernels read for the beta strings
   t.nslice = (n + kSlice - 1) / kSlice;
   std::vector<int32_t> w(t.nslice, 0);
