@@ -155,7 +155,9 @@ __global__ void __launch_bounds__(128) same_spin_kernel(int S, const double* __r
       const double v = info & 0x80000000u ? -row[j] : row[j];
       if (v == 0.0) continue;
       atomicAdd(&one[S * L2 + p + L1 * q], v);
-      for (uint64_t o = str[i] & str[j]; o; o &= o - 1) {  // spectators of this spin
+      // Spectators of this spin.  The created orbital's own terms cancel: they are
+      // added, as the reference adds them, only where their difference is a NaN.
+      for (uint64_t o = isfinite(v) ? str[i] & str[j] : str[i]; o; o &= o - 1) {
         const int r = low_bit(o);
         add(p, r, r, q, v);
         add(r, p, q, r, v);
@@ -312,6 +314,44 @@ __global__ void __launch_bounds__(kAbThreads) opposite_spin_kernel(
   }
   const size_t ncol = (size_t)ntile * 8;
   const int npair = L * (L - 1) / 2;
+  const auto add = [&](int g, int d, int t, int col, double v) {
+    if (v == 0.0) return;
+    const size_t at = d * ncol + (size_t)t * 8 + col;
+    if (gpair[g] >= 0) {
+      atomicAdd(&G[(size_t)gpair[g] * 2 * ncol + at], v);
+    } else {
+      for (uint64_t o = astr[ja]; o; o &= o - 1) atomicAdd(&G[(size_t)(npair + low_bit(o)) * 2 * ncol + at], v);
+    }
+  };
+  // A NaN or an infinity times the zero of an empty slot reaches columns that no
+  // entry of its beta string has: the warp's elements entry by entry instead.
+  bool bad = false;
+#pragma unroll
+  for (int i = 0; i < kWarpTiles; i++)
+#pragma unroll
+    for (int d = 0; d < 2; d++)
+#pragma unroll
+      for (int x = 0; x < 4; x++) bad |= !isfinite(acc[i][d][x]);
+  if (__any_sync(0xffffffffu, bad)) {
+    for (int x = lane; x < 16 * nt * 8; x += 32) {
+      const int g = x & 15, t = t0 + (x >> 7), col = (x >> 4) & 7;
+      if (tgt[g] < 0) continue;
+      const double* arow = Wp + (size_t)tgt[g] * nb;
+      double fwd = 0.0, back = 0.0;
+      for (size_t ib = 0; ib < nb; ib++) {
+        const uint32_t w = __ldg(&ent[((ib >> 2) * ntile + t) * 32 + col * 4 + (ib & 3)]);
+        if ((w & 0xFFFFu) == (uint32_t)nb) continue;
+        const double y = arow[ib] * ((w ^ gneg[g]) & 0x80000000u ? -wrow[w & 0xFFFFu] : wrow[w & 0xFFFFu]);
+        if (w & 0x40000000u)
+          fwd += y;
+        else
+          back += y;
+      }
+      add(g, 0, t, col, fwd);
+      add(g, 1, t, col, back);
+    }
+    return;
+  }
 #pragma unroll
   for (int h = 0; h < 2; h++) {
     const int g = r + 8 * h;
@@ -323,16 +363,7 @@ __global__ void __launch_bounds__(kAbThreads) opposite_spin_kernel(
 #pragma unroll
       for (int d = 0; d < 2; d++)
 #pragma unroll
-        for (int u = 0; u < 2; u++) {
-          const double v = s * acc[i][d][2 * h + u];
-          if (v == 0.0) continue;
-          const size_t at = d * ncol + (size_t)(t0 + i) * 8 + 2 * q + u;
-          if (gpair[g] >= 0) {
-            atomicAdd(&G[(size_t)gpair[g] * 2 * ncol + at], v);
-          } else {
-            for (uint64_t o = astr[ja]; o; o &= o - 1) atomicAdd(&G[(size_t)(npair + low_bit(o)) * 2 * ncol + at], v);
-          }
-        }
+        for (int u = 0; u < 2; u++) add(g, d, t0 + i, 2 * q + u, s * acc[i][d][2 * h + u]);
     }
   }
 }

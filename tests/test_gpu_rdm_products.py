@@ -46,3 +46,21 @@ def test_alpha_rows_and_columns(norb, nea):
 
 def test_repeated_strings_keep_the_scalar_kernels():
     _check(8, 3, 3, 20, 21, 3, repeat=2)
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_non_finite_input_stays_where_its_terms_go(bad):
+    ints = synth.make_integrals(9, 8)
+    a, b = synth.full_strings(9, 3)[::2], synth.full_strings(9, 3)[1::2]
+    ctx = sbd_b200.context_from_integrals(ints, a, b)
+    W = np.random.default_rng(8).normal(size=ctx.n)
+    W /= np.linalg.norm(W)
+    W[7 * ctx.nb + 11] = bad
+    got = ctx.rdm(W)
+    ref = oracle.Oracle(9, a, b, ints.ecore, ints.h, ints.eri).correlation(W)
+    for x, r in zip(got, ref):
+        finite = np.isfinite(r)
+        assert finite.any() and not finite.all()
+        assert np.array_equal(np.isfinite(x), finite)
+        assert np.abs(x[finite] - r[finite]).max() <= TOL
+    ctx.close()
