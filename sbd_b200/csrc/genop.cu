@@ -35,6 +35,7 @@
 #include <cmath>
 #include <cstring>
 #include <iostream>
+#include <mutex>
 #include <numeric>
 
 #include <cub/device/device_radix_sort.cuh>
@@ -51,6 +52,7 @@ struct sbdgpu_genop {
   int sign = 1;
   uint64_t* states = nullptr;
   void* slots = nullptr;      // hash table, Slot<nw> each
+  std::mutex mult_mu;         // the slots' elements belong to one mult at a time, from its scatter on
   int64_t* slot_of = nullptr; // [n] slot of every state
   uint64_t hmask = 0;         // slots - 1
   uint64_t absent[4] = {};    // key of an empty slot: a configuration outside the basis
@@ -540,6 +542,8 @@ TermList<NW> term_list(const sbdgpu_genop* g) {
 template <int NW>
 void mult_nw(sbdgpu_genop* g, const double* C, double* W) {
   Slot<NW>* slots = static_cast<Slot<NW>*>(g->slots);
+  // both launches in a row on the object's stream, whichever host threads call
+  std::lock_guard<std::mutex> lock(g->mult_mu);
   scatter_kernel<NW><<<(unsigned)std::min<size_t>(blocks_for(g->n), 148 * 8), kThreads, 0, g->base.stream>>>(
       slots, g->slot_of, C, g->n);
   SBD_CUDA(cudaGetLastError());

@@ -281,3 +281,30 @@ def test_cpp_generic_path_on_the_gpu():
     assert n == len(strs) ** 2 and n_new == n
     assert abs(e - e_tpb) < 1e-9
     assert abs(h2 - e * e) < 1e-7 * e * e
+
+
+def test_one_operator_from_two_host_threads():
+    import threading
+
+    import torch
+
+    rng = np.random.default_rng(4)
+    ints, states = _basis([0, 3, 5, 9, 12, 20, 33, 47, 50, 63], 4, 0.1, rng, 1)
+    g = sbd_b200.GenOp(states)
+    g.set_terms(*_operator(rng, [0, 3, 5, 9, 12, 20, 33, 47, 50, 63], 30, 60, True))
+    C = [torch.tensor(rng.normal(size=len(ints)), device="cuda") for _ in range(2)]
+    ref = [g.mult(c.cpu().numpy()) for c in C]
+    W = [torch.zeros(300, len(ints), dtype=torch.float64, device="cuda") for _ in C]
+    torch.cuda.synchronize()
+
+    def work(k):
+        for w in W[k]:
+            g.mult_device(C[k].data_ptr(), w.data_ptr())
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for w, r in zip(W, ref):
+        assert np.abs(w.cpu().numpy() - r).max() <= 1e-12 * np.abs(r).max()
+    g.close()
