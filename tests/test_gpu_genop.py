@@ -308,3 +308,22 @@ def test_one_operator_from_two_host_threads():
     for w, r in zip(W, ref):
         assert np.abs(w.cpu().numpy() - r).max() <= 1e-12 * np.abs(r).max()
     g.close()
+
+
+@pytest.mark.parametrize("nw,sites", [(1, [0, 3, 5, 9, 12, 20]), (2, [1, 17, 62, 64, 90, 127])])
+@pytest.mark.parametrize("bad", [np.inf, np.nan])
+def test_infinite_coefficient_reaches_only_states_with_a_target(bad, nw, sites):
+    # every pair of sites but {sites[4], sites[5]}: the hop sites[2] -> sites[4] leads out of the basis from the
+    # state {sites[2], sites[5]}
+    pairs = [p for p in itertools.combinations(sites, 2) if p != (sites[4], sites[5])]
+    states = np.array([_words((1 << p) | (1 << q), nw) for p, q in pairs], dtype=np.uint64)
+    hop = [(True, sites[2]), (False, sites[4])]
+    g = sbd_b200.GenOp(states)
+    g.set_terms([], [(bad, hop), (0.5, [(True, sites[0]), (False, sites[1])])])
+    C = np.arange(1.0, len(pairs) + 1)
+    got = g.mult(C)
+    hit = np.array([sites[2] in p and sites[4] not in p and sites[5] not in p for p in pairs])
+    assert hit.any() and not np.isfinite(got[hit]).any() and np.isfinite(got[~hit]).all()
+    g.set_terms([], [(0.5, [(True, sites[0]), (False, sites[1])])])
+    assert np.array_equal(got[~hit], g.mult(C)[~hit])
+    g.close()
