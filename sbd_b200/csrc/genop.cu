@@ -120,6 +120,11 @@ struct alignas(NW == 1 ? 16 : NW == 2 ? 32 : 64) Slot {
   double val;
 };
 
+template <int NW>
+struct Words {
+  uint64_t w[NW];
+};
+
 // The off-diagonal terms on the device.
 template <int NW>
 struct TermList {
@@ -270,10 +275,6 @@ __device__ __forceinline__ bool apply_term(const Term<NW>& t, const uint64_t* v,
 // probing for 32 at a time: 4.9 against 4.8 ms.)
 constexpr int kMultWarps = kThreads / 32;
 template <int NW>
-struct Words {
-  uint64_t w[NW];
-};
-template <int NW>
 __global__ void __launch_bounds__(kThreads) mult_kernel(const uint64_t* __restrict__ states, size_t n,
                                                        const Slot<NW>* __restrict__ slots, uint64_t hmask,
                                                        Words<NW> absent, TermList<NW> tl,
@@ -357,46 +358,99 @@ int guarded(sbdgpu_genop* g, F&& f) {
   }
 }
 
-// The basis on the device: states, hash table and every state's slot.
+constexpr uint32_t kFree = 0xFFFFFFFFu;
+
+// Every state claims the first free slot of its search: owner of a slot, slot
+// of a state; *repeated is set where a search meets the state's own key.
+template <int NW>
+__global__ void insert_kernel(const uint64_t* __restrict__ states, size_t n, uint64_t hmask,
+                              uint32_t* __restrict__ owner, int64_t* __restrict__ slot_of, int* __restrict__ repeated) {
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+    uint64_t w[NW];
+#pragma unroll
+    for (int x = 0; x < NW; x++) w[x] = states[i * NW + x];
+    uint64_t h = hash_state<NW>(w, hmask);
+    for (uint64_t probe = 0; probe <= hmask; probe++, h = (h + 1) & hmask) {
+      const uint32_t other = atomicCAS(&owner[h], kFree, (uint32_t)i);
+      if (other == kFree) {
+        slot_of[i] = (int64_t)h;
+        break;
+      }
+      bool eq = true;
+#pragma unroll
+      for (int x = 0; x < NW; x++) eq &= states[(size_t)other * NW + x] == w[x];
+      if (eq) {
+        *repeated = 1;
+        break;
+      }
+    }
+  }
+}
+
+template <int NW>
+__global__ void keys_kernel(const uint64_t* __restrict__ states, const uint32_t* __restrict__ owner, size_t count,
+                            Words<NW> absent, Slot<NW>* __restrict__ slots) {
+  for (size_t h = (size_t)blockIdx.x * blockDim.x + threadIdx.x; h < count; h += (size_t)gridDim.x * blockDim.x) {
+    const uint32_t i = owner[h];
+    Slot<NW> s;
+#pragma unroll
+    for (int x = 0; x < NW; x++) s.key[x] = i == kFree ? absent.w[x] : states[(size_t)i * NW + x];
+    s.val = 0.0;
+    slots[h] = s;
+  }
+}
+
+// The basis on the device: states, hash table and every state's slot.  The
+// table is filled there: 1,002,001 states take 4 ms, on the host they took 73-90
+// ms (24-30 ms as a half-full table of keys and indices), most of it the
+// table's cache misses and its copy.
 template <int NW>
 void build_basis(sbdgpu_genop* g, const uint64_t* states) {
   const size_t n = g->n;
+  if (n >= kFree) throw Error{SBDGPU_ERR_ALLOC, "basis larger than device memory"};
   cudaStream_t st = g->base.stream;
   // a power of two of at least four times the states (twice above 1 GiB: the
   // lanes of a warp wait for their longest search)
   size_t count = 1024;
   while (count < 4 * n && (count < 2 * n || count * sizeof(Slot<NW>) < (size_t(1) << 30))) count <<= 1;
   g->hmask = count - 1;
-  std::vector<int64_t> at(count, -1), slot_of(n);  // state of a slot, slot of a state
-  // slot of configuration w, or of the empty slot that ends its search
-  const auto find = [&](const uint64_t* w) {
-    uint64_t h = hash_state<NW>(w, g->hmask);
-    while (at[h] >= 0 && !std::equal(w, w + NW, &states[(size_t)at[h] * NW])) h = (h + 1) & g->hmask;
-    return h;
-  };
+  // the first configuration from the top that no state has
+  std::vector<uint64_t> top;  // distances of the states near it
   for (size_t i = 0; i < n; i++) {
-    const uint64_t h = find(&states[i * NW]);
-    if (at[h] >= 0) throw Error{SBDGPU_ERR_ARG, "repeated basis state"};
-    at[h] = (int64_t)i;
-    slot_of[i] = (int64_t)h;
-    for (int x = 0; x < NW; x++) g->site_or[x] |= states[i * NW + x];
+    bool high = true;
+    for (int x = 0; x < NW; x++) {
+      g->site_or[x] |= states[i * NW + x];
+      high &= x == 0 || states[i * NW + x] == ~0ull;
+    }
+    if (high && ~states[i * NW] < n) top.push_back(~states[i * NW]);
   }
-  uint64_t none[NW];
-  std::fill(none, none + NW, ~0ull);
-  while (at[find(none)] >= 0) none[0]--;
-  std::memcpy(g->absent, none, sizeof(none));
-  std::vector<Slot<NW>> table(count);
-  for (size_t h = 0; h < count; h++) {
-    std::memcpy(table[h].key, at[h] >= 0 ? &states[(size_t)at[h] * NW] : none, sizeof(none));
-    table[h].val = 0.0;
-  }
+  std::sort(top.begin(), top.end());
+  Words<NW> absent;
+  std::fill(absent.w, absent.w + NW, ~0ull);
+  for (uint64_t d : top)
+    if (d == ~absent.w[0]) absent.w[0]--;
+  std::memcpy(g->absent, absent.w, sizeof(absent.w));
   g->states = (uint64_t*)sbdgpu::dev_alloc(sizeof(uint64_t) * n * NW);
   g->slots = sbdgpu::dev_alloc(sizeof(Slot<NW>) * count);
   g->slot_of = (int64_t*)sbdgpu::dev_alloc(sizeof(int64_t) * n);
+  sbdgpu::Arena arena(st);
+  uint32_t* owner = nullptr;
+  int* repeated = nullptr;
+  arena.add(&owner, count);
+  arena.add(&repeated, 1);
+  arena.commit();
   SBD_CUDA(cudaMemcpyAsync(g->states, states, sizeof(uint64_t) * n * NW, cudaMemcpyHostToDevice, st));
-  SBD_CUDA(cudaMemcpyAsync(g->slots, table.data(), sizeof(Slot<NW>) * count, cudaMemcpyHostToDevice, st));
-  SBD_CUDA(cudaMemcpyAsync(g->slot_of, slot_of.data(), sizeof(int64_t) * n, cudaMemcpyHostToDevice, st));
-  SBD_CUDA(cudaStreamSynchronize(st));  // the host copies leave scope
+  SBD_CUDA(cudaMemsetAsync(owner, 0xFF, sizeof(uint32_t) * count, st));
+  SBD_CUDA(cudaMemsetAsync(repeated, 0, sizeof(int), st));
+  const auto grid = [](size_t m) { return (unsigned)std::min<size_t>((m + kThreads - 1) / kThreads, 148 * 8); };
+  insert_kernel<NW><<<grid(n), kThreads, 0, st>>>(g->states, n, g->hmask, owner, g->slot_of, repeated);
+  SBD_CUDA(cudaGetLastError());
+  keys_kernel<NW><<<grid(count), kThreads, 0, st>>>(g->states, owner, count, absent, static_cast<Slot<NW>*>(g->slots));
+  SBD_CUDA(cudaGetLastError());
+  int r = 0;
+  SBD_CUDA(cudaMemcpyAsync(&r, repeated, sizeof(int), cudaMemcpyDeviceToHost, st));
+  SBD_CUDA(cudaStreamSynchronize(st));
+  if (r) throw Error{SBDGPU_ERR_ARG, "repeated basis state"};
 }
 
 // One list's terms as host records.  Off-diagonal terms that repeat a site

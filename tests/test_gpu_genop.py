@@ -327,3 +327,26 @@ def test_infinite_coefficient_reaches_only_states_with_a_target(bad, nw, sites):
     g.set_terms([], [(0.5, [(True, sites[0]), (False, sites[1])])])
     assert np.array_equal(got[~hit], g.mult(C)[~hit])
     g.close()
+
+
+@pytest.mark.parametrize("nw,n", [(1, 1), (1, 255), (1, 257), (1, 20000), (2, 20000), (4, 3000)])
+def test_hash_table_holds_every_state_once(nw, n):
+    # states without structure, the highest configurations among them; one off-diagonal term without operators adds
+    # each state's own element
+    rng = np.random.default_rng(n)
+    states = np.unique(rng.integers(0, 2 ** 64, size=(n, nw), dtype=np.uint64), axis=0)
+    top = np.full((min(n, 3), nw), 2 ** 64 - 1, dtype=np.uint64)
+    top[:, 0] -= np.array([0, 1, 3], dtype=np.uint64)[:len(top)]
+    states = rng.permutation(np.concatenate([states[len(top):], top]))
+    g = sbd_b200.GenOp(states, sign=False)
+    g.set_terms([], [(1.0, [])])
+    C = rng.normal(size=len(states))
+    assert np.array_equal(g.mult(C), C)
+    # a number operator: only the states with site 1 occupied
+    g.set_terms([], [(1.0, [(True, 1), (False, 1)])])
+    has = (states[:, 0] >> np.uint64(1)) & np.uint64(1) == 1
+    assert np.array_equal(g.mult(C), np.where(has, C, 0.0))
+    g.close()
+    if n > 1:
+        with pytest.raises(sbd_b200.SbdGpuError):
+            sbd_b200.GenOp(np.concatenate([states, states[n // 2:n // 2 + 1]]))
