@@ -681,67 +681,72 @@ void build_ab_tiles(sbdgpu_ctx* c, SpinTables& t, const std::vector<uint64_t>& s
 // Without stages the kernel may use all that the opt-in limit leaves beside its
 // own 128 bytes (budget is the limit less 1 KiB): eight singles beside 20,000
 // beta strings at norb 48, where 490 ms replace the 1,180 ms of the gather
-// kernel at four singles (400M determinants; FP32: 446 ms).  Where stages fit
-// they stay the better choice: 93 against 125 ms at 144M.
+// kernel at four singles (400M determinants; FP32: 446 ms).
 constexpr size_t kUnstagedExtra = 1024 - 128;
 
-// Alpha singles per CTA of the tile kernel for a wanted number (0: the larger
-// that fits); 0 when this basis has no tiles or they do not fit.
-int ab_mma_group(const sbdgpu_ctx* c, int want, size_t budget) {
-  if (!c->tab[1].tile_grp) return 0;
-  for (int m : {16, 8})
-    if ((want == 0 || want == m) && mma_smem(c, m, 128, sizeof(double), 1) <= budget) return m;
-  if (want == 0 && mma_smem(c, 8, 0, 0, 0) <= budget + kUnstagedExtra) return 8;
-  return 0;
-}
-
-// The alpha-beta term by tiles, m alpha singles per CTA, nt threads (0: the
-// default); beta_j: the beta singles' Coulomb part as well (whole vectors
-// only).  Default threads: those that put most warps on an SM beside the shared
-// memory they need (at equal warps the smaller CTA), fewer while the warps
-// outnumber the groups; results are staged for one block of alpha singles at a
-// time where that lets more warps in.  Alpha-beta ms: 16M determinants 6.0 at
-// 256 threads, 4.6 at 512, 5.6 at 768; 1501 x 803 strings 0.40 at 128, 0.34 at
-// 256, 0.37 at 512; 144M 93 at 768 with both blocks staged, 97 and 88.6 at 768
-// and 1,024 with one (FP32 vectors: 82 at 768, 77 at 1,024).
-template <typename T>
-void ab_mma(sbdgpu_ctx* c, const T* C, T* S, const AlphaSingles& as, int m, int nt, size_t budget, bool beta_j) {
-  int sb = m / 8;
-  if (nt == 0) {
-    int best = 0;
-    for (int b = m / 8; b >= 1; b--)
+// Launch shape of the tile kernel for vectors of elem bytes.  group, threads:
+// what the context was tuned to (0, 0: the default).  m = 0 when this basis has
+// no tiles or they do not fit.
+//
+// Default: what bounds the kernel below some 24 warps per SM is latency, so the
+// shape with most warps beside the shared memory they need (at equal warps the
+// smaller CTA, with more stages); sixteen singles per CTA while 24 warps fit with
+// them, else eight, without stages where that lets more warps in.  Alpha-beta ms
+// at 16 singles and 24, 16, 8, 4 warps against 8 singles and 32 warps: 300 x
+// 15,000 strings at norb 36 0.98 against 1.12, 16,500 1.29 against 1.20, 17,200
+// 2.24 against 1.20, 17,900 4.28 against 1.18 (gather kernel 3.3).  Eight singles,
+// 24 and 4 warps with stages against 32 without: 200 x 16,500 strings at norb 48
+// 1.09 against 1.01, 19,300 6.06 against 1.20 (gather kernel 2.9).  Fewer threads
+// while the warps outnumber the groups.
+// Whole bases: 16M determinants 6.0 at 256 threads, 4.2 at 512, 5.0 at 768; 1501 x
+// 803 strings 0.40 at 128, 0.34 at 256, 0.37 at 512; 144M 93 at 768 with both
+// blocks staged, 97 and 88.6 at 768 and 1,024 with one (FP32 vectors: 82 at 768,
+// 77 at 1,024).
+MmaShape ab_mma_shape(const sbdgpu_ctx* c, int group, int threads, size_t elem, size_t budget) {
+  if (!c->tab[1].tile_grp) return {};
+  if (group > 0) {  // as many stages as fit beside the row of C
+    MmaShape s{group, threads, group / 8};
+    if ((group != 16 && group != 8) || mma_smem(c, group, 128, sizeof(double), 1) > budget) return {};
+    if (mma_smem(c, group, s.nt, elem, s.sb) > budget) s.sb = 1;
+    while (s.nt > 128 && mma_smem(c, group, s.nt, elem, s.sb) > budget) s.nt -= 128;
+    return s;
+  }
+  MmaShape s;
+  int best = 0;
+  for (int m : {16, 8}) {
+    for (int sb = m / 8; sb >= (m == 8 ? 0 : 1); sb--)
       for (int t : {256, 512, 768, 1024}) {
-        const size_t smem = mma_smem(c, m, t, sizeof(T), b);
-        if (smem > budget) break;
+        const size_t smem = mma_smem(c, m, t, elem, sb);
+        if (smem > budget + (sb == 0 ? kUnstagedExtra : 0)) break;
         const int warps = (int)std::min<size_t>(228 * 1024 / (smem + 1024), 1024 / t) * (t / 32);
         if (warps > best) {
           best = warps;
-          nt = t;
-          sb = b;
+          s = {m, t, sb};
         }
       }
-    if (nt == 0) {
-      const bool staged = mma_smem(c, m, 128, sizeof(T), 1) <= budget;
-      nt = staged ? 128 : 1024;
-      sb = staged ? 1 : 0;
-    }
-    while (nt > 128 && (size_t)(nt / 2) >= c->tab[1].n_tile_grp * 32) nt /= 2;
-  } else {  // a tuned number: as many stages as fit beside the row of C
-    if (mma_smem(c, m, nt, sizeof(T), sb) > budget) sb = 1;
-    while (nt > 128 && mma_smem(c, m, nt, sizeof(T), sb) > budget) nt -= 128;
+    if (best >= 24) break;
+    if (m == 16) best = 0;  // eight singles fit wherever sixteen do, with no fewer warps
   }
-  if (m == 16 && sb == 2)
-    launch_mma<T, 16, 2>(c, C, S, as, nt, beta_j);
-  else if (m == 16)
-    launch_mma<T, 16, 1>(c, C, S, as, nt, beta_j);
-  else if (sb == 1)
-    launch_mma<T, 8, 1>(c, C, S, as, nt, beta_j);
-  else
-    launch_mma<T, 8, 0>(c, C, S, as, nt, beta_j);
+  while (s.nt > 128 && (size_t)(s.nt / 2) >= c->tab[1].n_tile_grp * 32) s.nt /= 2;
+  return s;
 }
 
-template void ab_mma<double>(sbdgpu_ctx*, const double*, double*, const AlphaSingles&, int, int, size_t, bool);
-template void ab_mma<float>(sbdgpu_ctx*, const float*, float*, const AlphaSingles&, int, int, size_t, bool);
+// The alpha-beta term by tiles; beta_j: the beta singles' Coulomb part as well
+// (whole vectors only).
+template <typename T>
+void ab_mma(sbdgpu_ctx* c, const T* C, T* S, const AlphaSingles& as, const MmaShape& s, bool beta_j) {
+  if (s.m == 16 && s.sb == 2)
+    launch_mma<T, 16, 2>(c, C, S, as, s.nt, beta_j);
+  else if (s.m == 16)
+    launch_mma<T, 16, 1>(c, C, S, as, s.nt, beta_j);
+  else if (s.sb == 1)
+    launch_mma<T, 8, 1>(c, C, S, as, s.nt, beta_j);
+  else
+    launch_mma<T, 8, 0>(c, C, S, as, s.nt, beta_j);
+}
+
+template void ab_mma<double>(sbdgpu_ctx*, const double*, double*, const AlphaSingles&, const MmaShape&, bool);
+template void ab_mma<float>(sbdgpu_ctx*, const float*, float*, const AlphaSingles&, const MmaShape&, bool);
 
 void preload_ab_mma(int device) {
   allow_dynamic_smem(reinterpret_cast<const void*>(ab_mma_kernel<double, 16, 2>), device);

@@ -204,9 +204,12 @@ struct AlphaSingles {
 };
 // ab_mma.cu: the alpha-beta term on the FP64 tensor pipe
 void build_ab_tiles(sbdgpu_ctx* c, SpinTables& t, const std::vector<uint64_t>& strs);
-int ab_mma_group(const sbdgpu_ctx* c, int want, size_t budget);
+struct MmaShape {
+  int m = 0, nt = 0, sb = 0;  // alpha singles and threads per CTA, blocks of eight singles staged at a time
+};
+MmaShape ab_mma_shape(const sbdgpu_ctx* c, int group, int threads, size_t elem, size_t budget);
 template <typename T>
-void ab_mma(sbdgpu_ctx* c, const T* C, T* S, const AlphaSingles& as, int m, int nt, size_t budget, bool beta_j);
+void ab_mma(sbdgpu_ctx* c, const T* C, T* S, const AlphaSingles& as, const MmaShape& s, bool beta_j);
 // same_dense.cu: the FP64 same-spin terms as one dense product
 bool dense_same_spin(const sbdgpu_ctx* c);
 void ensure_dense_fp64(sbdgpu_ctx* c);

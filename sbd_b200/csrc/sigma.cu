@@ -428,8 +428,8 @@ void alpha_beta(sbdgpu_ctx* c, const T* C, T* S, const T* vf, const AlphaSingles
   const bool tuned = sizeof(T) == 8 && c->ab_group > 0;
   const int g = tuned ? c->ab_group : 0, nt = tuned ? c->ab_threads : 0;
   if (sizeof(T) == 8 || c->N >= kTilesFp32) {
-    if (const int m = ab_mma_group(c, g, budget)) {
-      ab_mma<T>(c, C, S, as, m, nt, budget, beta_j);
+    if (const MmaShape s = ab_mma_shape(c, g, nt, sizeof(T), budget); s.m) {
+      ab_mma<T>(c, C, S, as, s, beta_j);
       return;
     }
   }
@@ -451,7 +451,7 @@ void alpha_beta(sbdgpu_ctx* c, const T* C, T* S, const T* vf, const AlphaSingles
 bool uses_tiles(const sbdgpu_ctx* c) {
   int dev_smem = 0;
   SBD_CUDA(cudaDeviceGetAttribute(&dev_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
-  return ab_mma_group(c, c->ab_group, (size_t)dev_smem - 1024) > 0;
+  return ab_mma_shape(c, c->ab_group, c->ab_threads, sizeof(double), (size_t)dev_smem - 1024).m > 0;
 }
 
 // Whether its same-spin terms are the dense product (else, or before that, the

@@ -150,3 +150,21 @@ def test_tiles_without_stages():
         ref = ctx.sigma(C)
         assert np.abs(got - ref).max() <= TOL * np.abs(ref).max()
         ctx.close()
+
+
+@pytest.mark.parametrize("norb,ne,nb", [(36, 4, 15001), (36, 4, 16600), (36, 4, 18200), (48, 4, 16400), (48, 4, 19001)])
+def test_launch_shapes_beside_long_rows_of_c(norb, ne, nb):
+    # sixteen singles at 24 warps; eight with stages where sixteen leave fewer than 24 (16 and 4 here); eight without
+    # stages where those leave fewer than 32 (24 and 4); FP32 vectors from half a million determinants
+    ints = synth.make_integrals(norb, 3)
+    b = synth.selected_strings(norb, ne, nb, np.diag(ints.h), 4)
+    a = b[:36]
+    ctx = sbd_b200.context_from_integrals(ints, a, b)
+    C = np.random.default_rng(nb).normal(size=ctx.n)
+    C /= np.linalg.norm(C)
+    got, mixed = ctx.sigma(C), ctx.sigma(C, precision=sbd_b200.MIXED)
+    ctx.set_tuning(4, 512)  # the gather kernel
+    ref = ctx.sigma(C)
+    assert np.abs(got - ref).max() <= TOL * np.abs(ref).max()
+    assert np.abs(mixed - ref).max() <= 2e-5 * np.abs(ref).max()
+    ctx.close()
