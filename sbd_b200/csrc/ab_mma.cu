@@ -697,7 +697,9 @@ constexpr size_t kUnstagedExtra = 1024 - 128;
 // 2.24 against 1.20, 17,900 4.28 against 1.18 (gather kernel 3.3).  Eight singles,
 // 24 and 4 warps with stages against 32 without: 200 x 16,500 strings at norb 48
 // 1.09 against 1.01, 19,300 6.06 against 1.20 (gather kernel 2.9).  Fewer threads
-// while the warps outnumber the groups.
+// while the warps outnumber the groups of beta strings and the eights of
+// integral rows that they load: 20,000 x 40 strings at norb 36 10.6 ms at 128
+// threads, 4.2 at 512 (gather kernel 9.9, FP32 4.8).
 // Whole bases: 16M determinants 6.0 at 256 threads, 4.2 at 512, 5.0 at 768; 1501 x
 // 803 strings 0.40 at 128, 0.34 at 256, 0.37 at 512; 144M 93 at 768 with both
 // blocks staged, 97 and 88.6 at 768 and 1,024 with one (FP32 vectors: 82 at 768,
@@ -727,7 +729,8 @@ MmaShape ab_mma_shape(const sbdgpu_ctx* c, int group, int threads, size_t elem, 
     if (best >= 24) break;
     if (m == 16) best = 0;  // eight singles fit wherever sixteen do, with no fewer warps
   }
-  while (s.nt > 128 && (size_t)(s.nt / 2) >= c->tab[1].n_tile_grp * 32) s.nt /= 2;
+  const size_t loads = (size_t)(c->L * (c->L - 1) / 2 + 7) / 8;
+  while (s.nt > 128 && (size_t)(s.nt / 2) >= 32 * std::max(c->tab[1].n_tile_grp, loads)) s.nt /= 2;
   return s;
 }
 

@@ -168,3 +168,15 @@ def test_launch_shapes_beside_long_rows_of_c(norb, ne, nb):
     assert np.abs(got - ref).max() <= TOL * np.abs(ref).max()
     assert np.abs(mixed - ref).max() <= 2e-5 * np.abs(ref).max()
     ctx.close()
+
+
+@pytest.mark.parametrize("nb", [1, 17, 40])
+def test_few_beta_strings_of_many_orbitals(nb):
+    # fewer groups of beta strings than warps: the integral rows keep the others busy
+    ints = synth.make_integrals(30, 5)
+    strs = synth.full_strings(30, 3)
+    ctx = sbd_b200.context_from_integrals(ints, strs[:500], strs[:nb])
+    C = np.random.default_rng(nb).normal(size=ctx.n)
+    ref = oracle.Oracle(30, strs[:500], strs[:nb], ints.ecore, ints.h, ints.eri).sigma(C)
+    assert np.abs(ctx.sigma(C) - ref).max() <= TOL * np.abs(ref).max()
+    ctx.close()
