@@ -1,8 +1,8 @@
 // Excitation tables on the GPU.
 //
 // Replaces GenerateExcitation (chemistry/tpb/helper.h:132-182): for every bra
-// string i, the ascending list of kets j with popcount(s_i ^ s_j) == 2 (single)
-// or == 4 (double).  One warp per bra row scans all kets 32 at a time; a warp
+// string i, the ascending list of kets j of its electron count with
+// popcount(s_i ^ s_j) == 2 (single) or == 4 (double).  One warp per bra row scans all kets 32 at a time; a warp
 // ballot compacts the hits in ascending j, so the lists are bit-exact with the
 // reference's.  The same pass computes each entry's payload: the orbitals
 // involved, the string-internal fermionic sign and the FP64 matrix element part
@@ -28,6 +28,13 @@ __device__ __forceinline__ bool neg_between(uint64_t s, int p, int q) {
   return __popcll(s & mask) & 1;
 }
 
+// Orbitals in which two strings of one electron count differ; 0 for different
+// counts, which no excitation connects (a pair of created orbitals has no pair
+// of annihilated ones to index the integrals with).
+__device__ __forceinline__ int distance(uint64_t si, uint64_t sj) {
+  return __popcll(si) == __popcll(sj) ? __popcll(si ^ sj) : 0;
+}
+
 __global__ void count_kernel(const uint64_t* __restrict__ s, int n, int* cs, int* cd) {
   int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   int lane = threadIdx.x & 31;
@@ -35,7 +42,7 @@ __global__ void count_kernel(const uint64_t* __restrict__ s, int n, int* cs, int
   uint64_t si = s[warp];
   int a = 0, b = 0;
   for (int j = lane; j < n; j += 32) {
-    int d = __popcll(si ^ s[j]);
+    int d = distance(si, s[j]);
     a += (d == 2);
     b += (d == 4);
   }
@@ -63,7 +70,7 @@ __global__ void fill_kernel(const uint64_t* __restrict__ s, int n, int L, const 
     int j = j0 + lane;
     uint64_t sj = j < n ? s[j] : si;
     uint64_t diff = si ^ sj;
-    int d = __popcll(diff);
+    int d = distance(si, sj);
     unsigned ms = __ballot_sync(0xffffffffu, d == 2);
     unsigned md = __ballot_sync(0xffffffffu, d == 4);
     if (d == 2) {

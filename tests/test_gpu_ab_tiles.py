@@ -180,3 +180,33 @@ def test_few_beta_strings_of_many_orbitals(nb):
     ref = oracle.Oracle(30, strs[:500], strs[:nb], ints.ecore, ints.h, ints.eri).sigma(C)
     assert np.abs(ctx.sigma(C) - ref).max() <= TOL * np.abs(ref).max()
     ctx.close()
+
+
+@pytest.mark.parametrize("nea,neb", [((3,), (2, 4)), ((2, 4), (3,)), ((3, 5), (2, 4)), ((3,), (3, 4)), ((2, 3), (3,))])
+def test_strings_of_several_electron_counts(nea, neb):
+    # the operator keeps each spin's electrons: one block per pair of counts
+    ints = synth.make_integrals(9, 7)
+    rng = np.random.default_rng(7)
+
+    def pick(counts):
+        s = np.concatenate([rng.permutation(synth.full_strings(9, ne))[:25] for ne in counts])
+        return np.sort(s), np.array([bin(int(x)).count("1") for x in np.sort(s)])
+    (a, ca), (b, cb) = pick(nea), pick(neb)
+    ctx = sbd_b200.context_from_integrals(ints, a, b)
+    C = rng.normal(size=(len(a), len(b)))
+    C /= np.linalg.norm(C)
+    ref = np.zeros_like(C)
+    one, two = 0.0, 0.0
+    for x in nea:
+        for y in neb:
+            block = np.ix_(ca == x, cb == y)
+            sub = sbd_b200.context_from_integrals(ints, a[ca == x], b[cb == y])
+            ref[block] = sub.sigma(C[block].ravel()).reshape(ref[block].shape)
+            r = sub.rdm(C[block].ravel())
+            one, two = one + r[0], two + r[1]
+            sub.close()
+    assert np.abs(ctx.sigma(C.ravel()) - ref.ravel()).max() <= TOL * np.abs(ref).max()
+    assert np.abs(ctx.sigma(C.ravel(), precision=sbd_b200.MIXED) - ref.ravel()).max() <= 2e-5 * np.abs(ref).max()
+    got = ctx.rdm(C.ravel())
+    assert np.abs(got[0] - one).max() <= 1e-11 and np.abs(got[1] - two).max() <= 1e-11
+    ctx.close()
