@@ -304,8 +304,8 @@ int sbdgpu_autotune(sbdgpu_ctx* ctx, int reps, int* ab_group, int* ab_threads, f
  * least 1,024 strings (multiples of 4) and the residues fit in device memory;
  * as one dense FP64 product of both spins for other bases of at most 4,096
  * strings whose operators are dense enough; else the rows kernels; method 1 =
- * the rows kernels always (and the device memory of the integer products is
- * released). */
+ * the rows kernels always (and the device memory of the integer and the dense
+ * products is released). */
 int sbdgpu_set_fp64_same_spin(sbdgpu_ctx* ctx, int method);
 
 const char* sbdgpu_last_error(sbdgpu_ctx* ctx);

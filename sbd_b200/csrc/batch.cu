@@ -400,6 +400,8 @@ extern "C" int sbdgpu_autotune(sbdgpu_ctx* c, int reps, int* ab_group, int* ab_t
     sbdgpu::build_tables(c);
     sbdgpu::compute_hii(c);
     sbdgpu::ensure_scratch(c);
+    c->ab_group = c->ab_threads = 0;
+    if (!sbdgpu::wants_ozaki(c)) sbdgpu::ensure_dense_fp64(c);
     sbdgpu::ensure_ct(c);
     sbdgpu::ensure_io(c);
     sbdgpu::preload_fp64_sigma(c->device);

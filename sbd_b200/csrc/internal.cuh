@@ -130,6 +130,7 @@ struct sbdgpu_ctx {
   // allocation at dense[0]; row strides
   double* dense[2] = {nullptr, nullptr};
   size_t dense_ld[2] = {0, 0};
+  bool dense_failed = false;  // no room for them: not asked for again
   // RDM tables: beta singles grouped by excitation, bra row of every alpha single
   int64_t* rdm_bin_off = nullptr;
   uint32_t* rdm_bin_ent = nullptr;
@@ -193,6 +194,7 @@ void ensure_rdm_tables(sbdgpu_ctx* c);
 void free_rdm_tables(sbdgpu_ctx* c);
 // sigma.cu: the alpha-beta launch shapes (group size, threads) open to this context's FP64 sigma
 std::vector<std::pair<int, int>> ab_shapes(sbdgpu_ctx* c);
+bool uses_tiles(const sbdgpu_ctx* c);
 // The alpha singles an alpha-beta kernel walks: CSR by source string ja (all
 // targets, or only those of one block of target rows, ia0 .. ia0 + rows).
 struct AlphaSingles {

@@ -270,8 +270,11 @@ void build_j_tables(sbdgpu_ctx* c) {
 void compute_hii(sbdgpu_ctx* c) {
   if (c->hii_ready) return;
   build_j_tables(c);
-  double* Ea = (double*)dev_alloc(sizeof(double) * (c->na + c->nb));
-  double* Eb = Ea + c->na;
+  double *Ea = nullptr, *Eb = nullptr;
+  Arena arena(c->stream);
+  arena.add(&Ea, c->na);
+  arena.add(&Eb, c->nb);
+  arena.commit();
   spin_energy_kernel<<<(unsigned)((c->na + 255) / 256), 256, 0, c->stream>>>(c->astr, (int)c->na, c->L, c->h1,
                                                                              c->vf, c->P, Ea);
   spin_energy_kernel<<<(unsigned)((c->nb + 255) / 256), 256, 0, c->stream>>>(c->bstr, (int)c->nb, c->L, c->h1,
@@ -280,11 +283,7 @@ void compute_hii(sbdgpu_ctx* c) {
   dim3 g((unsigned)c->na, (unsigned)((c->nb + 255) / 256));
   hii_kernel<<<g, 256, 0, c->stream>>>(c->astr, c->na, c->nb, Ea, Eb, c->jb, c->P, c->ecore, c->hii);
   SBD_CUDA(cudaGetLastError());
-  // with the set-up, so that the no-allocation sigma finds it (its bases are too
-  // small for the integer products)
-  if (!wants_ozaki(c)) ensure_dense_fp64(c);
   SBD_CUDA(cudaStreamSynchronize(c->stream));
-  cudaFree(Ea);
   c->hii_ready = true;
 }
 

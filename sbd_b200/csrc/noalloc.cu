@@ -23,7 +23,9 @@
 //    nothing.
 //  - The context's own set-up allocations must be done beforehand: call
 //    sbdgpu_build_tables and sbdgpu_diag (or any sigma entry point) once.
-//    Otherwise the call returns SBDGPU_ERR_STATE.
+//    Otherwise the call returns SBDGPU_ERR_STATE.  The dense same-spin product
+//    (same_dense.cu) is taken where an FP64 sigma entry point has made its
+//    operators before, else the rows kernels.
 //  - All calls in the process share the array, and it keeps the previous
 //    call's contents.  Every element the build reads from it is written by the
 //    same call first, so nothing needs clearing; but two calls that overlap on

@@ -230,10 +230,19 @@ bool dense_same_spin(const sbdgpu_ctx* c) {
   return 5.0 * entries >= na * nb * (na + nb);
 }
 
+// Builds the operators where they would be used and are not there yet: by the
+// FP64 sigma and the batch, not by the set-up (an H_ii or an FP32 sigma has no
+// use for them).  Without room for them the rows kernels stay.
 void ensure_dense_fp64(sbdgpu_ctx* c) {
-  if (c->dense[0] || !dense_same_spin(c)) return;
+  if (c->dense[0] || c->dense_failed || c->oz.mode != 0 || !dense_same_spin(c) || !uses_tiles(c)) return;
   const size_t la = (c->na + 1) & ~size_t(1), lb = (c->nb + 1) & ~size_t(1);
-  double* h = (double*)dev_alloc(sizeof(double) * (c->na * la + c->nb * lb));
+  double* h = nullptr;
+  try {
+    h = (double*)dev_alloc(sizeof(double) * (c->na * la + c->nb * lb));
+  } catch (const Error&) {
+    c->dense_failed = true;
+    return;
+  }
   c->dense[0] = h;
   c->dense[1] = h + c->na * la;
   c->dense_ld[0] = la;
@@ -246,6 +255,7 @@ void ensure_dense_fp64(sbdgpu_ctx* c) {
 void free_dense_fp64(sbdgpu_ctx* c) {
   cudaFree(c->dense[0]);
   c->dense[0] = c->dense[1] = nullptr;
+  c->dense_failed = false;
 }
 
 // S += same-spin terms without the diagonal and the singles' Coulomb parts

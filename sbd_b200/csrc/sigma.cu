@@ -406,6 +406,13 @@ std::vector<std::pair<int, int>> ab_shapes(sbdgpu_ctx* c) {
   return out;
 }
 
+// Whether the FP64 alpha-beta term of this context runs on tiles.
+bool uses_tiles(const sbdgpu_ctx* c) {
+  int dev_smem = 0;
+  SBD_CUDA(cudaDeviceGetAttribute(&dev_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
+  return ab_mma_shape(c, c->ab_group, c->ab_threads, sizeof(double), (size_t)dev_smem - 1024).m > 0;
+}
+
 namespace {
 
 // The alpha-beta term: the context's tuned group size and threads for FP64
@@ -447,15 +454,8 @@ void alpha_beta(sbdgpu_ctx* c, const T* C, T* S, const T* vf, const AlphaSingles
     throw Error{SBDGPU_ERR_LIMIT, "alpha-beta kernel: one beta row and integral row exceed shared memory"};
 }
 
-// Whether the FP64 alpha-beta term of this context runs on tiles.
-bool uses_tiles(const sbdgpu_ctx* c) {
-  int dev_smem = 0;
-  SBD_CUDA(cudaDeviceGetAttribute(&dev_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
-  return ab_mma_shape(c, c->ab_group, c->ab_threads, sizeof(double), (size_t)dev_smem - 1024).m > 0;
-}
-
-// Whether its same-spin terms are the dense product (else, or before that, the
-// integer products): no transposes, no ct and st.
+// Whether the same-spin terms of an FP64 sigma are the dense product (else, or
+// before that, the integer products): no transposes, no ct and st.
 bool dense_path(const sbdgpu_ctx* c) { return c->dense[0] && c->oz.mode == 0 && uses_tiles(c); }
 
 // The full kernel sequence of one sigma on given scratch (ct, st: na*nb of T).
@@ -542,6 +542,7 @@ void sigma_fp64(sbdgpu_ctx* c, const double* C, double* S) {
   }
   ensure_scratch(c);
   const bool tiles = uses_tiles(c);
+  if (!wants_ozaki(c)) ensure_dense_fp64(c);
   if (wants_ozaki(c) || !dense_path(c)) ensure_ct(c);
   if (use_ozaki(c) && same_spin_ozaki_fp64(c, C, S, c->ct, c->st, true, !tiles)) {
     const SpinTables& ta = c->tab[0];

@@ -1,0 +1,70 @@
+"""Device memory of the dense same-spin product (csrc/same_dense.cu): made by the
+FP64 sigma, not by the set-up; given back with the rows kernels; without room
+for it the rows kernels run."""
+import numpy as np
+import pytest
+
+import sbd_b200
+from sbd_b200 import synth
+
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-12  # the bound of the sigma parity tests
+MB = 1 << 20
+OPERATORS = 8 * (4060 ** 2 + 3 * 4)  # bytes: rows padded to even lengths
+
+
+def _context():
+    # 4,060 x 3 strings: vectors of 0.1 MB beside 132 MB of operators
+    ints = synth.make_integrals(30, 6)
+    a = synth.full_strings(30, 3)
+    ctx = sbd_b200.context_from_integrals(ints, a, a[:3])
+    ctx.tables(0)
+    return ctx, np.random.default_rng(6).normal(size=ctx.n)
+
+
+def _free():
+    import torch
+    torch.cuda.synchronize()
+    return torch.cuda.mem_get_info(0)[0]
+
+
+def test_operators_are_made_by_the_fp64_sigma_and_given_back():
+    ctx, C = _context()
+    free0 = _free()
+    ctx.hii()
+    assert free0 - _free() < OPERATORS // 2
+    got = ctx.sigma(C)
+    free1 = _free()
+    assert free0 - free1 >= OPERATORS
+    ctx.set_fp64_same_spin(1)
+    assert _free() - free1 >= OPERATORS
+    ref = ctx.sigma(C)
+    assert free0 - _free() < OPERATORS // 2
+    assert np.abs(got - ref).max() <= TOL * np.abs(ref).max()
+    ctx.set_fp64_same_spin(0)
+    assert np.abs(ctx.sigma(C) - ref).max() <= TOL * np.abs(ref).max()
+    assert free0 - _free() >= OPERATORS
+    ctx.close()
+
+
+def test_rows_kernels_without_room_for_the_operators():
+    import torch
+    small, _ = _context()  # loads every kernel
+    small.sigma(np.ones(small.n))
+    small.rdm(np.ones(small.n) / small.n ** 0.5)
+    small.close()
+    ctx, C = _context()
+    torch.cuda.empty_cache()
+    taken = torch.empty(_free() - 96 * MB, dtype=torch.uint8, device="cuda")
+    ctx.hii()
+    got = ctx.sigma(C)
+    e, _, _, _ = ctx.davidson(C / np.linalg.norm(C), 1, 4, 1e-10)
+    (eb,), _, _ = sbd_b200.davidson_batch([ctx], [C / np.linalg.norm(C)], 1, 4, 1e-10)
+    del taken
+    torch.cuda.empty_cache()
+    ctx.set_fp64_same_spin(1)
+    ref = ctx.sigma(C)
+    assert np.abs(got - ref).max() <= TOL * np.abs(ref).max()
+    assert abs(e - eb) < 1e-10
+    ctx.close()
