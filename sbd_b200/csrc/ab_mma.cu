@@ -601,10 +601,9 @@ void launch_mma(sbdgpu_ctx* c, const T* C, T* S, const AlphaSingles& as, int nt,
 
 }  // namespace
 
-// Tiles of the beta singles for ab_mma_kernel.  A string given twice would put
-// two kets into one slot, and the slots hold 16-bit kets with one value free
-// for the zero: such bases keep the gather kernel.
-void build_ab_tiles(sbdgpu_ctx* c, SpinTables& t, const std::vector<uint64_t>& strs) {
+namespace {
+
+void build_tiles(sbdgpu_ctx* c, SpinTables& t, const std::vector<uint64_t>& strs) {
   const size_t n = strs.size();
   if (n == 0 || n + kZeros > 65536) return;
   std::vector<uint64_t> sorted(strs);
@@ -676,6 +675,26 @@ void build_ab_tiles(sbdgpu_ctx* c, SpinTables& t, const std::vector<uint64_t>& s
       (int)n, words, t.s_off, t.s_idx, t.s_info, t.tile_pos, t.tile_grp, t.tile_ent, large);
   SBD_CUDA(cudaGetLastError());
   SBD_CUDA(cudaStreamSynchronize(st));
+}
+
+}  // namespace
+
+// Tiles of the beta singles for ab_mma_kernel.  A string given twice would put
+// two kets into one slot, and the slots hold 16-bit kets with sixteen values
+// free for the zeros: such bases keep the gather kernel, and so does one whose
+// tiles device memory has no room for.
+void build_ab_tiles(sbdgpu_ctx* c, SpinTables& t, const std::vector<uint64_t>& strs) {
+  try {
+    build_tiles(c, t, strs);
+  } catch (const Error& e) {
+    if (e.code != SBDGPU_ERR_ALLOC) throw;
+    cudaFree(t.tile_grp);
+    cudaFree(t.tile_ent);
+    t.tile_grp = nullptr;
+    t.tile_pos = nullptr;
+    t.tile_ent = nullptr;
+    t.n_tile_grp = 0;
+  }
 }
 
 // Without stages the kernel may use all that the opt-in limit leaves beside its

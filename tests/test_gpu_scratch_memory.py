@@ -1,6 +1,7 @@
-"""Device memory of the dense same-spin product (csrc/same_dense.cu): made by the
-FP64 sigma, not by the set-up; given back with the rows kernels; without room
-for it the rows kernels run."""
+"""Device memory of what speeds a context up: the dense same-spin operators
+(csrc/same_dense.cu) are made by the FP64 sigma, not by the set-up, and given
+back with the choice of the rows kernels; without room for them, or for the
+alpha-beta tiles (csrc/ab_mma.cu), the kernels that need none run."""
 import numpy as np
 import pytest
 
@@ -70,4 +71,32 @@ def test_rows_kernels_without_room_for_the_operators():
     for e, w in runs:  # the energies are the Rayleigh quotients of the vectors
         s = ctx.sigma(w)
         assert abs(e - w @ s) <= TOL * np.abs(s).max() * np.abs(w).sum()
+    ctx.close()
+
+
+def test_gather_kernel_without_room_for_the_tiles():
+    import torch
+
+    ints = synth.make_integrals(20, 6)
+    b = synth.full_strings(20, 6)[:26000]  # some 14 MB of tiles, allocated last
+
+    def build(leave=None):
+        ctx = sbd_b200.context_from_integrals(ints, b[:2], b)
+        torch.cuda.empty_cache()
+        free = _free()
+        taken = torch.empty(free - leave, dtype=torch.uint8, device="cuda") if leave else None
+        assert sbd_b200.lib().sbdgpu_build_tables(ctx._h) == 0
+        del taken
+        torch.cuda.empty_cache()
+        return ctx, free - _free()
+    ctx, size = build()
+    C = np.random.default_rng(6).normal(size=ctx.n)
+    W = C / np.linalg.norm(C)
+    ref, (ref1, ref2) = ctx.sigma(C), ctx.rdm(W)
+    ctx.close()
+    ctx, without = build(size - 6 * MB)
+    assert without < size - 6 * MB
+    assert np.abs(ctx.sigma(C) - ref).max() <= TOL * np.abs(ref).max()
+    one, two = ctx.rdm(W)
+    assert np.abs(one - ref1).max() <= 1e-11 and np.abs(two - ref2).max() <= 1e-11
     ctx.close()
