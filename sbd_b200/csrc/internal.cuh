@@ -189,7 +189,7 @@ void rdm(sbdgpu_ctx* c, const double* dW, double* one, double* two);
 // rdm.cu: the off-diagonal terms, added into device arrays one [2][L*L] and two [4][L^4]
 void rdm_offdiag(sbdgpu_ctx* c, const double* dW, double* one, double* two);
 // rdm_mma.cu: the same, opposite-spin diagonal included, by products of W' (phase applied)
-void rdm_products(sbdgpu_ctx* c, const double* Wp, double* one, double* two, double* dia);
+bool rdm_products(sbdgpu_ctx* c, const double* Wp, double* one, double* two, double* dia);
 void ensure_rdm_tables(sbdgpu_ctx* c);
 void free_rdm_tables(sbdgpu_ctx* c);
 // sigma.cu: the alpha-beta launch shapes (group size, threads) open to this context's FP64 sigma

@@ -448,38 +448,40 @@ void occupation(sbdgpu_ctx* c, const double* dW, double* dens) {
 void rdm(sbdgpu_ctx* c, const double* dW, double* one, double* two) {
   int L = c->L;
   size_t L2 = (size_t)L * L, L4 = L2 * L2;
-  // bases with alpha-beta tiles (distinct strings, at most 65,535 beta ones):
-  // products on the tensor pipe, the opposite-spin diagonal included
-  const bool products = c->tab[1].tile_grp != nullptr;
-  double *d_one = nullptr, *Da = nullptr;
+  double *d_one = nullptr, *Da = nullptr, *X = nullptr;
   Arena arena(c->stream);
   arena.add(&d_one, 2 * L2 + 4 * L4);
-  arena.add(&Da, c->na + c->nb + (products ? 0 : c->na * L));
+  arena.add(&Da, c->na + c->nb);
   arena.commit();
   double* d_two = d_one + 2 * L2;
   SBD_CUDA(cudaMemsetAsync(d_one, 0, sizeof(double) * (2 * L2 + 4 * L4), c->stream));
+  // bases with alpha-beta tiles (distinct beta strings, at most 65,520): products
+  // on the tensor pipe, the opposite-spin diagonal included
+  bool products = c->tab[1].tile_grp != nullptr;
   if (products) {
     ensure_io(c);
     phase_copy(c, dW, c->io_b);
-    rdm_products(c, c->io_b, d_one, d_two, Da);
-  } else {
+    products = rdm_products(c, c->io_b, d_one, d_two, Da);
+  }
+  std::vector<double> h(c->na + c->nb), hX(products ? 0 : c->na * L);
+  Arena moment(c->stream);
+  if (!products) {
+    moment.add(&X, hX.size());
+    moment.commit();
     rdm_offdiag(c, dW, d_one, d_two);
     // diagonal contributions (ZeroDiffCorrelation, correlation.h:15-44) from the
     // alpha-row weights, beta-column weights and the alpha x beta occupation moment
-    double* Db = Da + c->na;
-    double* X = Db + c->nb;
     row_weights_kernel<<<(unsigned)c->na, 256, 0, c->stream>>>(dW, c->bstr, c->nb, L, Da, X);
-    col_weights_kernel<<<(unsigned)((c->nb + 255) / 256), 256, 0, c->stream>>>(dW, c->na, c->nb, Db);
+    col_weights_kernel<<<(unsigned)((c->nb + 255) / 256), 256, 0, c->stream>>>(dW, c->na, c->nb, Da + c->na);
     SBD_CUDA(cudaGetLastError());
+    SBD_CUDA(cudaMemcpyAsync(hX.data(), X, sizeof(double) * hX.size(), cudaMemcpyDeviceToHost, c->stream));
   }
-  std::vector<double> h(c->na + c->nb + (products ? 0 : c->na * L));
   SBD_CUDA(cudaMemcpyAsync(h.data(), Da, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, c->stream));
   SBD_CUDA(cudaMemcpyAsync(one, d_one, sizeof(double) * 2 * L2, cudaMemcpyDeviceToHost, c->stream));
   SBD_CUDA(cudaMemcpyAsync(two, d_two, sizeof(double) * 4 * L4, cudaMemcpyDeviceToHost, c->stream));
   SBD_CUDA(cudaStreamSynchronize(c->stream));
   const double* hDa = h.data();
   const double* hDb = hDa + c->na;
-  const double* hX = hDb + c->nb;
   std::vector<double> Aaa(L2, 0.0), Abb(L2, 0.0), M(L2, 0.0), na1(L, 0.0), nb1(L, 0.0);
   for (size_t ia = 0; ia < c->na; ia++) {
     uint64_t a = c->h_astr[ia];

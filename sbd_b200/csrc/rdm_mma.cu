@@ -409,8 +409,9 @@ __global__ void opposite_spin_place_kernel(const double* __restrict__ G, int L, 
 }  // namespace
 
 // one [2][L^2] and two [4][L^4] += every element of W' W' but the same-spin
-// diagonal ones; dia [na + nb]: the strings' weights
-void rdm_products(sbdgpu_ctx* c, const double* Wp, double* one, double* two, double* dia) {
+// diagonal ones; dia [na + nb]: the strings' weights.  False, with nothing done,
+// where device memory has no room for its tables.
+bool rdm_products(sbdgpu_ctx* c, const double* Wp, double* one, double* two, double* dia) {
   const int L = c->L, P = c->P, ntile = (P + 7) / 8;
   const size_t na = c->na, nb = c->nb, quads = (nb + 3) / 4, ncol = (size_t)ntile * 8;
   cudaStream_t st = c->stream;
@@ -424,7 +425,11 @@ void rdm_products(sbdgpu_ctx* c, const double* Wp, double* one, double* two, dou
   arena.add(&G, (size_t)P * 2 * ncol);
   arena.add(&ent, quads * ntile * 32);
   arena.add(&flags, quads * ntile);
-  arena.commit();
+  try {
+    arena.commit();
+  } catch (const Error&) {
+    return false;
+  }
   SBD_CUDA(cudaMemsetAsync(G, 0, sizeof(double) * P * 2 * ncol, st));
   const SpinTables& ta = c->tab[0];
   const SpinTables& tb = c->tab[1];
@@ -468,6 +473,7 @@ void rdm_products(sbdgpu_ctx* c, const double* Wp, double* one, double* two, dou
     }
   }
   SBD_CUDA(cudaStreamSynchronize(st));
+  return true;
 }
 
 }  // namespace sbdgpu

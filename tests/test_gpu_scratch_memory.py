@@ -100,3 +100,21 @@ def test_gather_kernel_without_room_for_the_tiles():
     one, two = ctx.rdm(W)
     assert np.abs(one - ref1).max() <= 1e-11 and np.abs(two - ref2).max() <= 1e-11
     ctx.close()
+
+
+def test_scalar_rdm_kernels_without_room_for_the_products():
+    import torch
+
+    ints = synth.make_integrals(20, 7)
+    b = synth.full_strings(20, 6)[:26000]  # panels of 1 GiB
+    ctx = sbd_b200.context_from_integrals(ints, b[:2], b)
+    W = np.random.default_rng(7).normal(size=ctx.n)
+    W /= np.linalg.norm(W)
+    ref1, ref2 = ctx.rdm(W)
+    torch.cuda.empty_cache()
+    taken = torch.empty(_free() - 256 * MB, dtype=torch.uint8, device="cuda")
+    one, two = ctx.rdm(W)
+    del taken
+    torch.cuda.empty_cache()
+    assert np.abs(one - ref1).max() <= 1e-11 and np.abs(two - ref2).max() <= 1e-11
+    ctx.close()
