@@ -292,9 +292,10 @@ int sbdgpu_mlp_loss_grad(int device, const float* w, int B, const float* X, cons
  * basis is refused. */
 int sbdgpu_set_tuning(sbdgpu_ctx* ctx, int ab_group, int ab_threads);
 
-/* Time every alpha-beta shape that fits (reps FP64 sigma builds each, after
- * one warm-up) and keep the fastest on the context; its shape and sigma time
- * in *ab_group, *ab_threads, *best_ms (each may be NULL). */
+/* Time every alpha-beta shape that fits, and the default where its launch is
+ * none of those (reps FP64 sigma builds each, after one warm-up), and keep the
+ * fastest on the context; its shape ((0, 0): the default) and sigma time in
+ * *ab_group, *ab_threads, *best_ms (each may be NULL). */
 int sbdgpu_autotune(sbdgpu_ctx* ctx, int reps, int* ab_group, int* ab_threads, float* best_ms);
 
 /* How the FP64 sigma forms its same-spin terms (an extension): method 0 (the

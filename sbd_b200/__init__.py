@@ -236,8 +236,8 @@ class Context:
         self._check(lib().sbdgpu_set_tuning(self._h, int(ab_group), int(ab_threads)))
 
     def autotune(self, reps: int = 3):
-        """Time every alpha-beta shape that fits, keep the fastest:
-        (ab_group, ab_threads, sigma ms)."""
+        """Time every alpha-beta shape that fits and the default, keep the
+        fastest: (ab_group, ab_threads, sigma ms); (0, 0): the default."""
         g, t, ms = ctypes.c_int(0), ctypes.c_int(0), ctypes.c_float(0.0)
         self._check(lib().sbdgpu_autotune(self._h, int(reps), ctypes.byref(g), ctypes.byref(t), ctypes.byref(ms)))
         return g.value, t.value, ms.value

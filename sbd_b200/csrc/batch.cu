@@ -418,9 +418,13 @@ extern "C" int sbdgpu_autotune(sbdgpu_ctx* c, int reps, int* ab_group, int* ab_t
         cudaEventDestroy(b);
       }
     } ev{e0, e1};
+    // the default too, where its launch is none of the listed ones: it is kept
+    // unless one of them beats it
+    auto shapes = sbdgpu::ab_shapes(c);
+    if (!sbdgpu::ab_default_listed(c, shapes)) shapes.insert(shapes.begin(), std::make_pair(0, 0));
     float best = 1e30f;
     std::pair<int, int> pick{0, 0};
-    for (const auto& sh : sbdgpu::ab_shapes(c)) {
+    for (const auto& sh : shapes) {
       c->ab_group = sh.first;
       c->ab_threads = sh.second;
       sbdgpu::sigma_fp64_prepared(c, c->io_a, c->io_b, c->ct, c->st);  // warm-up

@@ -194,6 +194,7 @@ void ensure_rdm_tables(sbdgpu_ctx* c);
 void free_rdm_tables(sbdgpu_ctx* c);
 // sigma.cu: the alpha-beta launch shapes (group size, threads) open to this context's FP64 sigma
 std::vector<std::pair<int, int>> ab_shapes(sbdgpu_ctx* c);
+bool ab_default_listed(const sbdgpu_ctx* c, const std::vector<std::pair<int, int>>& shapes);
 bool uses_tiles(const sbdgpu_ctx* c);
 // The alpha singles an alpha-beta kernel walks: CSR by source string ja (all
 // targets, or only those of one block of target rows, ia0 .. ia0 + rows).

@@ -406,6 +406,23 @@ std::vector<std::pair<int, int>> ab_shapes(sbdgpu_ctx* c) {
   return out;
 }
 
+// Whether the launch of the default is that of one of the shapes: the gather
+// kernel's always is; the tiles may run with 768 threads, or without stages where
+// no group of 8 or 16 leaves the gather kernel room.
+bool ab_default_listed(const sbdgpu_ctx* c, const std::vector<std::pair<int, int>>& shapes) {
+  int dev_smem = 0;
+  SBD_CUDA(cudaDeviceGetAttribute(&dev_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
+  const auto of = [&](int group, int threads) {
+    return ab_mma_shape(c, group, threads, sizeof(double), (size_t)dev_smem - 1024);
+  };
+  const MmaShape d = of(0, 0);
+  if (!d.m) return true;
+  return std::any_of(shapes.begin(), shapes.end(), [&](const std::pair<int, int>& sh) {
+    const MmaShape s = of(sh.first, sh.second);
+    return s.m == d.m && s.nt == d.nt && s.sb == d.sb;
+  });
+}
+
 // Whether the FP64 alpha-beta term of this context runs on tiles.
 bool uses_tiles(const sbdgpu_ctx* c) {
   int dev_smem = 0;

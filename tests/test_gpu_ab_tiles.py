@@ -210,3 +210,26 @@ def test_strings_of_several_electron_counts(nea, neb):
     got = ctx.rdm(C.ravel())
     assert np.abs(got[0] - one).max() <= 1e-11 and np.abs(got[1] - two).max() <= 1e-11
     ctx.close()
+
+
+def test_autotune_keeps_the_default_where_no_listed_shape_is_faster():
+    # tiles without stages are none of the shapes that can be set: only the gather kernel's groups of 4 and fewer fit
+    ints = synth.make_integrals(48, 3)
+    b = synth.selected_strings(48, 4, 19990, np.diag(ints.h), 4)
+    ctx = sbd_b200.context_from_integrals(ints, b[:60], b)
+    C = np.random.default_rng(1).normal(size=ctx.n)
+
+    def alpha_beta_ms():
+        ctx.sigma(C)
+        ms = []
+        for _ in range(5):
+            ctx.sigma(C)
+            ms.append(ctx.last_sigma_ms()[2])
+        return min(ms)
+    default = alpha_beta_ms()
+    ctx.set_tuning(4, 1024)
+    assert alpha_beta_ms() > 1.5 * default
+    g, t, ms = ctx.autotune(3)
+    assert (g, t) == (0, 0) and ms > 0
+    assert alpha_beta_ms() <= 1.2 * default
+    ctx.close()
