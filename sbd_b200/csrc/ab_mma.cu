@@ -611,6 +611,8 @@ void build_tiles(sbdgpu_ctx* c, SpinTables& t, const std::vector<uint64_t>& strs
   if (std::adjacent_find(sorted.begin(), sorted.end()) != sorted.end()) return;
   for (uint64_t s : strs)
     if (__builtin_popcountll(s) != __builtin_popcountll(strs[0])) return;
+  // an infinite integral times the zero of an empty slot would be a NaN
+  if (!c->vf_finite) return;
   cudaStream_t st = c->stream;
   const int npair = c->L * (c->L - 1) / 2, words = (npair + 31) / 32;
   // Tiles: runs of up to eight strings, cut where the union of their pairs would
@@ -680,9 +682,10 @@ void build_tiles(sbdgpu_ctx* c, SpinTables& t, const std::vector<uint64_t>& strs
 }  // namespace
 
 // Tiles of the beta singles for ab_mma_kernel.  A string given twice would put
-// two kets into one slot, and the slots hold 16-bit kets with sixteen values
-// free for the zeros: such bases keep the gather kernel, and so does one whose
-// tiles device memory has no room for.
+// two kets into one slot, the slots hold 16-bit kets with sixteen values free
+// for the zeros, and the integrals of a step meet strings without its pairs:
+// bases of repeated or too many strings and non-finite integrals keep the
+// gather kernel, and so does one whose tiles device memory has no room for.
 void build_ab_tiles(sbdgpu_ctx* c, SpinTables& t, const std::vector<uint64_t>& strs) {
   try {
     build_tiles(c, t, strs);

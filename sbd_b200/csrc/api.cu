@@ -454,6 +454,13 @@ int sbdgpu_create(sbdgpu_ctx** out, int norb, size_t na, size_t nb, const uint64
         size_t a = std::max(i, j), b = std::min(i, j);
         c->h_vf[i * P + j] = eri_packed[a * (a + 1) / 2 + b];
       }
+    unsigned bad = 0;  // by the exponent bits: a loop the compiler takes in vectors
+    for (size_t i = 0; i < P * (P + 1) / 2; i++) {
+      uint64_t bits;
+      std::memcpy(&bits, &eri_packed[i], sizeof(bits));
+      bad |= (bits & 0x7FF0000000000000ull) == 0x7FF0000000000000ull;
+    }
+    c->vf_finite = !bad;
     SBD_CUDA(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
     for (int k = 0; k < 8; k++) SBD_CUDA(cudaEventCreate(&c->ev[k]));
     c->astr = (uint64_t*)sbdgpu::dev_alloc(sizeof(uint64_t) * na);

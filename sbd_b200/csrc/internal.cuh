@@ -84,6 +84,7 @@ struct sbdgpu_ctx {
   double ecore = 0.0;
   std::vector<uint64_t> h_astr, h_bstr;
   std::vector<double> h_h1, h_vf;  // host copies
+  bool vf_finite = true;           // no integral of h_vf is an infinity or a NaN
   uint64_t* astr = nullptr;
   uint64_t* bstr = nullptr;
   double* h1 = nullptr;  // [L*L]

@@ -233,3 +233,21 @@ def test_autotune_keeps_the_default_where_no_listed_shape_is_faster():
     assert (g, t) == (0, 0) and ms > 0
     assert alpha_beta_ms() <= 1.2 * default
     ctx.close()
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_non_finite_integral_stays_where_the_operator_has_it(bad):
+    ints, a, b = _system(9, 3, 3, 40, 41, 11)
+    for p, q, r, s in ((1, 4, 2, 7), (2, 7, 1, 4)):  # (pq|rs), all eight orders
+        for x, y in ((p, q), (q, p)):
+            for u, v in ((r, s), (s, r)):
+                ints.eri[x, y, u, v] = bad
+    C = np.random.default_rng(11).normal(size=len(a) * len(b))
+    ctx = sbd_b200.context_from_integrals(ints, a, b)
+    got = ctx.sigma(C)
+    ref = oracle.Oracle(9, a, b, ints.ecore, ints.h, ints.eri).sigma(C)
+    finite = np.isfinite(ref)
+    assert finite.any() and not finite.all()
+    assert np.array_equal(np.isfinite(got), finite)
+    assert np.abs(got[finite] - ref[finite]).max() <= TOL * np.abs(ref[finite]).max()
+    ctx.close()
