@@ -251,3 +251,29 @@ def test_non_finite_integral_stays_where_the_operator_has_it(bad):
     assert np.array_equal(np.isfinite(got), finite)
     assert np.abs(got[finite] - ref[finite]).max() <= TOL * np.abs(ref[finite]).max()
     ctx.close()
+
+
+@pytest.mark.parametrize("na,nb", [(193, 257), (257, 194), (256, 256), (65, 449)])
+def test_dense_same_spin_product_of_64_wide_tiles(na, nb):
+    # at least 16 tiles of 64 x 64 with and without remainders, odd and even rows; then a NaN and an infinity, whose
+    # tiles are evaluated again
+    ints, a, b = _system(11, 5, 5, na, nb, 60 + na)
+    ctx = sbd_b200.context_from_integrals(ints, a, b)
+    C = np.random.default_rng(9).normal(size=(na, nb))
+    orc = oracle.Oracle(11, a, b, ints.ecore, ints.h, ints.eri)
+    ref = orc.sigma(C.ravel())
+    assert np.abs(ctx.sigma(C.ravel()) - ref).max() <= TOL * np.abs(ref).max()
+    C[na - 1, 70], C[3, nb - 1] = np.nan, np.inf
+    got, ref = ctx.sigma(C.ravel()), orc.sigma(C.ravel())
+    finite = np.isfinite(ref)
+    assert finite.any() and not finite.all()
+    assert np.array_equal(np.isfinite(got), finite)
+    assert np.abs(got[finite] - ref[finite]).max() <= TOL * np.abs(ref[finite]).max()
+    ctx.close()
+
+
+@pytest.mark.parametrize("na,nb", [(30, 41), (250, 260)])
+def test_repeated_alpha_strings(na, nb):
+    # only beta strings have to be distinct: tiles, the dense product and the RDM products take such a basis
+    ints, a, b = _system(11, 5, 5, na, nb, 80 + na)
+    _check(ints, np.concatenate([a, a[:3]]), b, shapes=((0, 0), (16, 128), (4, 128)))
