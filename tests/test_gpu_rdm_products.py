@@ -64,3 +64,33 @@ def test_non_finite_input_stays_where_its_terms_go(bad):
         assert np.array_equal(np.isfinite(x), finite)
         assert np.abs(x[finite] - r[finite]).max() <= TOL
     ctx.close()
+
+
+def test_repeated_alpha_strings():
+    ints = synth.make_integrals(8, 5)
+    s = synth.full_strings(8, 3)
+    a, b = np.concatenate([s[:20], s[5:8]]), s[10:31]
+    ctx = sbd_b200.context_from_integrals(ints, a, b)
+    W = np.random.default_rng(5).normal(size=ctx.n)
+    W /= np.linalg.norm(W)
+    for x, r in zip(ctx.rdm(W), oracle.Oracle(8, a, b, ints.ecore, ints.h, ints.eri).correlation(W)):
+        assert np.abs(x - r).max() <= TOL
+    ctx.close()
+
+
+@pytest.mark.parametrize("na,nb", [(12000, 3), (3, 12000), (2, 29200)])
+def test_long_spins(na, nb):
+    # 12,000 strings: two panels of the same-spin products; 29,200 beta strings: more than shared memory holds of a
+    # row of W
+    s = synth.full_strings(26, 6)
+    ints = synth.make_integrals(26, 4)
+    rng = np.random.default_rng(na)
+    near = s[(s & np.uint64(0x3F)) == 7]  # 1,140 strings that share three orbitals, so that the short spin connects
+    a, b = (np.sort(rng.choice(s if n > 100 else near[:20], n, replace=False)) for n in (na, nb))
+    ctx = sbd_b200.context_from_integrals(ints, a, b)
+    W = rng.normal(size=ctx.n)
+    W /= np.linalg.norm(W)
+    one, two = ctx.rdm(W)
+    ref1, ref2 = oracle.Oracle(26, a, b, ints.ecore, ints.h, ints.eri).correlation(W)
+    assert np.abs(one - ref1).max() <= TOL and np.abs(two - ref2).max() <= TOL
+    ctx.close()
