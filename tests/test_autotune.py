@@ -50,3 +50,22 @@ def test_committed_table_is_well_formed():
         assert key.startswith("nb<=") and ",P<=" in key
         assert e["ab_group"] in (1, 2, 4, 8, 16) and e["ab_threads"] in (128, 256, 512, 1024)
         assert e["ms"] > 0 and e["contexts"] >= 1
+
+
+def test_tune_keeps_a_shape_only_where_it_beats_the_default(monkeypatch):
+    ms = {(0, 0): 1.0, (16, 128): 0.99, (8, 256): 0.9, (4, 512): 1.2}
+    monkeypatch.setattr(autotune, "_SHAPES", list(ms))
+    monkeypatch.setattr(autotune, "_sigma_ms", lambda c, reps: ms[c.shape] * c.scale.get(c.shape, 1.0))
+
+    def ctx(nb, scale={}, fits=True):
+        c = FakeCtx(300, nb, 10)
+        c.scale = scale
+        if not fits:
+            set_any = c.set_tuning
+            c.set_tuning = lambda g, t: (_ for _ in ()).throw(RuntimeError()) if g == 8 else set_any(g, t)
+        return c
+    # 10 % on a class of one; on the total of a class of two; not where it does not fit one of them or wins by 1 %
+    table = autotune.tune([ctx(200), ctx(400), ctx(500, {(8, 256): 1.3}), ctx(900), ctx(1000, fits=False)])
+    assert {k: (e["ab_group"], e["ab_threads"], e["contexts"]) for k, e in table.items()} == {
+        "nb<=256,P<=64": (8, 256, 1)}
+    assert autotune.tune([ctx(400), ctx(500)])["nb<=512,P<=64"]["default_ms"] == 2.0
