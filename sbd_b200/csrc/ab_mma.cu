@@ -26,6 +26,7 @@
 // pair; the empty slots of a half-warp point at one that none of its kets
 // collides with.
 #include <algorithm>
+#include <functional>
 #include <type_traits>
 #include <vector>
 
@@ -114,7 +115,10 @@ __global__ void __launch_bounds__(32) tile_count_kernel(int words, const int64_t
   if (lane == 0) grp[g] = make_int4(0, (c[0] + 3) / 4, (c[1] + 3) / 4, (c[2] + 3) / 4);
 }
 
-constexpr size_t kPlannedTiles = 2048;  // strings from which cuts and deals are planned
+// Beta and alpha strings from which cuts and deals are planned.  Planning takes
+// 0.5 to 0.8 ms of a first pass at 12,000 to 20,000 beta strings; with 100 alpha
+// strings or fewer the alpha-beta term takes less than 0.9 ms, planned or not.
+constexpr size_t kPlannedTiles = 2048, kPlannedSources = 128;
 
 // Per pair of a group, while its steps are dealt out.
 struct PairPlan {
@@ -606,9 +610,11 @@ namespace {
 void build_tiles(sbdgpu_ctx* c, SpinTables& t, const std::vector<uint64_t>& strs) {
   const size_t n = strs.size();
   if (n == 0 || n + kZeros > 65536) return;
-  std::vector<uint64_t> sorted(strs);
-  std::sort(sorted.begin(), sorted.end());
-  if (std::adjacent_find(sorted.begin(), sorted.end()) != sorted.end()) return;
+  if (std::adjacent_find(strs.begin(), strs.end(), std::greater_equal<uint64_t>()) != strs.end()) {  // not ascending
+    std::vector<uint64_t> sorted(strs);
+    std::sort(sorted.begin(), sorted.end());
+    if (std::adjacent_find(sorted.begin(), sorted.end()) != sorted.end()) return;
+  }
   for (uint64_t s : strs)
     if (__builtin_popcountll(s) != __builtin_popcountll(strs[0])) return;
   // an infinite integral times the zero of an empty slot would be a NaN
@@ -622,7 +628,7 @@ void build_tiles(sbdgpu_ctx* c, SpinTables& t, const std::vector<uint64_t>& strs
   // of sigma has no 16-byte lines to keep): 53 -> 58 % of the slots are filled at
   // 4,000 strings of 26 orbitals.
   std::vector<int> cut;  // first strings, then n
-  const bool large = n >= kPlannedTiles;
+  const bool large = n >= kPlannedTiles && c->na >= kPlannedSources;
   if (!large) {
     for (size_t i = 0; i < n; i += 8) cut.push_back((int)i);
     cut.push_back((int)n);
