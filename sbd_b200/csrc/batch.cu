@@ -46,8 +46,7 @@ constexpr int kMaxNb = 32;
 constexpr int kH = 0;                       // projected matrix, column-major [kMaxNb][kMaxNb]
 constexpr int kU = kH + kMaxNb * kMaxNb;    // eigenvectors
 constexpr int kE = kU + kMaxNb * kMaxNb;    // eigenvalues
-constexpr int kDot = kE + kMaxNb;           // scratch dot results
-constexpr int kTol = kDot + 8;              // residual norm
+constexpr int kTol = kE + kMaxNb;           // residual norm
 constexpr int kEn = kTol + 1;               // final energy
 constexpr int kPart = kEn + 7;              // block sums of the vector kernels
 constexpr int kScal = kPart + 32 * kKrylovBlocks;

@@ -989,11 +989,10 @@ void expand_nw(sbdgpu_genop* g, const double* dW, double eps, int select, bool w
   else
     SBD_CUDA(cub::DeviceRadixSort::SortKeys(nullptr, tsort, kn, kn, x.m, 0, 64, st));
   SBD_CUDA(cub::DeviceScan::InclusiveSum(nullptr, tseg, in, in, x.m, st));
-  // one allocation: keys, weights, the sort's second buffers head
-  // flags, segment numbers and the libraries' scratch
+  // one allocation: keys, weights, the sort's second buffers, head flags, segment numbers and the libraries' scratch
   Slices b;
   const size_t at_keys = b.add(sizeof(uint64_t) * x.m * NW), at_vals = b.add(weights ? sizeof(double) * x.m : 0),
-               at_k2 = b.add(sizeof(uint64_t) * x.m), at_v2 = b.add(sizeof(double) * x.m),
+               at_k2 = b.add(sizeof(uint64_t) * x.m), at_v2 = b.add(NW > 1 || weights ? sizeof(double) * x.m : 0),
                at_k3 = b.add(NW > 1 ? sizeof(uint64_t) * x.m : 0), at_i3 = b.add(NW > 1 ? sizeof(int64_t) * x.m : 0),
                at_head = b.add(sizeof(int64_t) * x.m), at_seg = b.add(sizeof(int64_t) * x.m),
                at_t = b.add(std::max(tsort, tseg));

@@ -132,10 +132,10 @@ __device__ __forceinline__ void store_all_residues(std::index_sequence<L...>, co
 
 // symmetric residues modulo the primes of round(X * 2^e_row), int8, planes of
 // `plane` bytes with rows of ld (a multiple of 16, zeros past cols); one block
-// per row of the rows x cols matrix X, four consecutive entries per thread
-// (vec: its rows are 16-byte aligned)
+// per row of the rows x cols matrix X, four consecutive entries per thread (cols
+// a multiple of 4, X 16-byte aligned)
 __global__ void __launch_bounds__(kT) residue_kernel(const double* __restrict__ X, size_t cols, size_t ld, size_t plane,
-                                                    bool vec, const int* __restrict__ e, int8_t* __restrict__ out) {
+                                                    const int* __restrict__ e, int8_t* __restrict__ out) {
   const size_t row = blockIdx.x;
   const int er = e[row];
   const double scale = er == kNonFinite ? 0.0 : pow2(er);  // e <= kMaxExp; >= kBits - 1024
@@ -144,17 +144,13 @@ __global__ void __launch_bounds__(kT) residue_kernel(const double* __restrict__ 
     double x[4] = {0.0, 0.0, 0.0, 0.0};
     if (er == kNonFinite) {
       // residues 0: the reconstruction writes NaN for this row
-    } else if (vec && c + 4 <= cols) {
+    } else if (c < cols) {
       const double2 x01 = *reinterpret_cast<const double2*>(xr + c);
       const double2 x23 = *reinterpret_cast<const double2*>(xr + c + 2);
       x[0] = x01.x;
       x[1] = x01.y;
       x[2] = x23.x;
       x[3] = x23.y;
-    } else {
-#pragma unroll
-      for (int j = 0; j < 4; j++)
-        if (c + j < cols) x[j] = xr[c + j];
     }
     unsigned hu[4], lo[4];
 #pragma unroll
@@ -335,7 +331,7 @@ bool ensure_ozaki(sbdgpu_ctx* c) {
       const size_t p = pad16(n);
       c->oz.h0r[spin] = (int8_t*)dev_alloc((size_t)kMods * p * p);
       if (p != n) SBD_CUDA(cudaMemsetAsync(c->oz.h0r[spin], 0, (size_t)kMods * p * p, st));
-      residue_kernel<<<(unsigned)n, kT, 0, st>>>(tmp, n, p, p * p, n % 2 == 0, c->oz.h0e[spin], c->oz.h0r[spin]);
+      residue_kernel<<<(unsigned)n, kT, 0, st>>>(tmp, n, p, p * p, c->oz.h0e[spin], c->oz.h0r[spin]);
       SBD_CUDA(cudaGetLastError());
       SBD_CUDA(cudaStreamSynchronize(st));
     }
@@ -418,9 +414,8 @@ bool same_spin_ozaki_fp64(sbdgpu_ctx* c, const double* C, double* S, double* ct,
   transpose(C, ct, na, nb, s);
   row_exp_kernel<<<(unsigned)na, kT, 0, s>>>(C, nb, c->oz.ce);
   row_exp_kernel<<<(unsigned)nb, kT, 0, s>>>(ct, na, c->oz.cte);
-  residue_kernel<<<(unsigned)na, kT, 0, s>>>(C, nb, pb, plane, nb % 2 == 0 && ((uintptr_t)C & 15) == 0, c->oz.ce,
-                                             c->oz.cr);
-  residue_kernel<<<(unsigned)nb, kT, 0, s>>>(ct, na, pa, plane, na % 2 == 0, c->oz.cte, c->oz.ctr);
+  residue_kernel<<<(unsigned)na, kT, 0, s>>>(C, nb, pb, plane, c->oz.ce, c->oz.cr);
+  residue_kernel<<<(unsigned)nb, kT, 0, s>>>(ct, na, pa, plane, c->oz.cte, c->oz.ctr);
   SBD_CUDA(cudaGetLastError());
   // alpha: sigma^T (nb x na, column-major) = (C^T)(H0a^T), one INT8 product per prime
   for (int l = 0; l < kMods; l++)
