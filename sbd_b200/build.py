@@ -30,7 +30,7 @@ def _stale(target: str, deps: list[str]) -> bool:
 
 def build_lib(force: bool = False, verbose: bool = False) -> str:
     srcs = [os.path.join(CSRC, s) for s in SOURCES]
-    deps = srcs + [os.path.join(CSRC, "internal.cuh"), os.path.join(ROOT, "include", "sbdgpu.h"),
+    deps = srcs + [os.path.join(CSRC, "internal.cuh"), os.path.join(CSRC, "device.cuh"), os.path.join(ROOT, "include", "sbdgpu.h"),
                    os.path.join(HERE, "include", "sbd_gpu", "generalop.h"), os.path.join(HERE, "include", "sbd_gpu", "tpb.h")]
     if not force and not _stale(LIB, deps):
         return LIB

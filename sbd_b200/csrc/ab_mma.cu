@@ -30,6 +30,7 @@
 #include <type_traits>
 #include <vector>
 
+#include "device.cuh"
 #include "internal.cuh"
 
 namespace sbdgpu {
@@ -41,20 +42,12 @@ constexpr int kZeros = 16;     // zeros behind the row of C, one in each pair of
 constexpr int kMaxWords = 63;  // bitmap words of the off-diagonal pairs: 64 * 63 / 2 = 2016
 
 __device__ __forceinline__ int od_pair(uint32_t info) {  // off-diagonal pair index of a single
-  const int p = info & 63, q = (info >> 6) & 63;
-  const int hi = max(p, q), lo = min(p, q);
-  return hi * (hi - 1) / 2 + lo;
+  return sbdgpu::od_pair((int)(info & 63), (int)((info >> 6) & 63));
 }
 
-// The folded pair (diagonal ones included) of off-diagonal pair o: the larger
-// orbital hi has hi (hi - 1) / 2 <= o < hi (hi + 1) / 2, and hi diagonal
-// pairs come before.
-__device__ __forceinline__ int folded_pair(int o) {
-  int hi = (int)((1.0f + sqrtf(8.0f * (float)o + 1.0f)) * 0.5f);
-  hi += hi * (hi + 1) / 2 <= o;
-  hi -= hi * (hi - 1) / 2 > o;
-  return o + hi;
-}
+// The folded pair (diagonal ones included) of off-diagonal pair o: as many
+// diagonal pairs as its larger orbital come before.
+__device__ __forceinline__ int folded_pair(int o) { return o + od_larger(o); }
 
 // unions[i][l] = pairs used by the strings i .. i + l (l < 8), one warp per i
 __global__ void __launch_bounds__(32) union_kernel(int n, int words, const int64_t* __restrict__ s_off,
@@ -183,62 +176,62 @@ __global__ void __launch_bounds__(32) tile_fill_kernel(int n, int words, const i
       }
     __syncwarp();
   } else {
-  for_entries([&](int t, int nn, int32_t ket, uint32_t info) {
-    const int o = od_pair(info);
-    PairPlan& p = plan[index(o, section_of(o, t))];
-    atomicOr(&p.bank[t], (uint32_t)(ket & 15) << (4 * nn));
-  });
-  __syncwarp();
-  // the strings' bits: one lane per pair would race on the half-word, one string at a time does not
-  for (int t = 0; t < 2; t++)
-    for (int nn = 0; nn < (t ? pos.y >> 8 : pos.y & 0xFF); nn++) {
-      const int i = pos.x + (t ? pos.y & 0xFF : 0) + nn;
-      for (int64_t k = s_off[i] + lane; k < s_off[i + 1]; k += 32) {
-        const int o = od_pair(s_info[k]);
-        plan[index(o, section_of(o, t))].set |= (uint16_t)(1u << (8 * t + nn));
-      }
-      __syncwarp();
-    }
-  // Deal the pairs of a section to its steps: the first one left, then three
-  // times the one whose integral row differs in class from the step's others
-  // and whose kets share fewest banks with theirs (per tile and half-warp of
-  // four strings).
-  for (int s = 0; s < 3; s++) {
-    const int b0 = base[s], cnt = base[s + 1] - b0;
-    uint64_t load[4] = {0, 0, 0, 0};  // 4-bit counts of 16 bank pairs by (tile, half)
-    unsigned classes = 0;
-    for (int at = 0; at < cnt; at++) {
-      if ((at & 3) == 0) {
-        classes = 0;
-        for (int h = 0; h < 4; h++) load[h] = 0;
-      }
-      uint32_t best = 0xFFFFFFFFu;
-      for (int c = lane; c < cnt; c += 32) {
-        const PairPlan& p = plan[b0 + c];
-        if (p.place >= 0) continue;
-        uint32_t cost = 0;
-        if (at & 3) {
-          cost = (classes >> (p.pair & 3)) & 1u ? 8 : 0;
-          for (int h = 0; h < 4; h++)
-            for (int x = 0; x < 4; x++)
-              if ((p.set >> (4 * h + x)) & 1)
-                cost += (uint32_t)(load[h] >> (4 * ((p.bank[h >> 1] >> (4 * (4 * (h & 1) + x))) & 15))) & 15u;
+    for_entries([&](int t, int nn, int32_t ket, uint32_t info) {
+      const int o = od_pair(info);
+      PairPlan& p = plan[index(o, section_of(o, t))];
+      atomicOr(&p.bank[t], (uint32_t)(ket & 15) << (4 * nn));
+    });
+    __syncwarp();
+    // the strings' bits: one lane per pair would race on the half-word, one string at a time does not
+    for (int t = 0; t < 2; t++)
+      for (int nn = 0; nn < (t ? pos.y >> 8 : pos.y & 0xFF); nn++) {
+        const int i = pos.x + (t ? pos.y & 0xFF : 0) + nn;
+        for (int64_t k = s_off[i] + lane; k < s_off[i + 1]; k += 32) {
+          const int o = od_pair(s_info[k]);
+          plan[index(o, section_of(o, t))].set |= (uint16_t)(1u << (8 * t + nn));
         }
-        best = min(best, cost << 16 | (uint32_t)c);
+        __syncwarp();
       }
-      const int pick = (int)(__reduce_min_sync(0xffffffffu, best) & 0xFFFFu);
-      const PairPlan p = plan[b0 + pick];
-      classes |= 1u << (p.pair & 3);
-      for (int h = 0; h < 4; h++) {
-        for (int x = 0; x < 4; x++)
-          if ((p.set >> (4 * h + x)) & 1)
-            load[h] += 1ull << (4 * ((p.bank[h >> 1] >> (4 * (4 * (h & 1) + x))) & 15));
+    // Deal the pairs of a section to its steps: the first one left, then three
+    // times the one whose integral row differs in class from the step's others
+    // and whose kets share fewest banks with theirs (per tile and half-warp of
+    // four strings).
+    for (int s = 0; s < 3; s++) {
+      const int b0 = base[s], cnt = base[s + 1] - b0;
+      uint64_t load[4] = {0, 0, 0, 0};  // 4-bit counts of 16 bank pairs by (tile, half)
+      unsigned classes = 0;
+      for (int at = 0; at < cnt; at++) {
+        if ((at & 3) == 0) {
+          classes = 0;
+          for (int h = 0; h < 4; h++) load[h] = 0;
+        }
+        uint32_t best = 0xFFFFFFFFu;
+        for (int c = lane; c < cnt; c += 32) {
+          const PairPlan& p = plan[b0 + c];
+          if (p.place >= 0) continue;
+          uint32_t cost = 0;
+          if (at & 3) {
+            cost = (classes >> (p.pair & 3)) & 1u ? 8 : 0;
+            for (int h = 0; h < 4; h++)
+              for (int x = 0; x < 4; x++)
+                if ((p.set >> (4 * h + x)) & 1)
+                  cost += (uint32_t)(load[h] >> (4 * ((p.bank[h >> 1] >> (4 * (4 * (h & 1) + x))) & 15))) & 15u;
+          }
+          best = min(best, cost << 16 | (uint32_t)c);
+        }
+        const int pick = (int)(__reduce_min_sync(0xffffffffu, best) & 0xFFFFu);
+        const PairPlan p = plan[b0 + pick];
+        classes |= 1u << (p.pair & 3);
+        for (int h = 0; h < 4; h++) {
+          for (int x = 0; x < 4; x++)
+            if ((p.set >> (4 * h + x)) & 1)
+              load[h] += 1ull << (4 * ((p.bank[h >> 1] >> (4 * (4 * (h & 1) + x))) & 15));
+        }
+        __syncwarp();
+        if (lane == 0) plan[b0 + pick].place = (int16_t)at;
+        __syncwarp();
       }
-      __syncwarp();
-      if (lane == 0) plan[b0 + pick].place = (int16_t)at;
-      __syncwarp();
     }
-  }
   }
   const int4 d = grp[g];
   uint32_t* out = ent + (size_t)d.x * 32;
@@ -291,12 +284,6 @@ __global__ void __launch_bounds__(32) tile_fill_kernel(int n, int words, const i
   }
 }
 
-// D (16 x 8) += A (16 x 4) B (4 x 8), FP64
-__device__ __forceinline__ void mma16(double (&d)[4], double a0, double a1, double b) {
-  asm("mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3},{%4,%5},{%6},{%0,%1,%2,%3};"
-      : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
-      : "d"(a0), "d"(a1), "d"(b));
-}
 // D (8 x 8) += A (8 x 4) B (4 x 8), FP64
 __device__ __forceinline__ void mma8(double (&d)[4], double a0, double b) {
   asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1},{%2},{%3},{%0,%1};"
@@ -748,7 +735,7 @@ MmaShape ab_mma_shape(const sbdgpu_ctx* c, int group, int threads, size_t elem, 
       for (int t : {256, 512, 768, 1024}) {
         const size_t smem = mma_smem(c, m, t, elem, sb);
         if (smem > budget + (sb == 0 ? kUnstagedExtra : 0)) break;
-        const int warps = (int)std::min<size_t>(228 * 1024 / (smem + 1024), 1024 / t) * (t / 32);
+        const int warps = (int)std::min<size_t>(kSmemPerSM / (smem + 1024), 1024 / t) * (t / 32);
         if (warps > best) {
           best = warps;
           s = {m, t, sb};

@@ -100,7 +100,8 @@ struct Bucket {
 // Hash of a state, in 32-bit steps: two odd multipliers per word, then one
 // round of shifts and a multiply, enough to spread bit strings that differ in a
 // few sites (at a quarter full: 1.15 probes per search, 97 % within two).  The
-// upper half only serves tables of more than 2^32 slots.
+// upper half only serves tables of more than 2^32 slots.  Multipliers: xxHash's
+// first three 32-bit primes, and one of C. Wellons's hash prospector.
 template <int NW>
 __host__ __device__ __forceinline__ uint64_t hash_state(const uint64_t* w, uint64_t hmask) {
   uint32_t h = 0;

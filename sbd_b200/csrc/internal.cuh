@@ -46,6 +46,8 @@ constexpr uint32_t kSellInvalid = 0xFFFFFFFFu;
 // limit sbdgpu_wait_selftest accepts)
 constexpr long long kMaxSpinLimit = 1ll << 26;
 constexpr int kSlice = 32;
+constexpr int kSMs = 148;                  // of a B200
+constexpr size_t kSmemPerSM = 228 * 1024;  // 1 KiB of it for every resident CTA
 
 struct SpinTables {
   size_t n = 0;
@@ -236,7 +238,7 @@ void occupation(sbdgpu_ctx* c, const double* dW, double* dens);
 void alpha_weights(sbdgpu_ctx* c, const double* dW, double* D);
 
 // krylov.cu: Davidson vector kernels (basis vectors of type B)
-constexpr int kKrylovBlocks = 592;  // 4 x 148 SMs
+constexpr int kKrylovBlocks = 4 * kSMs;
 template <typename B>
 struct BasisPack {
   const B* p[32];

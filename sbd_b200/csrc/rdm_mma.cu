@@ -25,6 +25,7 @@
 // values: 1M determinants, norb 20, 11.2 -> 3 ms a call.
 #include <algorithm>
 
+#include "device.cuh"
 #include "internal.cuh"
 
 namespace sbdgpu {
@@ -37,12 +38,6 @@ constexpr int kStages = 4;
 constexpr int kAbThreads = 256;  // opposite spins
 constexpr int kWarpTiles = 4;    // n8 tiles per warp
 constexpr int kCtaTiles = kWarpTiles * kAbThreads / 32;
-
-__device__ __forceinline__ void mma16(double (&d)[4], double a0, double a1, double b) {
-  asm("mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3},{%4,%5},{%6},{%0,%1,%2,%3};"
-      : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
-      : "d"(a0), "d"(a1), "d"(b));
-}
 
 __device__ __forceinline__ void copy8(double* dst, const double* src, bool on) {
   const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
@@ -178,11 +173,6 @@ __global__ void __launch_bounds__(128) same_spin_kernel(int S, const double* __r
       add(p2, p1, q2, q1, -v);
     }
   }
-}
-
-__device__ __forceinline__ int od_pair(int a, int b) {
-  const int hi = max(a, b), lo = min(a, b);
-  return hi * (hi - 1) / 2 + lo;
 }
 
 // Beta entries by (four strings, eight columns): ket | forward << 30 | sign <<
@@ -380,9 +370,7 @@ __global__ void opposite_spin_place_kernel(const double* __restrict__ G, int L, 
       hi = lo = x - npair;
       return;
     }
-    hi = (int)((1.0f + sqrtf(8.0f * (float)x + 1.0f)) * 0.5f);
-    hi += hi * (hi + 1) / 2 <= x;
-    hi -= hi * (hi - 1) / 2 > x;
+    hi = od_larger(x);
     lo = x - hi * (hi - 1) / 2;
   };
   // <E_ki (alpha) E_lj (beta)>
@@ -449,7 +437,7 @@ bool rdm_products(sbdgpu_ctx* c, const double* Wp, double* one, double* two, dou
                                                             ent, flags, G);
   }
   SBD_CUDA(cudaGetLastError());
-  opposite_spin_place_kernel<<<148 * 4, 256, 0, st>>>(G, L, ntile, two);
+  opposite_spin_place_kernel<<<kSMs * 4, 256, 0, st>>>(G, L, ntile, two);
   SBD_CUDA(cudaGetLastError());
   for (int S = 0; S < 2; S++) {
     const SpinTables& t = S == 0 ? ta : tb;

@@ -23,6 +23,7 @@
 #include <algorithm>
 #include <cmath>
 
+#include "device.cuh"
 #include "internal.cuh"
 
 namespace sbdgpu {
@@ -41,12 +42,6 @@ struct Tables {
   const double* d_val;
 };
 Tables view(const SpinTables& t) { return Tables{t.s_off, t.s_idx, t.s_val, t.d_off, t.d_idx, t.d_val}; }
-
-__device__ __forceinline__ void mma16(double (&d)[4], double a0, double a1, double b) {
-  asm("mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3},{%4,%5},{%6},{%0,%1,%2,%3};"
-      : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
-      : "d"(a0), "d"(a1), "d"(b));
-}
 
 template <int BYTES>
 __device__ __forceinline__ void copy_async(double* dst, const double* src, bool on) {
@@ -209,7 +204,7 @@ void launch(sbdgpu_ctx* c, const double* C, double* S) {
   // K in shares: eight CTAs per SM, of at least four steps each (1501 x 803
   // strings, 312 tiles: 0.33 ms in one share, 0.27 in three, 0.25 in four)
   const unsigned steps = (unsigned)((c->na + kBK - 1) / kBK + (c->nb + kBK - 1) / kBK);
-  grid.z = std::max(1u, std::min({(148u * 8 + grid.x * grid.y - 1) / (grid.x * grid.y), steps / 4, 16u}));
+  grid.z = std::max(1u, std::min({(kSMs * 8u + grid.x * grid.y - 1) / (grid.x * grid.y), steps / 4, 16u}));
   allow_dynamic_smem(reinterpret_cast<const void*>(same_dense_kernel<WM, WN, V>), c->device);
   same_dense_kernel<WM, WN, V><<<grid, kThreads, smem_bytes<WM, WN>(), c->stream>>>(
       c->dense[0], c->dense_ld[0], c->dense[1], c->dense_ld[1], C, S, c->na, c->nb, view(c->tab[0]), view(c->tab[1]));
