@@ -161,6 +161,27 @@ def ab_smem_floor(st, group, sm_count, sm_mhz):
             "sm_count": sm_count, "sm_mhz": sm_mhz, "floor_ms": floor_ms}
 
 
+def ab_tiles(bstr, norb, smem_optin):
+    """Whether the FP64 alpha-beta term runs on tiles (csrc/ab_mma.cu): distinct
+    beta strings of one electron count, at most 65,520, whose row of C and eight
+    singles' integrals fit in shared memory."""
+    nb = len(bstr)
+    return (nb <= 65520 and len(np.unique(bstr)) == nb and len({int(s).bit_count() for s in bstr}) == 1
+            and norb * (norb - 1) // 2 * 64 + (nb + 16) * 8 <= smem_optin - 128)
+
+
+def same_spin_path(method, na, nb, st, tiles):
+    """How the FP64 sigma forms its same-spin terms by the library's rules
+    (sbdgpu_set_fp64_same_spin): st[spin] = (singles, doubles).  INT8 products
+    need room in device memory as well, which every workload here has."""
+    if method == 1:
+        return "rows"
+    if min(na, nb) >= 1024 and na % 4 == 0 and nb % 4 == 0:
+        return "int8"
+    entries = sum(st[0]) * nb + sum(st[1]) * na
+    return "dense" if tiles and max(na, nb) <= 4096 and 5 * entries >= na * nb * (na + nb) else "rows"
+
+
 def ab_default_group(nb, P, smem_optin):
     """The group size of the FP64 alpha-beta gather kernel without a tuning table:
     the largest of 16, 8, 4, 2 whose integral rows ([P][group + 2] doubles) fit
@@ -731,10 +752,16 @@ def run_gpu(args):
         return 0
     hbm_peak, peak_kind = measured_peaks()
     ab_ms = parts[2] / args.steps
-    same_spin = ("rows" if args.fp64_same_spin == 1
-                 else "int8" if min(ctx.na, ctx.nb) >= 1024 and ctx.na % 4 == 0 and ctx.nb % 4 == 0 else "dense")
+    props = torch.cuda.get_device_properties(dev)
+    smem_optin = getattr(props, "shared_memory_per_block_optin", 232448)
+    tiles = ab_tiles(strs, ints.norb, smem_optin)
+    same_spin = same_spin_path(args.fp64_same_spin, ctx.na, ctx.nb, st, tiles)
+    ab_kernel = "ab_mma_kernel" if tiles else "ab_kernel"
     kernel_names = [f"alpha same-spin and diagonal ({same_spin})", f"beta same-spin ({same_spin})",
-                    "ab_mma_kernel (alpha-beta)"]
+                    f"{ab_kernel} (alpha-beta)"]
+    if same_spin == "dense":
+        kernel_names[:2] = ["same-spin and diagonal (dense)", ""]
+    launches = LAUNCHES_PER_SIGMA[same_spin] + (2 if same_spin == "int8" and not tiles else 0)
     dom = int(np.argmax(parts))
     dom_ms = parts[dom] / args.steps
     dom_bytes = [8.0 * n * 3 + st[0][0] * 16 + st[0][1] * 12, 8.0 * n * 6 + st[1][0] * 16 + st[1][1] * 12,
@@ -743,21 +770,30 @@ def run_gpu(args):
     traffic = args.traffic
     if traffic is None and dom == 2:
         traffic = AB_TRAFFIC_BYTES_PER_DET * n
-    smem_floor = None
-    if dom == 2:
-        props = torch.cuda.get_device_properties(dev)
-        group = ab_default_group(ctx.nb, ctx.norb * (ctx.norb + 1) // 2,
-                                 getattr(props, "shared_memory_per_block_optin", 232448))
-        clk = sampler.summary().get("sm_mhz") or 1965.0
-        if group:
-            smem_floor = ab_smem_floor(st, group, props.multi_processor_count, clk)
-            smem_floor["measured_ms"] = ab_ms
-            smem_floor["frac"] = smem_floor["floor_ms"] / ab_ms
-            smem_floor["note"] = "floor of the one-integral-per-product gather that the tiles replace"
-    ab_flops = 2.0 * st[0][0] * st[1][0]
-    fp64_floor = {"flops": ab_flops, "tflops_peak": FP64_TENSOR_TFLOPS,
-                  "floor_ms": ab_flops / FP64_TENSOR_TFLOPS / 1e9, "measured_ms": ab_ms,
-                  "frac": ab_flops / FP64_TENSOR_TFLOPS / 1e9 / ab_ms}
+    hbm = {"achieved": achieved, "peak": hbm_peak, "unit": "GB/s", "frac": achieved / hbm_peak,
+           "peak_source": peak_kind, "traffic": traffic}
+    if dom == 2 and tiles:
+        # two operations per pair of singles, against the FP64 tensor pipe
+        ab_flops = 2.0 * st[0][0] * st[1][0]
+        tflops = ab_flops / (ab_ms * 1e-3) / 1e12
+        roofline = {"bound": "fp64_tensor", "kernel": kernel_names[dom], "achieved": tflops,
+                    "peak": FP64_TENSOR_TFLOPS, "unit": "TFLOP/s", "frac": tflops / FP64_TENSOR_TFLOPS,
+                    "peak_source": "register-only FP64 mma loop at 1,965 MHz", "flops": ab_flops,
+                    "floor_ms": ab_flops / FP64_TENSOR_TFLOPS / 1e9, "measured_ms": ab_ms,
+                    "limiter": "shared-memory pipe, then the FP64 tensor pipe (ncu at 16M dets: "
+                               "profiles/ab_mma_kernel_c1_L26_6e_4000.md)",
+                    "hbm": hbm}
+    else:
+        roofline = {"bound": "hbm", "kernel": kernel_names[dom], **hbm}
+        if dom == 2:  # the gather kernel: one integral per product from shared memory
+            group = ab_default_group(ctx.nb, ctx.norb * (ctx.norb + 1) // 2, smem_optin)
+            if group:
+                clk = sampler.summary().get("sm_mhz") or 1965.0
+                roofline["smem_floor"] = floor = ab_smem_floor(st, group, props.multi_processor_count, clk)
+                floor["measured_ms"] = ab_ms
+                floor["frac"] = floor["floor_ms"] / ab_ms
+        elif same_spin == "rows":
+            roofline["limiter"] = "L1/L2 streaming of C rows (profiles/rows_kernel_c1_L26_6e_4000.md)"
     line = {
         "metric": METRIC, "value": world * 1000.0 / t_step, "unit": UNIT, "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": t_step, "higher_is_better": True, "scaling": "weak",
@@ -767,15 +803,8 @@ def run_gpu(args):
                    "l2": "inputs (1.15 GB per vector) larger than L2; no flush"},
         "e2e": {"value": world * 1000.0 / t_e2e, "unit": UNIT, "h2d_bytes_per_step": 8 * n,
                 "d2h_bytes_per_step": 8 * n},
-        "gpu_launches": LAUNCHES_PER_SIGMA[same_spin] * args.steps * 2,
-        "roofline": {"bound": "hbm", "kernel": kernel_names[dom], "achieved": achieved, "peak": hbm_peak,
-                     "unit": "GB/s", "frac": achieved / hbm_peak, "peak_source": peak_kind,
-                     "traffic": traffic,
-                     "limiter": ("shared-memory pipe, then the FP64 tensor pipe (ncu at 16M dets: "
-                                 "profiles/ab_mma_kernel_c1_L26_6e_4000.md)")
-                     if dom == 2 else "L1/L2 streaming of C rows (profiles/rows_kernel_c1_L26_6e_4000.md)",
-                     "fp64_tensor_floor": fp64_floor,
-                     "smem_floor": smem_floor},
+        "gpu_launches": launches * args.steps * 2,
+        "roofline": roofline,
         "phases_ms": {"alpha_same_spin_with_diag": parts[0] / args.steps,
                       "beta_same_spin": parts[1] / args.steps, "alpha_beta": ab_ms},
         "flops_per_sigma": alg["flops"], "fp64_tflops": alg["flops"] / (t_step * 1e-3) / 1e12,
