@@ -6,12 +6,12 @@
 // Layout in HBM:
 //   states      [n][nw] uint64 in the caller's order (site q at bit q%64 of
 //               word q/64), nw = 1, 2 or 4
-//   hash table  open addressing with linear probing over a power-of-two
-//               table of at least two to four times the states: a slot holds the key words
-//               and, during a mult, the state's vector element, so that one
-//               probe returns the value itself (a slot of one-word states is 16
-//               bytes: one sector per term instead of three for index, key and
-//               element).  An empty slot's key is a configuration outside the
+//   hash table  open addressing with linear probing over a power-of-two table
+//               of at least four times the states (twice above 1 GiB): a slot
+//               holds the key words and, during a mult, the state's vector
+//               element, so that one probe returns the value itself (a slot of
+//               one-word states is 16 bytes: one sector per term instead of
+//               three for index, key and element).  An empty slot's key is a configuration outside the
 //               basis and its element 0.
 //   terms       the off-diagonal list as arrays (creation mask, sign mask,
 //               coefficient) sorted by annihilation mask, with one bucket
