@@ -539,6 +539,7 @@ int sbdgpu_diag(sbdgpu_ctx* c, double* hii) {
     if (!hii) throw Error{SBDGPU_ERR_ARG, "null output"};
     sbdgpu::build_tables(c);
     sbdgpu::compute_hii(c);
+    sbdgpu::noalloc_setup(c);
     SBD_CUDA(cudaMemcpyAsync(hii, c->hii, sizeof(double) * c->N, cudaMemcpyDeviceToHost, c->stream));
     SBD_CUDA(cudaStreamSynchronize(c->stream));
   });

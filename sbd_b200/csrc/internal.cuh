@@ -309,6 +309,7 @@ void sigma_rows_fp64(sbdgpu_ctx* c, const double* dC, double* S, size_t r0, size
 
 // noalloc.cu
 void noalloc_prepare(int device);
+void noalloc_setup(sbdgpu_ctx* c);  // with sbdgpu_diag
 
 // gemm_same.cu
 bool ensure_dense_same(sbdgpu_ctx* c);

@@ -24,8 +24,9 @@
 //  - The context's own set-up allocations must be done beforehand: call
 //    sbdgpu_build_tables and sbdgpu_diag (or any sigma entry point) once.
 //    Otherwise the call returns SBDGPU_ERR_STATE.  The dense same-spin product
-//    (same_dense.cu) is taken where an FP64 sigma entry point has made its
-//    operators before, else the rows kernels.
+//    (same_dense.cu) is taken where its operators are there: sbdgpu_diag makes
+//    those that take no more than the array itself, an FP64 sigma entry point
+//    any.  Else the rows kernels run.
 //  - All calls in the process share the array, and it keeps the previous
 //    call's contents.  Every element the build reads from it is written by the
 //    same call first, so nothing needs clearing; but two calls that overlap on
@@ -74,6 +75,10 @@ void noalloc_prepare(int device) {
     throw Error{SBDGPU_ERR_CUDA, std::string("cudaGetSymbolAddress(g_sigma_scratch): ") + cudaGetErrorString(e)};
   preload_fp64_sigma(device);
   g_scratch_addr[device] = static_cast<double*>(p);
+}
+
+void noalloc_setup(sbdgpu_ctx* c) {
+  if (c->N <= kNoAllocMaxDets && c->na * c->na + c->nb * c->nb <= 3 * kNoAllocMaxDets) ensure_dense_fp64(c);
 }
 
 }  // namespace sbdgpu

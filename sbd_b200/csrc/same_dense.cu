@@ -226,8 +226,9 @@ bool dense_same_spin(const sbdgpu_ctx* c) {
 }
 
 // Builds the operators where they would be used and are not there yet: by the
-// FP64 sigma and the batch, not by the set-up (an H_ii or an FP32 sigma has no
-// use for them).  Without room for them the rows kernels stay.
+// FP64 sigma and the batch (an FP32 sigma has no use for them; the set-up makes
+// small ones for the no-allocation sigma).  Without room for them the rows
+// kernels stay.
 void ensure_dense_fp64(sbdgpu_ctx* c) {
   if (c->dense[0] || c->dense_failed || c->oz.mode != 0 || !dense_same_spin(c) || !uses_tiles(c)) return;
   const size_t la = (c->na + 1) & ~size_t(1), lb = (c->nb + 1) & ~size_t(1);
